@@ -55,7 +55,12 @@ inline bool allowed_match(const lcg_pair_tables &t, int i, int j) {
     return !t.match_lo || (t.match_lo[i] <= j && j <= t.match_hi[i]);
 }
 
-lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p) {
+// Limits of the lane-per-group fill: the shared-memory rows of its top-level
+// items (span), and 80 MB of matrix storage per warp
+constexpr int LANE_MAX_SPAN = 640;
+constexpr int LANE_MAX_BANDCELLS = 600000;
+
+lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes) {
     auto bad = [&](lcg_status c, const std::string &s) {
         p.code = c;
         p.err = s;
@@ -233,10 +238,38 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p)
             cnt[cell_of[k]]++;
         }
     }
-    p.cre_start.assign(p.bandcells + 1, 0);
-    for (int c = 0; c < p.bandcells; ++c) p.cre_start[c + 1] = p.cre_start[c] + cnt[c];
-    std::vector<int> fillp(p.cre_start.begin(), p.cre_start.end() - 1);
-    std::vector<int> ord(p.cre_start[p.bandcells]);
+    if (o.struct_local || anchors || t.indel_opening > 0 || p.span > LANE_MAX_SPAN || p.bandcells > LANE_MAX_BANDCELLS)
+        lanes = 0;
+    p.lane_groups = lanes;
+    int entries = 0;
+    if (lanes) {
+        // by blocks of 8 columns, quads of 4 rows, rows and columns; the lists
+        // then have starts and ends
+        p.flags |= PF_LANES;
+        p.cre_start.resize(2 * (size_t)p.bandcells);
+        const int *mn = p.min_col.data(), *mx = p.max_col.data();
+        for (int J = 0; J <= m >> 3; ++J) {
+            const int first = (int)(std::lower_bound(mx, mx + n + 1, 8 * J) - mx);
+            const int last = (int)(std::upper_bound(mn, mn + n + 1, 8 * J + 7) - mn) - 1;
+            const int q0 = first <= last ? first >> 2 : 1, q1 = first <= last ? last >> 2 : 0;
+            p.blkrows.push_back(make_int4(q0, q1, (int)p.quad_start.size(), 0));
+            for (int q = q0; q <= q1; ++q) {
+                p.quad_start.push_back(entries);
+                for (int i = std::max(4 * q, first); i <= std::min(4 * q + 3, last); ++i)
+                    for (int j = std::max(mn[i], 8 * J), c = p.bandoff[i] + j - mn[i]; j <= std::min(mx[i], 8 * J + 7); ++j, ++c) {
+                        p.cre_start[c] = entries;
+                        p.cre_start[p.bandcells + c] = entries += cnt[c];
+                    }
+            }
+        }
+        p.quad_start.push_back(entries);
+    } else {
+        p.cre_start.assign(p.bandcells + 1, 0);
+        for (int c = 0; c < p.bandcells; ++c) p.cre_start[c + 1] = p.cre_start[c] + cnt[c];
+        entries = p.cre_start[p.bandcells];
+    }
+    std::vector<int> fillp(p.cre_start.begin(), p.cre_start.begin() + p.bandcells);
+    std::vector<int> ord(entries);
     for (int k = 0; k < na; ++k)
         if (cell_of[k] >= 0) ord[fillp[cell_of[k]]++] = k;
     p.cre.resize(4 * ord.size());
@@ -248,7 +281,7 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p)
         return p.am_ends[4 * x + 2] > p.am_ends[4 * y + 2];
     };
     for (int c = 0; c < p.bandcells; ++c) {
-        auto b = ord.begin() + p.cre_start[c], e = ord.begin() + p.cre_start[c + 1];
+        auto b = ord.begin() + p.cre_start[c], e = b + cnt[c];
         if (e - b > 1 && !std::is_sorted(b, e, lex_greater_left)) std::sort(b, e, lex_greater_left);
     }
     // the same candidates per row a.r: a.l descending, then b.l descending
@@ -293,11 +326,12 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p)
         p.rowarc[2 * r + 1] = (int)q;
     }
     for (size_t q = 0; q < ord.size(); ++q) {
-        int k = ord[q];
-        p.cre[4 * q] = p.am_pos[k];                   // D entry
-        p.cre[4 * q + 1] = p.am_ends[4 * k] - 1;      // a.l - 1: row of the inner corner
-        p.cre[4 * q + 2] = p.am_ends[4 * k + 2] - 1;  // b.l - 1: column of the inner corner
-        p.cre[4 * q + 3] = k;                         // the arc match
+        const int k = ord[q], i = p.am_ends[4 * k] - 1, j = p.am_ends[4 * k + 2] - 1;  // inner corner
+        const unsigned cc = in_band(i, j) ? p.bandoff[i] + j - p.min_col[i] : 0;
+        p.cre[4 * q] = p.am_pos[k];  // D entry
+        p.cre[4 * q + 1] = i | (j << 16);
+        p.cre[4 * q + 2] = (int)(cc << 5 | (p.am_ends[4 * k + 1] & 3) << 3 | (p.am_ends[4 * k + 3] & 7));
+        p.cre[4 * q + 3] = k;  // the arc match
     }
     p.num_pos = (int)ordr.size();
 
@@ -403,7 +437,14 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p)
             g.top = 0;
             ks.clear();
             for (size_t q = s; q < e; ++q) ks.push_back(byleft[q].second);
-            auto ar_less = [&](int x, int y) { return p.am_ends[4 * x + 1] < p.am_ends[4 * y + 1]; };
+            // the order in which the group's sweep reaches their corners
+            auto ar_less = [&](int x, int y) {
+                if (lanes) {
+                    const int bx = (p.am_ends[4 * x + 3] - sh - 1) >> 3, by = (p.am_ends[4 * y + 3] - sh - 1) >> 3;
+                    if (bx != by) return bx < by;
+                }
+                return p.am_ends[4 * x + 1] < p.am_ends[4 * y + 1];
+            };
             if (!std::is_sorted(ks.begin(), ks.end(), ar_less)) std::stable_sort(ks.begin(), ks.end(), ar_less);
             for (int k : ks) {
                 // fill_D_entries_noLP: only arc matches with an inner arc
@@ -446,17 +487,51 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p)
                 } else {
                     g.rect_off = (int)p.rect_cells;
                     p.rect_cells += sz;
-                    if (!nolp)
+                    if (!nolp && !lanes)
                         for (size_t q = s; q < e; ++q) p.am_rect[byleft[q].second] = make_int2(g.rect_off, rect_pitch);
                 }
             }
             p.cells += rect_cells(al + 1, max_ar, bl + 1, max_br - 1);
             g.cpl = 1;
+            if (lanes)
+                for (size_t q = s; q < e; ++q) p.am_rect[byleft[q].second].x = (int)p.groups.size();
             p.groups.push_back(g);
             p.rows_max = std::max(p.rows_max, max_ar - al);
             p.width_max = std::max(p.width_max, max_br - bl + 1);
         }
         s = e;
+    }
+    if (lanes) {
+        // items: consecutive groups, and what their sweeps cover
+        for (size_t g0 = 0; g0 < p.groups.size(); g0 += lanes) {
+            LaneItem it{};
+            it.g0 = (int)g0;
+            it.ng = (int)std::min<size_t>(lanes, p.groups.size() - g0);
+            it.a0 = it.b0 = INT_MAX;
+            for (int k = 0; k < it.ng; ++k) {
+                const GroupItem &g = p.groups[g0 + k];
+                it.a0 = std::min(it.a0, g.al);
+                it.amax = std::max(it.amax, g.al);
+                it.a1 = std::max(it.a1, g.ar);
+                it.b0 = std::min(it.b0, g.bl);
+                it.b1 = std::max(it.b1, g.br);
+            }
+            const long long lines = p.bandoff[it.a1] - p.bandoff[it.a0];
+            it.line = (int)p.lane_lines;
+            p.lane_slot = std::max(p.lane_slot, lines);
+            if (p.lane_lines >= 0) p.lane_lines += lines;
+            if (p.lane_lines >= (1ll << 31)) p.lane_lines = -1;
+            p.litems.push_back(it);
+        }
+        for (int k = 0; k < na; ++k) {
+            const int g = p.am_rect[k].x;
+            if (g < 0 || nolp) {
+                p.am_rect[k] = make_int2(0, -1);
+                continue;
+            }
+            const LaneItem &it = p.litems[g / lanes];
+            p.am_rect[k] = make_int2(it.line - p.bandoff[it.a0], g % lanes);
+        }
     }
 #ifdef LCG_TEST_DROP_LAST_D_WRITE
     // test build only (tests/test_zy_wait_timeout.py): the last group's last
@@ -526,6 +601,9 @@ struct Assembler {
     }
 };
 
+// at most this much scratch for the slots of a lane-per-group launch
+constexpr long long LANE_SCRATCH_BYTES = 24ll << 30;
+
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // One buffer set of the engine, by reference: set 0 is the engine's own
@@ -554,7 +632,8 @@ Slot slot_of(lcg_engine e, int k) {
 // byte offsets of one pair's tables in the arena
 struct PairOff {
     size_t sigma, scls, rcls, ccls, gapA, gapB, minc, maxc, bandoff, rowinfo, anc, cre_start, cre, crow, rowarc,
-        am_score, D, topM, res, tok, tq, segs, groups, dw, gbc, dwn, inner, sscore, rect, am_rect;
+        am_score, D, topM, res, tok, tq, segs, groups, dw, gbc, dwn, inner, sscore, rect, am_rect,
+        litems, blkrows, quad_start;
 };
 
 // One chunk of an lcg_align_pairs call: pairs [q0, q0 + nq) of the batch.
@@ -580,6 +659,35 @@ struct Chunk {
     int bps = 0;
     double wave_mb = 0;
 };
+
+// Groups per item of the lane-per-group fill for a chunk, 0: one warp per group
+// (sankoff_fill_kernel). An estimate of the three fill times from the pairs'
+// sizes; the constants are fits to measured fills on a GB300. Matrix cells:
+// 2 (n + m) per arc match within 30 % over 60-500 nt. One warp per group fills
+// 90 cells/ns, lane per group 130 (32 groups) or 170 (64); a lane item of a pair
+// is serial, its longest one takes 2.2 us per quad and 50 ns per arc match, of
+// which a launch ends with three quarters (a third more with 64 groups), and
+// the row sweep of one group a sixth of that. So single pairs and small batches
+// go to one warp per group (one 400 x 400 pair: 3.1 ms against 9.6 ms), batches
+// to lanes (28 profile pairs of 80-300: 5.0 -> 4.6 ms with 32 groups, 5.9 with
+// 64; 66 pairs of 60-300 nt: 8.9 -> 7.3 and 7.2 ms; 276 pairs of 60-400 nt in
+// two chunks: 126 -> 82 and 64 ms).
+int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg_align_opts *opts) {
+    if (e->counting || opts->struct_local) return 0;
+    if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) == 64 ? 64 : std::atoi(v) == 32 ? 32 : 0;
+    double cells = 0, longest = 0;
+    for (int q = 0; q < npairs; ++q) {
+        const lcg_pair_tables &t = pairs[q];
+        if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || !t.min_col || !t.max_col) continue;
+        double band = 0;
+        for (int i = 0; i <= t.len_a; ++i) band += t.max_col[i] - t.min_col[i] + 1;
+        cells += 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
+        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
+    }
+    if (opts->no_lonely_pairs) cells /= 50;  // few arc matches have a stacked partner
+    const double warp = cells / 90 + longest / 6, l32 = cells / 130 + 0.75 * longest, l64 = cells / 170 + longest;
+    return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
+}
 
 // pairs per chunk: one chunk for small batches, else up to 8 chunks of at
 // least 128 pairs (the first chunk's host preparation is not overlapped)
@@ -692,12 +800,13 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         const long long budget = e->rect_budget >= 0 ? e->rect_budget
                                                      : (opts->struct_local ? RECT_BUDGET_SL : RECT_BUDGET_PLAIN);
         keep = budget > 0;
-        long long cells = 0;
+        double bytes = 0;
         for (auto &p : prep) {
-            if (p.rect_cells < 0 || (p.flags & PF_NOLP)) keep = false;
-            cells += p.rect_cells;
+            const bool ln = p.flags & PF_LANES;
+            if ((ln ? p.lane_lines : p.rect_cells) < 0 || (p.flags & PF_NOLP)) keep = false;
+            bytes += ln ? 4.0 * p.lane_groups * (double)p.lane_lines : (double)rect_bytes_per_cell * (double)p.rect_cells;
         }
-        keep = keep && (double)rect_bytes_per_cell * (double)cells <= (double)budget;
+        keep = keep && bytes <= (double)budget;
     }
     c.off.assign(npairs, PairOff{});
     std::vector<PairOff> &off = c.off;
@@ -708,10 +817,21 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         return o;
     };
     size_t off_pairs = take(up, sizeof(PairDev) * npairs);
-    size_t nitems = 0;
-    for (auto &p : prep) nitems += p.groups.size();
-    size_t off_queue = take(up, sizeof(int2) * nitems);  // (pair, group) work items
-    c.off_ctrl = take(up, 64);  // qhead, status, abort, pad, 2 x u64 counters
+    // the pairs filled lane per group and the others, each with a queue of
+    // (pair, item) work items and a launch of its own
+    std::vector<int> of[2];
+    size_t nitems[2] = {0, 0};
+    for (int q = 0; q < npairs; ++q) {
+        const bool ln = prep[q].flags & PF_LANES;
+        of[ln].push_back(q);
+        nitems[ln] += ln ? prep[q].litems.size() + 1 : prep[q].groups.size();
+    }
+    // lane items run long (the outermost ones sweep the whole pair): largest
+    // pairs first, so that the launch ends with short ones
+    std::stable_sort(of[1].begin(), of[1].end(), [&](int x, int y) { return prep[x].cells > prep[y].cells; });
+    const size_t off_queue = take(up, sizeof(int2) * nitems[0]);
+    const size_t off_lqueue = take(up, sizeof(int2) * nitems[1]);
+    c.off_ctrl = take(up, 64);  // qhead, status, abort, pad, 2 x u64 counters, qhead of the lane launch
     const size_t off_ctrl = c.off_ctrl;
     for (int q = 0; q < npairs; ++q) {
         const auto &p = prep[q];
@@ -735,13 +855,16 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         o.bandoff = take(up, 4ull * (p.n + 2));
         o.rowinfo = take(up, 16ull * (p.n + 2));
         o.anc = t.match_lo ? take(up, 4ull * (2 * (p.n + 1) + 2 * (p.n + 1) + 2 * (p.m + 1))) : 0;
-        o.cre_start = take(up, 4ull * (p.bandcells + 1));
+        o.cre_start = take(up, 4ull * p.cre_start.size());
         o.cre = take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
         o.crow = take(up, 4ull * std::max<size_t>(p.crow.size(), 4));
         o.rowarc = take(up, 4ull * p.rowarc.size());
         o.am_score = take(up, 4ull * std::max(t.num_arcmatches, 1));
         o.D = take(up, 4ull * std::max(p.num_pos, 1));
         o.am_rect = keep ? take(up, 8ull * p.am_rect.size()) : 0;
+        o.litems = take(up, sizeof(LaneItem) * p.litems.size());
+        o.blkrows = take(up, sizeof(int4) * p.blkrows.size());
+        o.quad_start = take(up, 4ull * p.quad_start.size());
     }
     c.down_begin = up;
     size_t dn = up;
@@ -760,7 +883,9 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         PairOff &o = off[q];
         o.tq = take(dev_only, 16ull * p.tq_cap);
         o.topM = take(dev_only, 4ull * (p.n + 1) * (p.m + 1));
-        o.rect = keep ? take(dev_only, (size_t)rect_bytes_per_cell * std::max<long long>(p.rect_cells, 1)) : 0;
+        const size_t rect_bytes = (p.flags & PF_LANES) ? 4ull * p.lane_groups * std::max<long long>(p.lane_lines, 1)
+                                                       : (size_t)rect_bytes_per_cell * std::max<long long>(p.rect_cells, 1);
+        o.rect = keep ? take(dev_only, rect_bytes) : 0;
     }
     // normalized / penalized alignment: per pair its penalty, the selected
     // pairs and their gathered result words
@@ -800,11 +925,18 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         // pairs' work lists are interleaved so that every pair progresses
         // proportionally; within a pair the order is kept. Waves follow each
         // other in the queue without a barrier.
-        std::vector<size_t> ng(npairs);
-        for (int q = 0; q < npairs; ++q) ng[q] = prep[q].groups.size();
-        lcg_host::queue_order(
-            ng, [&](int q) { return 12.0 * prep[q].num_pos + 4.0 * prep[q].bandcells; }, (int2 *)(H + off_queue),
-            [](int n, auto fn) { lcg_host::parallel_for(n, fn); }, c.wave_mb * 1048576.0);
+        for (int ln = 0; ln < 2; ++ln) {
+            if (of[ln].empty()) continue;
+            std::vector<size_t> ng;
+            for (int q : of[ln]) ng.push_back(ln ? prep[q].litems.size() + 1 : prep[q].groups.size());
+            int2 *const queue = (int2 *)(H + (ln ? off_lqueue : off_queue));
+            lcg_host::queue_order(
+                ng,
+                [&](int k) { return 12.0 * prep[of[ln][k]].num_pos + 4.0 * prep[of[ln][k]].bandcells; }, queue,
+                [](int n, auto fn) { lcg_host::parallel_for(n, fn); }, c.wave_mb * 1048576.0);
+            if (ln || !of[1].empty())
+                for (size_t k = 0; k < nitems[ln]; ++k) queue[k].x = of[ln][queue[k].x];
+        }
     }
     std::memset(H + off_ctrl, 0, 64);
     lcg_host::parallel_for(npairs, [&](int q) {
@@ -833,7 +965,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             std::memcpy(a + 4 * (p.n + 1), t.ins_lo, 4ull * (p.m + 1));
             std::memcpy(a + 4 * (p.n + 1) + (p.m + 1), t.ins_hi, 4ull * (p.m + 1));
         }
-        std::memcpy(H + o.cre_start, p.cre_start.data(), 4ull * (p.bandcells + 1));
+        std::memcpy(H + o.cre_start, p.cre_start.data(), 4ull * p.cre_start.size());
         if (!p.cre.empty()) std::memcpy(H + o.cre, p.cre.data(), 4ull * p.cre.size());
         if (!p.crow.empty()) std::memcpy(H + o.crow, p.crow.data(), 4ull * p.crow.size());
         std::memcpy(H + o.rowarc, p.rowarc.data(), 4ull * p.rowarc.size());
@@ -889,6 +1021,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             d.ins_hi = a + 4 * (p.n + 1) + (p.m + 1);
         }
         d.cre_start = (const int *)(Dv + o.cre_start);
+        d.cre_end = d.cre_start + ((p.flags & PF_LANES) ? p.bandcells : 1);
         d.cre = (const int4 *)(Dv + o.cre);
         d.crow = (const int2 *)(Dv + o.crow);
         d.num_pos = p.num_pos;
@@ -906,6 +1039,16 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         d.groups = (const GroupItem *)(Dv + o.groups);
         d.rect = keep ? (int *)(Dv + o.rect) : nullptr;
         d.am_rect = keep ? (const int2 *)(Dv + o.am_rect) : nullptr;
+        if (p.flags & PF_LANES) {
+            std::memcpy(H + o.litems, p.litems.data(), sizeof(LaneItem) * p.litems.size());
+            std::memcpy(H + o.blkrows, p.blkrows.data(), sizeof(int4) * p.blkrows.size());
+            std::memcpy(H + o.quad_start, p.quad_start.data(), 4ull * p.quad_start.size());
+            d.quad_start = (const int *)(Dv + o.quad_start);
+            d.litems = (const LaneItem *)(Dv + o.litems);
+            d.nlitems = (int)p.litems.size();
+            d.lane_groups = p.lane_groups;
+            d.blkrows = (const int4 *)(Dv + o.blkrows);
+        }
         d.dw = (const int4 *)(Dv + o.dw);
         d.dwn = p.inner.empty() ? nullptr : (const int2 *)(Dv + o.dwn);
         d.inner = p.inner.empty() ? nullptr : (const int2 *)(Dv + o.inner);
@@ -916,36 +1059,65 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     // ---- scratch
     const bool sl = opts->struct_local != 0;
     const int rb = lcg_host::ring_size(span);
-    bool fast = true, sl_fast = true;
+    bool fast = true, lfast = true, sl_fast = true;
     for (auto &p : prep) {
-        fast = fast && (p.flags & PF_SCLS) && !(p.flags & (PF_ANCHORS | PF_NOLP | PF_STACK));
+        bool &f = (p.flags & PF_LANES) ? lfast : fast;
+        f = f && (p.flags & PF_SCLS) && !(p.flags & (PF_ANCHORS | PF_NOLP | PF_STACK));
         sl_fast = sl_fast && (p.flags & PF_SCLS) && !(p.flags & PF_ANCHORS);
     }
     c.sl_fast = sl_fast;
     c.rb = rb;
-    int blocks_per_sm = 0;
-    if (sl) {
-        CUDA_TRY(sl_prepare(sw, rb, sl_fast, keep, &blocks_per_sm));
-    } else {
-        CUDA_TRY(fill_occupancy(rb, e->counting, fast, &blocks_per_sm));
-        CUDA_TRY(trace_prepare(rb));
-    }
-    if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
-    if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
-    int blocks = e->sms * blocks_per_sm;
     long long stride = (long long)rows_max * sw;
-    // state matrices per slot: fill 1 (plain) / 4 (struct-local); traceback 1 / 8
-    size_t fill_slots = (size_t)blocks * (sl ? sl_fill_warps_per_block() * 4 : fill_warps_per_block());
+    int blocks = 0, lblocks = 0;
+    size_t group_ints = 0, lane_ints = 0;  // scratch of the fill launches
+    int lgroups = 0;
+    long long lslot = 0, lqslot = 0;
+    if (!sl) CUDA_TRY(trace_prepare(rb));
+    if (!of[0].empty()) {
+        int blocks_per_sm = 0;
+        if (sl) CUDA_TRY(sl_prepare(sw, rb, sl_fast, keep, &blocks_per_sm));
+        else CUDA_TRY(fill_occupancy(rb, e->counting, fast, &blocks_per_sm));
+        if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
+        if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
+        blocks = e->sms * blocks_per_sm;
+        // state matrices per slot: 1 (plain) / 4 (struct-local)
+        group_ints = (size_t)blocks * (sl ? sl_fill_warps_per_block() * 4 : fill_warps_per_block()) * (size_t)stride;
+    }
+    if (!of[1].empty()) {
+        int blocks_per_sm = 0, rows = 0;
+        lgroups = prep[of[1][0]].lane_groups;  // one width per chunk
+        for (int q : of[1]) {
+            lslot = std::max(lslot, lgroups * prep[q].lane_slot);
+            rows = std::max(rows, prep[q].n + 1);
+        }
+        if (keep) lslot = 0;
+        lqslot = (long long)lgroups * (rows + 3);
+        CUDA_TRY(lane_occupancy(lgroups, rb, lfast, &blocks_per_sm));
+        if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
+        if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
+        // no more blocks than items, and at most LANE_SCRATCH_BYTES of slots
+        const long long block_ints = lane_warps_per_block() * (lslot + lqslot);
+        long long b = std::min<long long>((long long)e->sms * blocks_per_sm,
+                                          ((long long)nitems[1] + lane_warps_per_block() - 1) / lane_warps_per_block());
+        lblocks = (int)std::max<long long>(1, std::min<long long>(b, LANE_SCRATCH_BYTES / 4 / block_ints));
+        lane_ints = (size_t)lblocks * (size_t)block_ints;
+    }
     size_t trace_slots = (size_t)npairs * (sl ? 8 : 1);
-    size_t need = std::max(fill_slots, trace_slots) * (size_t)stride;
-    if (need > *s.scratch_cap) {
+    auto scratch_need = [&]() { return std::max({group_ints, lane_ints, trace_slots * (size_t)stride}); };
+    if (scratch_need() > *s.scratch_cap) {
         s.graph->release();
         if (*s.d_scratch) cudaFree(*s.d_scratch);
         *s.d_scratch = nullptr;
         *s.scratch_cap = 0;
-        if (cudaMalloc(s.d_scratch, need * sizeof(int)) != cudaSuccess)
-            return fail(LCG_ERR_NOMEM, "device scratch allocation failed");
-        *s.scratch_cap = need;
+        // with little memory left, a lane launch takes fewer warps
+        while (cudaMalloc(s.d_scratch, scratch_need() * sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();
+            *s.d_scratch = nullptr;
+            if (lblocks <= 1) return fail(LCG_ERR_NOMEM, "device scratch allocation failed");
+            lblocks /= 2;
+            lane_ints /= 2;
+        }
+        *s.scratch_cap = scratch_need();
     }
     int *scratch = *s.d_scratch;
 
@@ -959,12 +1131,13 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     std::vector<long long> key;
     if (use_graph) {
         key = {(long long)(uintptr_t)Dv, (long long)(uintptr_t)H, (long long)(uintptr_t)scratch, (long long)down_begin,
-               (long long)down_end, (long long)off_ctrl, (long long)off_pairs, (long long)off_queue, (long long)nitems,
-               blocks, sw, rb, stride, fast, e->counting, sl, sl_fast, keep, opts->do_trace, npairs};
+               (long long)down_end, (long long)off_ctrl, (long long)off_pairs, (long long)off_queue, (long long)nitems[0],
+               blocks, sw, rb, stride, fast, e->counting, sl, sl_fast, keep, opts->do_trace, npairs,
+               (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lfast, lgroups};
         if (s.graph->exec && s.graph->key == key) {
             CUDA_TRY(cudaGraphLaunch(s.graph->exec, st));
             ++e->last_graph_replays;
-            c.launches = opts->do_trace ? 2 : 1;
+            c.launches = !of[0].empty() + !of[1].empty() + (opts->do_trace ? 1 : 0);
             c.off_pairs = off_pairs;
             c.off_mod = off_mod;
             c.sw = sw;
@@ -1007,21 +1180,29 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     int *abort_flag = (int *)(Dv + off_ctrl + 8);
     CUDA_TRY_CAP(record(s.ev0));
     unsigned long long *counters = e->counting ? (unsigned long long *)(Dv + off_ctrl + 16) : nullptr;
+    c.launches = 0;
+    if (!of[1].empty()) {
+        CUDA_TRY_CAP(launch_lane_fill(lgroups, (const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_lqueue),
+                                      (int)nitems[1], scratch, lslot, lqslot, rb, lfast,
+                                      (unsigned int *)(Dv + off_ctrl + 32), status, abort_flag, lblocks, st));
+        ++c.launches;
+    }
     if (sl) {
         if (counters) {
             end_capture();
             return fail(LCG_ERR_UNSUPPORTED, "work counting covers the plain mode only");
         }
         CUDA_TRY_CAP(launch_sl_fill((const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_queue),
-                                (int)nitems, scratch, stride, sw, rb, sl_fast, keep, qhead,
+                                (int)nitems[0], scratch, stride, sw, rb, sl_fast, keep, qhead,
                                 status, abort_flag, blocks, st));
-    } else {
+        ++c.launches;
+    } else if (!of[0].empty()) {
         CUDA_TRY_CAP(launch_fill((const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_queue),
-                             (int)nitems, scratch, stride, sw, rb, fast, qhead,
+                             (int)nitems[0], scratch, stride, sw, rb, fast, qhead,
                              status, abort_flag, blocks, st, counters));
+        ++c.launches;
     }
     CUDA_TRY_CAP(record(s.ev1));
-    c.launches = 1;
     TraceSel sel;
     if (modv) {
         lcg_status ms = mod_top_levels(opts, c, (const PairDev *)(Dv + off_pairs), (int *)(Dv + off_mod), npairs,
@@ -1378,7 +1559,8 @@ static lcg_status align_impl(lcg_engine e, const lcg_pair_tables *pairs, int32_t
         }
         next.clear();
         next.resize(nq);
-        lcg_host::parallel_for(nq, [&](int q) { prep_pair(pairs[q0 + q], *opts, next[q]); });
+        const int lanes = lane_width(e, pairs + q0, nq, opts);
+        lcg_host::parallel_for(nq, [&](int q) { prep_pair(pairs[q0 + q], *opts, next[q], lanes); });
         t_prep += ms_between(a, clk::now());
         for (int q = 0; q < nq && rc == LCG_OK; ++q)
             if (next[q].code != LCG_OK)
@@ -1577,7 +1759,8 @@ lcg_status lcg_align_kbest(lcg_engine e, const lcg_pair_tables *pairs, int32_t n
     c.nq = npairs;
     c.kbest = true;
     c.prep.resize(npairs);
-    lcg_host::parallel_for(npairs, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q]); });
+    const int lanes = lane_width(e, pairs, npairs, opts);
+    lcg_host::parallel_for(npairs, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q], lanes); });
     for (int q = 0; q < npairs; ++q)
         if (c.prep[q].code != LCG_OK) return fail(c.prep[q].code, "pair " + std::to_string(q) + ": " + c.prep[q].err);
     const Slot sl0 = slot_of(e, 0);

@@ -23,8 +23,8 @@ struct Prep {
     std::vector<int4> rowinfo;                   // n+2
     int maxband = 0;
     int span = 2;  // max over i of max_col[i+1] - min_col[i] + 3 (ring rows of the kernels)
-    std::vector<int> cre_start;                  // bandcells+1
-    std::vector<int> cre;                        // 4 per entry: D position, a.l-1, b.l-1, am
+    std::vector<int> cre_start;                  // bandcells+1; with PF_LANES the starts, then the ends
+    std::vector<int> cre;                        // 4 per entry (PairDev::cre)
     std::vector<int> crow;                       // 2 per entry by row a.r, a.l desc, b.l desc:
                                                  //   (a.l-1) | (b.l-1) << 16, b.r
     std::vector<int> rowarc;                     // 2 per row 0..n+1: [start, end) in crow
@@ -49,6 +49,14 @@ struct Prep {
     // (rect_off, pitch) or (-1, 0); rect_cells = -1: too large to keep
     long long rect_cells = 0;
     std::vector<int2> am_rect;
+    // pairs filled lane per group (PF_LANES in flags): PairDev::litems,
+    // blkrows and quad_start, the lines of one item's storage at most and of all (-1: too
+    // many to keep); am_rect then holds (line of band cell 0, lane) or (0, -1)
+    std::vector<lcg::LaneItem> litems;
+    std::vector<int4> blkrows;
+    std::vector<int> quad_start;
+    int lane_groups = 0;
+    long long lane_slot = 0, lane_lines = 0;
     int token_cap = 0, tq_cap = 0;
     long long cells = 0;                         // M cells of all groups + top level
     std::string err;
@@ -56,8 +64,9 @@ struct Prep {
 };
 
 // Validate one pair's tables and build its derived structures; on error
-// p.code / p.err describe it.
-lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p);
+// p.code / p.err describe it. lanes: groups per item of the
+// lane-per-group fill where the pair allows it (then p.flags has PF_LANES), 0: none.
+lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes = 0);
 
 void set_error(const std::string &msg);
 

@@ -32,6 +32,7 @@ enum PairFlags : int {
     PF_SCLS = 16,  // sigma(i,j) = scls[rcls[i] * 16 + ccls[j]] (at most 16 row / column classes)
     PF_NOLP = 32,  // no lonely pairs (AlignerParams::no_lonely_pairs)
     PF_STACK = 64, // stacking terms (Scoring::stacking())
+    PF_LANES = 128,  // filled lane per group
 };
 
 // status word bits (device -> host)
@@ -42,6 +43,16 @@ enum StatusBits : int {
 };
 
 struct GroupItem;
+
+// Work item of the lane-per-group fill: up to 32 or 64
+// (PairDev::lane_groups) consecutive left-end groups
+// of a pair (PairDev::groups[g0 .. g0 + ng)) and what their sweeps cover
+struct LaneItem {
+    int g0, ng;
+    int a0, amax, a1;  // smallest and largest left end of A, largest right end
+    int b0, b1;        // smallest left end and largest right end of B
+    int line;          // first line (lane_groups ints) of its kept storage in PairDev::rect
+};
 
 struct PairDev {
     int n, m;
@@ -65,8 +76,12 @@ struct PairDev {
     const int *bandoff;   // n+2: band cell offset of row i
     const int4 *rowinfo;  // n+2: (min_col, max_col, gapA, bandoff) of row i
     const int *match_lo, *match_hi, *del_lo, *del_hi, *ins_lo, *ins_hi;
-    const int *cre_start; // bandcells+1: arc matches with right ends at a band cell
-    const int4 *cre;      // (D index, a.l-1, b.l-1, am), lex-greater-left-ends order
+    const int *cre_start, *cre_end;  // bandcells: the entries of cre with right ends at a band cell
+    // the arc matches by band cell of their right ends, lex-greater-left-ends
+    // order: (D index, (a.l-1) | (b.l-1) << 16, band cell of the inner corner
+    // (a.l-1, b.l-1) << 5 | (a.r & 3) << 3 | b.r & 7, am); a corner outside the
+    // band has cell 0 (the third word is for pairs with PF_LANES)
+    const int4 *cre;
     const int2 *crow;     // the same arc matches by row a.r, then a.l descending, b.l descending:
                           // ((a.l-1) | (b.l-1) << 16, b.r); the position is the D index
     const int2 *rowarc;   // n+2: [start, end) of row i's entries in crow
@@ -105,6 +120,19 @@ struct PairDev {
     // group computes it.
     int *rect;
     const int2 *am_rect;
+    // PF_LANES: the pair's D is filled lane per group (sankoff_lane_kernels.cu):
+    // its work items, and per block of 8 columns the first and last quad of 4
+    // rows whose bands meet it and the index of its first quad. A kept rectangle is then the item's storage,
+    // one line of lane_groups ints per band cell, and am_rect holds per arc
+    // match (line of band cell 0, place of the group) or (0, -1); the D writes of a group are
+    // ordered by column block, then row.
+    // cre is then ordered by quad: block J's quads q = blkrows[J].x .. .y hold
+    // the entries quad_start[k] to quad_start[k + 1], k = blkrows[J].z + q -
+    // blkrows[J].x, rows and columns ascending.
+    const LaneItem *litems;
+    int nlitems, lane_groups;
+    const int4 *blkrows;
+    const int *quad_start;
 };
 
 // Scoring::basematch(i,j) from the class table or the dense table

@@ -207,6 +207,7 @@ extern "C" lcg_status lcg_align_score_static(const lcg_pair_tables *pair, const 
         d.ins_hi = a + 4 * (n + 1) + (m + 1);
     }
     d.cre_start = (const int *)(base + o_cs);
+    d.cre_end = d.cre_start + 1;
     d.cre = (const int4 *)(base + o_cre);
     d.crow = (const int2 *)(base + o_crow);
     d.num_pos = p.num_pos;

@@ -687,7 +687,9 @@ static __device__ __noinline__ bool trace_stack(Walker &w, int k, int kpos, int4
 // Mg (pitch), emitting tokens in reverse append order. Arc-match tokens are
 // (-2, am); each traced arc match is queued for its own walk. On the top level
 // (tl) lam is the penalty of the modified scoring view of normalized and
-// penalized alignment (0 otherwise).
+// penalized alignment (0 otherwise). LANE: the rectangle is a lane of a kept
+// item storage (PF_LANES): Mg + lane_groups c holds band cell c.
+template <bool LANE = false>
 static __device__ __noinline__ void walk(Walker &w, const int *Mg, int pitch, int al, int bl, int i, int j, bool tl,
                      int *status, int lam = 0) {
     const PairDev &P = w.P;
@@ -695,7 +697,8 @@ static __device__ __noinline__ void walk(Walker &w, const int *Mg, int pitch, in
     const bool local = P.flags & PF_SEQU_LOCAL;
     const int fe = P.free_endgaps;
     const int go = P.go;
-#define MM(x, y) Mg[(size_t)((x) - al) * pitch + ((y) - bl)]
+#define MM(x, y) \
+    Mg[LANE ? (long long)(P.bandoff[x] - P.min_col[x] + (y)) * P.lane_groups : (long long)((x) - al) * pitch + ((y) - bl)]
     for (int guard = 0; guard < 4 * (P.n + P.m + 4); ++guard) {
         const int Mij = MM(i, j);
         if (tl && local && Mij == 0) {
@@ -760,10 +763,10 @@ static __device__ __noinline__ void walk(Walker &w, const int *Mg, int pitch, in
         }
         if (!(a_match(P, i, j) && w.valid(i - 1, j - 1))) return;
         const int cell = P.bandoff[i] + j - P.min_col[i];
-        for (int q = P.cre_start[cell]; q < P.cre_start[cell + 1]; ++q) {
+        for (int q = P.cre_start[cell]; q < P.cre_end[cell]; ++q) {
             const int4 ent = P.cre[q];
-            const int alq = ent.y + 1, blq = ent.z + 1;
-            if (alq <= al || blq <= bl) continue;
+            const int alq = (ent.y & 0xffff) + 1, blq = (ent.y >> 16) + 1;
+            if (alq <= al || blq <= bl || !w.valid(alq - 1, blq - 1)) continue;
             if (Mij == MM(alq - 1, blq - 1) + P.D[ent.x] - tlam * ((i - alq + 1) + (j - blq + 1))) {
                 w.emit(i, j);
                 w.emit(-2, ent.w);

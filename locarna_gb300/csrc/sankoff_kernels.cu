@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
             P.res[R_MINJ] = 1;
         }
         const int sA = sel.rst ? sel.rst[pair].x : 1, sB = sel.rst ? sel.rst[pair].y : 1;
-        walk(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), P.m + 1, sA - 1, sB - 1, P.res[R_MAXI],
+        walk<false>(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), P.m + 1, sA - 1, sB - 1, P.res[R_MAXI],
              P.res[R_MAXJ], true, status, lam);
         P.segs[nseg++] = make_int4(-1, 0, w.ntok, 0);
     }
@@ -124,11 +124,13 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         }
         // the arc match's rectangle: its group's kept one from the fill, else
         // recomputed into the pair's scratch slot
-        const int2 kr = P.am_rect ? P.am_rect[k] : make_int2(-1, 0);
+        const bool lanes = P.flags & PF_LANES;
+        const int2 kr = P.am_rect ? P.am_rect[k] : make_int2(-1, -1);
+        const bool kept = P.am_rect && (lanes ? kr.y >= 0 : kr.x >= 0);
         const int *Mw = Mg;
         int pw = sw;
-        if (kr.x >= 0) {
-            Mw = P.rect + kr.x;
+        if (kept) {
+            Mw = lanes ? P.rect + ((long long)kr.x * P.lane_groups + kr.y) : P.rect + kr.x;
             pw = kr.y;
         } else {
             const int cpl = min(4, max(1, (min(ends.w - ends.z, P.maxband) + 31) / 32));
@@ -138,7 +140,8 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         __syncwarp();
         if (lane == 0) {
             const int start = w.ntok;
-            walk(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
+            if (kept && lanes) walk<true>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
+            else walk<false>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
             if (nseg < P.tq_cap + 1) P.segs[nseg] = make_int4(k, start, w.ntok, 0);
             ++nseg;
         }

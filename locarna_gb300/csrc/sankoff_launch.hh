@@ -13,6 +13,15 @@ namespace lcg {
 cudaError_t launch_fill(const PairDev *pairs, const int2 *queue, int nitems, int *scratch,
                         long long scratch_stride, int sw, int rb, bool fast, unsigned int *qhead, int *status,
                         int *abort_flag, int blocks, cudaStream_t st, unsigned long long *counters);
+// the lane-per-group fill (pairs with PF_LANES); queue: (pair, lane item)
+// work items, item nlitems = the top level; per warp `slot` ints of matrix
+// storage (0 with kept rectangles) and `qslot` ints of gap states in scratch
+// groups: groups per item, 32 or 64 (PairDev::lane_groups)
+cudaError_t launch_lane_fill(int groups, const PairDev *pairs, const int2 *queue, int nitems, int *scratch,
+                             long long slot, long long qslot, int rb, bool fast, unsigned int *qhead, int *status,
+                             int *abort_flag, int blocks, cudaStream_t st);
+cudaError_t lane_occupancy(int groups, int rb, bool fast, int *blocks_per_sm);
+int lane_warps_per_block();
 cudaError_t launch_trace(const PairDev *pairs, int npairs, int *scratch, long long scratch_stride, int sw, int rb,
                          int *status, cudaStream_t st, TraceSel sel = TraceSel());
 // the top level of the selected pairs under the scoring modified by lam[pair]

@@ -182,10 +182,10 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
                 gb = P.gapB[j];
                 if (mok) {
                     const int cell = cell0 + j;
-                    const int q1 = P.cre_start[cell + 1];
+                    const int q1 = P.cre_end[cell];
                     for (int q = P.cre_start[cell]; q < q1; ++q) {
                         const int4 ent = P.cre[q];
-                        const int alq = ent.y + 1, blq = ent.z + 1;
+                        const int alq = (ent.y & 0xffff) + 1, blq = (ent.y >> 16) + 1;
                         if (alq <= al) break;
                         if (blq <= bl) continue;
                         const int dv = WAIT ? wait_D(P.D, ent.x, status, abort_flag) : P.D[ent.x];
@@ -811,10 +811,10 @@ static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long 
         }
         if (!(a_match(P, i, j) && w.valid(i - 1, j - 1))) return;
         const int cell = P.bandoff[i] + j - P.min_col[i];
-        for (int q = P.cre_start[cell]; q < P.cre_start[cell + 1]; ++q) {
+        for (int q = P.cre_start[cell]; q < P.cre_end[cell]; ++q) {
             const int4 ent = P.cre[q];
-            const int alq = ent.y + 1, blq = ent.z + 1;
-            if (alq <= al || blq <= bl) continue;
+            const int alq = (ent.y & 0xffff) + 1, blq = (ent.y >> 16) + 1;
+            if (alq <= al || blq <= bl || !w.valid(alq - 1, blq - 1)) continue;
             if (Mij == MS(state, alq - 1, blq - 1) + P.D[ent.x] - tlam * ((i - alq + 1) + (j - blq + 1))) {
                 w.emit(i, j);
                 w.emit(-2, ent.w);
