@@ -276,7 +276,8 @@ lcg_status lcg_engine_set_autotune(lcg_engine eng, int32_t on);
 
 /* Device time (ms) of the last lcg_align_pairs call's kernels (summed over its
  * chunks, whose kernels may overlap on the two streams), and the number of
- * kernel launches it made. */
+ * fill, top-level and traceback launches it made (the two that make a larger
+ * chunk's index structures are in the time, not in the number). */
 lcg_status lcg_engine_last_stats(lcg_engine eng, double *kernel_ms,
                                  int64_t *launches);
 

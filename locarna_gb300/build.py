@@ -27,7 +27,7 @@ GENCODE = "-gencode=arch=compute_103a,code=sm_103a"
 # tuning defines for the CUDA sources, e.g. LCG_NVCC_DEFS="-DLCG_FILL_WARPS=4"
 EXTRA_DEFS = os.environ.get("LCG_NVCC_DEFS", "").split()
 
-CUDA_SOURCES = ["engine.cu", "sankoff_kernels.cu", "sankoff_lane_kernels.cu", "sankoff_sl_kernels.cu", "noalloc.cu",
+CUDA_SOURCES = ["engine.cu", "index_kernels.cu", "sankoff_kernels.cu", "sankoff_lane_kernels.cu", "sankoff_sl_kernels.cu", "noalloc.cu",
                 "pf_kernels.cu", "engine_pf.cu", "envelope.cu"]
 PROBE_SOURCE = "microbench.cu"  # the measurement probe, a library of its own
 HOST_SOURCES = ["host_prep.cpp"]  # C++ host-only translation units

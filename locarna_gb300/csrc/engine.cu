@@ -22,6 +22,7 @@
 #include "lcg_device.cuh"
 #include "engine_prep.hh"
 #include "engine_state.hh"
+#include "index_device.cuh"
 
 #include "sankoff_launch.hh"
 
@@ -55,12 +56,121 @@ inline bool allowed_match(const lcg_pair_tables &t, int i, int j) {
     return !t.match_lo || (t.match_lo[i] <= j && j <= t.match_hi[i]);
 }
 
+// The host's part of the index structures when the device makes the rest: one
+// pass over the arc matches that gives the arc matches per band cell (cnt) and
+// row, and per left-end group its extent and number of D writes, in dependency
+// order. It takes arcs and arc matches in the order in which ArcMatches has
+// them: arcs by left end descending, then right end ascending, arc matches by
+// arc of A, then arc of B; false for any other order (or an index out of
+// range), which the host path then takes (or reports).
+static bool scan_arc_matches(const lcg_pair_tables &t, Prep &p, std::vector<int> &cnt,
+                             std::vector<GroupItem> &groups) {
+    const int n = p.n, m = p.m, na = t.num_arcmatches, aa = t.num_arcs_a, ab = t.num_arcs_b;
+    const bool stack = t.am_stack_score != nullptr;
+    for (int w = 0; w < 2; ++w) {
+        const int32_t *arcs = w ? t.arcs_b : t.arcs_a;
+        for (int k = 1; k < (w ? ab : aa); ++k)
+            if (arcs[2 * k] > arcs[2 * k - 2] || (arcs[2 * k] == arcs[2 * k - 2] && arcs[2 * k + 1] <= arcs[2 * k - 1]))
+                return false;
+    }
+    auto in_band = [&](int i, int j) { return p.min_col[i] <= j && j <= p.max_col[i]; };
+    p.arcs4.resize(aa);
+    p.am_lr.resize(na);
+    p.row_start.assign(n + 2, 0);
+    p.rowarc.assign(2 * (size_t)(n + 2), 0);
+    std::vector<int> rows(n + 2, 0);                          // arc matches with right ends in the band, by row
+    std::vector<int> gar(m + 2, 0), gbr(m + 2, 0), gdw(m + 2, 0);  // the current left end's groups, by bl
+    int k = 0;
+    for (int a0 = 0; a0 < aa;) {
+        const int al = t.arcs_a[2 * a0], kfirst = k;
+        int a = a0;
+        for (; a < aa && t.arcs_a[2 * a] == al; ++a) {
+            const int ar = t.arcs_a[2 * a + 1];
+            const int lo = p.min_col[ar], hi = p.max_col[ar], lo1 = p.min_col[ar - 1], hi1 = p.max_col[ar - 1];
+            int *const row = cnt.data() + p.bandoff[ar] - lo;
+            const int k0 = k;
+            int in = 0, last = -1;
+            for (; k < na && t.am_arcs[2 * k] == a; ++k) {
+                const int b = t.am_arcs[2 * k + 1];
+                if (b <= last || b >= ab) return false;
+                last = b;
+                const int bl = t.arcs_b[2 * b], br = t.arcs_b[2 * b + 1];
+                p.am_lr[k] = bl | (br << 16);
+                gar[bl] = ar;  // (right ends ascend)
+                gbr[bl] = std::max(gbr[bl], br);
+                if (br >= lo && br <= hi) {
+                    ++row[br];
+                    ++in;
+                    if (br - 1 >= lo1 && br - 1 <= hi1) ++gdw[bl];  // the corner (ar-1, br-1) is computed
+                }
+            }
+            p.arcs4[a] = make_int4(al, ar, k0, k);
+            rows[ar] += in;
+            p.row_start[ar + 1]++;
+        }
+        // the left end's groups, bl descending
+        const int g0 = (int)groups.size();
+        if (k > kfirst) {
+            const int lo = p.min_col[al], hi = p.max_col[al];
+            for (int bl = m; bl >= 1; --bl) {
+                if (!gar[bl]) continue;
+                if (bl >= lo && bl <= hi && allowed_match(t, al, bl) && in_band(al - 1, bl - 1)) {
+                    GroupItem g{};
+                    g.al = al;
+                    g.ar = gar[bl];
+                    g.bl = bl;
+                    g.br = gbr[bl];
+                    g.dw_start = p.num_dw;
+                    g.dw_count = gdw[bl];
+                    p.num_dw += gdw[bl];
+                    groups.push_back(g);
+                }
+                gar[bl] = gbr[bl] = gdw[bl] = 0;
+            }
+        }
+        p.lefts.push_back(make_int4(a0, a, g0, (int)groups.size()));
+        a0 = a;
+    }
+    if (k != na) return false;  // an arc of A out of order or out of range
+    for (int i = 0; i <= n; ++i) p.row_start[i + 1] += p.row_start[i];
+    p.row_arcs.resize(aa);
+    std::vector<int> at(p.row_start.begin(), p.row_start.end() - 1);
+    for (int a = 0; a < aa; ++a) p.row_arcs[at[t.arcs_a[2 * a + 1]]++] = a;
+    for (int r = 0, q = 0; r <= n + 1; ++r) {
+        p.rowarc[2 * r] = q;
+        if (r <= n) q += rows[r];
+        p.rowarc[2 * r + 1] = q;
+    }
+    if (stack) {
+        p.am_b.resize(na);
+        for (int q = 0; q < na; ++q) p.am_b[q] = t.am_arcs[2 * q + 1];
+        for (int w = 0; w < 2; ++w) {
+            const int32_t *arcs = w ? t.arcs_b : t.arcs_a;
+            const int num = w ? ab : aa;
+            std::vector<int> &inner = w ? p.inner_b : p.inner_a;
+            inner.assign(num, -1);
+            for (int q = 0; q < num; ++q) {
+                const int l = arcs[2 * q] + 1, r = arcs[2 * q + 1] - 1;
+                int x = 0, y = num;  // the first arc not before (l, r)
+                while (x < y) {
+                    const int c = (x + y) / 2;
+                    if (arcs[2 * c] > l || (arcs[2 * c] == l && arcs[2 * c + 1] < r)) x = c + 1;
+                    else y = c;
+                }
+                if (x < num && arcs[2 * x] == l && arcs[2 * x + 1] == r) inner[q] = x;
+            }
+        }
+    }
+    return true;
+}
+
 // Limits of the lane-per-group fill: the shared-memory rows of its top-level
 // items (span), and 80 MB of matrix storage per warp
 constexpr int LANE_MAX_SPAN = 640;
 constexpr int LANE_MAX_BANDCELLS = 600000;
 
-lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes) {
+lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes,
+                     bool device_index) {
     auto bad = [&](lcg_status c, const std::string &s) {
         p.code = c;
         p.err = s;
@@ -216,26 +326,38 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
         if (l < 1 || r > m || r - l < 3) return bad(LCG_ERR_ARG, "arc of B out of range (1 <= l, l+3 <= r <= len)");
     }
     const int na = t.num_arcmatches;
-    p.am_ends.resize(4 * (size_t)na);
-    for (int k = 0; k < na; ++k) {
-        int a = t.am_arcs[2 * k], b = t.am_arcs[2 * k + 1];
-        if (a < 0 || a >= t.num_arcs_a || b < 0 || b >= t.num_arcs_b) return bad(LCG_ERR_ARG, "arc match index out of range");
-        p.am_ends[4 * k] = t.arcs_a[2 * a];
-        p.am_ends[4 * k + 1] = t.arcs_a[2 * a + 1];
-        p.am_ends[4 * k + 2] = t.arcs_b[2 * b];
-        p.am_ends[4 * k + 3] = t.arcs_b[2 * b + 1];
-    }
     auto in_band = [&](int i, int j) { return i >= 0 && i <= n && p.min_col[i] <= j && j <= p.max_col[i]; };
 
-    // common right end lists over band cells, lex greater left ends
-    // (arc_matches.cc:76-110, arc_matches.hh:188-220)
-    std::vector<int> cnt(p.bandcells + 1, 0);
-    std::vector<int> cell_of(na, -1);
-    for (int k = 0; k < na; ++k) {
-        int ar = p.am_ends[4 * k + 1], br = p.am_ends[4 * k + 3];
-        if (in_band(ar, br)) {
-            cell_of[k] = p.bandoff[ar] + br - p.min_col[ar];
-            cnt[cell_of[k]]++;
+    std::vector<int> cnt(p.bandcells + 1, 0);  // arc matches per band cell of their right ends
+    std::vector<GroupItem> groups;             // of the device path: ends and D-write counts
+#ifdef LCG_TEST_DROP_LAST_D_WRITE
+    device_index = false;
+#endif
+    p.device_index = device_index && !nolp && scan_arc_matches(t, p, cnt, groups);
+    if (!p.device_index) {
+        std::fill(cnt.begin(), cnt.end(), 0);
+        groups.clear();
+    }
+    std::vector<int> cell_of;
+    if (!p.device_index) {
+        p.am_ends.resize(4 * (size_t)na);
+        for (int k = 0; k < na; ++k) {
+            int a = t.am_arcs[2 * k], b = t.am_arcs[2 * k + 1];
+            if (a < 0 || a >= t.num_arcs_a || b < 0 || b >= t.num_arcs_b) return bad(LCG_ERR_ARG, "arc match index out of range");
+            p.am_ends[4 * k] = t.arcs_a[2 * a];
+            p.am_ends[4 * k + 1] = t.arcs_a[2 * a + 1];
+            p.am_ends[4 * k + 2] = t.arcs_b[2 * b];
+            p.am_ends[4 * k + 3] = t.arcs_b[2 * b + 1];
+        }
+        // common right end lists over band cells, lex greater left ends
+        // (arc_matches.cc:76-110, arc_matches.hh:188-220)
+        cell_of.assign(na, -1);
+        for (int k = 0; k < na; ++k) {
+            int ar = p.am_ends[4 * k + 1], br = p.am_ends[4 * k + 3];
+            if (in_band(ar, br)) {
+                cell_of[k] = p.bandoff[ar] + br - p.min_col[ar];
+                cnt[cell_of[k]]++;
+            }
         }
     }
     if (o.struct_local || anchors || t.indel_opening > 0 || p.span > LANE_MAX_SPAN || p.bandcells > LANE_MAX_BANDCELLS)
@@ -268,78 +390,80 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
         for (int c = 0; c < p.bandcells; ++c) p.cre_start[c + 1] = p.cre_start[c] + cnt[c];
         entries = p.cre_start[p.bandcells];
     }
-    std::vector<int> fillp(p.cre_start.begin(), p.cre_start.begin() + p.bandcells);
-    std::vector<int> ord(entries);
-    for (int k = 0; k < na; ++k)
-        if (cell_of[k] >= 0) ord[fillp[cell_of[k]]++] = k;
-    p.cre.resize(4 * ord.size());
-    // (arc matches in the reference's index order come per cell already in
-    // this order; sort only where they do not)
-    auto lex_greater_left = [&](int x, int y) {
-        int alx = p.am_ends[4 * x], aly = p.am_ends[4 * y];
-        if (alx != aly) return alx > aly;
-        return p.am_ends[4 * x + 2] > p.am_ends[4 * y + 2];
-    };
-    for (int c = 0; c < p.bandcells; ++c) {
-        auto b = ord.begin() + p.cre_start[c], e = b + cnt[c];
-        if (e - b > 1 && !std::is_sorted(b, e, lex_greater_left)) std::sort(b, e, lex_greater_left);
-    }
-    // the same candidates per row a.r: a.l descending, then b.l descending
-    // (within a row, the valid ones for a group (al,bl) with a.l > al are a
-    // prefix). The position of an arc match in this order is also the index
-    // of its D entry, so a row's D values are contiguous.
-    // bucket by a.r (counting sort of the arc matches in index order), then
-    // order each row where the index order does not already give it
-    std::vector<int> ordr(ord.size());
-    {
-        std::vector<int> rstart(n + 2, 0);
+    p.num_pos = entries;
+    if (!p.device_index) {
+        std::vector<int> fillp(p.cre_start.begin(), p.cre_start.begin() + p.bandcells);
+        std::vector<int> ord(entries);
         for (int k = 0; k < na; ++k)
-            if (cell_of[k] >= 0) rstart[p.am_ends[4 * k + 1] + 1]++;
-        for (int r = 0; r <= n; ++r) rstart[r + 1] += rstart[r];
-        std::vector<int> fill(rstart.begin(), rstart.end() - 1);
-        for (int k = 0; k < na; ++k)
-            if (cell_of[k] >= 0) ordr[fill[p.am_ends[4 * k + 1]]++] = k;
-        auto row_less = [&](int x, int y) {
-            const int *ex = &p.am_ends[4 * x], *ey = &p.am_ends[4 * y];
-            if (ex[0] != ey[0]) return ex[0] > ey[0];
-            if (ex[2] != ey[2]) return ex[2] > ey[2];
-            return ex[3] < ey[3];
+            if (cell_of[k] >= 0) ord[fillp[cell_of[k]]++] = k;
+        p.cre.resize(4 * ord.size());
+        // (arc matches in the reference's index order come per cell already in
+        // this order; sort only where they do not)
+        auto lex_greater_left = [&](int x, int y) {
+            int alx = p.am_ends[4 * x], aly = p.am_ends[4 * y];
+            if (alx != aly) return alx > aly;
+            return p.am_ends[4 * x + 2] > p.am_ends[4 * y + 2];
         };
-        for (int r = 0; r <= n; ++r) {
-            auto b = ordr.begin() + rstart[r], e = ordr.begin() + rstart[r + 1];
-            if (e - b > 1 && !std::is_sorted(b, e, row_less)) std::sort(b, e, row_less);
+        for (int c = 0; c < p.bandcells; ++c) {
+            auto b = ord.begin() + p.cre_start[c], e = b + cnt[c];
+            if (e - b > 1 && !std::is_sorted(b, e, lex_greater_left)) std::sort(b, e, lex_greater_left);
+        }
+        // the same candidates per row a.r: a.l descending, then b.l descending
+        // (within a row, the valid ones for a group (al,bl) with a.l > al are a
+        // prefix). The position of an arc match in this order is also the index
+        // of its D entry, so a row's D values are contiguous.
+        // bucket by a.r (counting sort of the arc matches in index order), then
+        // order each row where the index order does not already give it
+        std::vector<int> ordr(ord.size());
+        {
+            std::vector<int> rstart(n + 2, 0);
+            for (int k = 0; k < na; ++k)
+                if (cell_of[k] >= 0) rstart[p.am_ends[4 * k + 1] + 1]++;
+            for (int r = 0; r <= n; ++r) rstart[r + 1] += rstart[r];
+            std::vector<int> fill(rstart.begin(), rstart.end() - 1);
+            for (int k = 0; k < na; ++k)
+                if (cell_of[k] >= 0) ordr[fill[p.am_ends[4 * k + 1]]++] = k;
+            auto row_less = [&](int x, int y) {
+                const int *ex = &p.am_ends[4 * x], *ey = &p.am_ends[4 * y];
+                if (ex[0] != ey[0]) return ex[0] > ey[0];
+                if (ex[2] != ey[2]) return ex[2] > ey[2];
+                return ex[3] < ey[3];
+            };
+            for (int r = 0; r <= n; ++r) {
+                auto b = ordr.begin() + rstart[r], e = ordr.begin() + rstart[r + 1];
+                if (e - b > 1 && !std::is_sorted(b, e, row_less)) std::sort(b, e, row_less);
+            }
+        }
+        p.am_pos.assign(na, -1);
+        p.crow.resize(2 * ordr.size());
+        p.rowarc.assign(2 * (size_t)(n + 2), 0);
+        for (size_t q = 0; q < ordr.size(); ++q) {
+            int k = ordr[q];
+            p.am_pos[k] = (int)q;
+            // (a.l-1) | (b.l-1) << 16: the inner corner; positions are < 2^15
+            p.crow[2 * q] = (p.am_ends[4 * k] - 1) | ((p.am_ends[4 * k + 2] - 1) << 16);
+            p.crow[2 * q + 1] = p.am_ends[4 * k + 3];  // b.r: the cell's column
+        }
+        for (size_t q = 0, r = 0; r <= (size_t)n + 1; ++r) {
+            p.rowarc[2 * r] = (int)q;
+            while (q < ordr.size() && (size_t)p.am_ends[4 * ordr[q] + 1] == r) ++q;
+            p.rowarc[2 * r + 1] = (int)q;
+        }
+        for (size_t q = 0; q < ord.size(); ++q) {
+            const int k = ord[q], i = p.am_ends[4 * k] - 1, j = p.am_ends[4 * k + 2] - 1;  // inner corner
+            const unsigned cc = in_band(i, j) ? p.bandoff[i] + j - p.min_col[i] : 0;
+            p.cre[4 * q] = p.am_pos[k];  // D entry
+            p.cre[4 * q + 1] = i | (j << 16);
+            p.cre[4 * q + 2] = (int)(cc << 5 | (p.am_ends[4 * k + 1] & 3) << 3 | (p.am_ends[4 * k + 3] & 7));
+            p.cre[4 * q + 3] = k;  // the arc match
         }
     }
-    p.am_pos.assign(na, -1);
-    p.crow.resize(2 * ordr.size());
-    p.rowarc.assign(2 * (size_t)(n + 2), 0);
-    for (size_t q = 0; q < ordr.size(); ++q) {
-        int k = ordr[q];
-        p.am_pos[k] = (int)q;
-        // (a.l-1) | (b.l-1) << 16: the inner corner; positions are < 2^15
-        p.crow[2 * q] = (p.am_ends[4 * k] - 1) | ((p.am_ends[4 * k + 2] - 1) << 16);
-        p.crow[2 * q + 1] = p.am_ends[4 * k + 3];  // b.r: the cell's column
-    }
-    for (size_t q = 0, r = 0; r <= (size_t)n + 1; ++r) {
-        p.rowarc[2 * r] = (int)q;
-        while (q < ordr.size() && (size_t)p.am_ends[4 * ordr[q] + 1] == r) ++q;
-        p.rowarc[2 * r + 1] = (int)q;
-    }
-    for (size_t q = 0; q < ord.size(); ++q) {
-        const int k = ord[q], i = p.am_ends[4 * k] - 1, j = p.am_ends[4 * k + 2] - 1;  // inner corner
-        const unsigned cc = in_band(i, j) ? p.bandoff[i] + j - p.min_col[i] : 0;
-        p.cre[4 * q] = p.am_pos[k];  // D entry
-        p.cre[4 * q + 1] = i | (j << 16);
-        p.cre[4 * q + 2] = (int)(cc << 5 | (p.am_ends[4 * k + 1] & 3) << 3 | (p.am_ends[4 * k + 3] & 7));
-        p.cre[4 * q + 3] = k;  // the arc match
-    }
-    p.num_pos = (int)ordr.size();
 
     // left-end groups (aligner.cc:660-732): bucket arc matches by (al,bl)
     // ordered by (al, bl) descending, index order within equal left ends:
     // two stable counting sorts (by bl descending, then by al descending)
-    std::vector<std::pair<long long, int>> byleft(na);
-    {
+    std::vector<std::pair<long long, int>> byleft(p.device_index ? 0 : na);
+    if (!p.device_index) {
         std::vector<int> tmp(na), cntb(m + 2, 0), cnta(n + 2, 0);
         for (int k = 0; k < na; ++k) cntb[m - p.am_ends[4 * k + 2] + 1]++;
         for (int j = 0; j <= m; ++j) cntb[j + 1] += cntb[j];
@@ -360,7 +484,7 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
         p.sscore.assign(std::max(na, 1), NEG);
         for (int k = 0; k < na; ++k) p.sscore[k] = t.am_stack_score[k] <= LCG_STACK_NONE ? NEG : t.am_stack_score[k];
     }
-    if (nolp || stack) {
+    if ((nolp || stack) && !p.device_index) {
         inner.assign(na, -1);
         p.inner.assign(std::max(na, 1), make_int2(-1, -1));
         for (int k = 0; k < na; ++k) {
@@ -379,7 +503,7 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
             }
         }
     }
-    p.Dinit.assign(p.num_pos, NEG);
+    if (!p.device_index) p.Dinit.assign(p.num_pos, NEG);
     std::vector<int> ks;
     // band cells of rows [r0, r1) inside columns [A, B], in O(log n) from
     // prefix sums (min_col and max_col are nondecreasing)
@@ -404,7 +528,31 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
     p.rows_max = 0;
     p.width_max = 0;
     p.rect_cells = 0;
-    p.am_rect.assign(std::max(na, 1), make_int2(-1, 0));
+    if (!p.device_index) p.am_rect.assign(std::max(na, 1), make_int2(-1, 0));
+    // the next group: its kept rectangle (rows al..ar-1, columns bl..br-1) and
+    // what it adds to the pair's totals
+    auto add_group = [&](GroupItem &g) {
+        const int rect_pitch = g.br - g.bl;
+        g.rect_off = -1;
+        if (p.rect_cells >= 0) {
+            const long long sz = (long long)(g.ar - g.al) * rect_pitch;
+            if (p.rect_cells + sz >= (1ll << 31)) {
+                p.rect_cells = -1;
+            } else {
+                g.rect_off = (int)p.rect_cells;
+                p.rect_cells += sz;
+            }
+        }
+        p.cells += rect_cells(g.al + 1, g.ar, g.bl + 1, g.br - 1);
+        g.cpl = 1;
+        p.groups.push_back(g);
+        p.rows_max = std::max(p.rows_max, g.ar - g.al);
+        p.width_max = std::max(p.width_max, g.br - g.bl + 1);
+    };
+    if (p.device_index) {
+        p.groups.reserve(groups.size() + 1);
+        for (GroupItem &g : groups) add_group(g);
+    }
     for (size_t s = 0; s < byleft.size();) {
         size_t e = s;
         while (e < byleft.size() && byleft[e].first == byleft[s].first) ++e;
@@ -474,30 +622,16 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
                 }
             }
             g.dw_count = (int)p.dw.size() - g.dw_start;
-            // the kept rectangle (rows al..ar-1, columns bl..br-1); the
-            // traceback reads it for the arc matches of this bucket (left
-            // ends (al, bl); without lonely pairs the group's left ends are
-            // shifted, and the traceback recomputes)
-            const int rect_pitch = max_br - bl;
-            g.rect_off = -1;
-            if (p.rect_cells >= 0) {
-                const long long sz = (long long)(max_ar - al) * rect_pitch;
-                if (p.rect_cells + sz >= (1ll << 31)) {
-                    p.rect_cells = -1;
-                } else {
-                    g.rect_off = (int)p.rect_cells;
-                    p.rect_cells += sz;
-                    if (!nolp && !lanes)
-                        for (size_t q = s; q < e; ++q) p.am_rect[byleft[q].second] = make_int2(g.rect_off, rect_pitch);
-                }
-            }
-            p.cells += rect_cells(al + 1, max_ar, bl + 1, max_br - 1);
-            g.cpl = 1;
+            // the traceback reads the kept rectangle for the arc matches of this
+            // bucket (left ends (al, bl); without lonely pairs the group's left
+            // ends are shifted, and the traceback recomputes)
+            const int index = (int)p.groups.size();
+            add_group(g);
             if (lanes)
-                for (size_t q = s; q < e; ++q) p.am_rect[byleft[q].second].x = (int)p.groups.size();
-            p.groups.push_back(g);
-            p.rows_max = std::max(p.rows_max, max_ar - al);
-            p.width_max = std::max(p.width_max, max_br - bl + 1);
+                for (size_t q = s; q < e; ++q) p.am_rect[byleft[q].second].x = index;
+            else if (!nolp && p.groups.back().rect_off >= 0)
+                for (size_t q = s; q < e; ++q)
+                    p.am_rect[byleft[q].second] = make_int2(p.groups.back().rect_off, max_br - bl);
         }
         s = e;
     }
@@ -523,7 +657,7 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
             if (p.lane_lines >= (1ll << 31)) p.lane_lines = -1;
             p.litems.push_back(it);
         }
-        for (int k = 0; k < na; ++k) {
+        for (int k = 0; k < (int)(p.device_index ? 0 : na); ++k) {
             const int g = p.am_rect[k].x;
             if (g < 0 || nolp) {
                 p.am_rect[k] = make_int2(0, -1);
@@ -633,7 +767,8 @@ Slot slot_of(lcg_engine e, int k) {
 struct PairOff {
     size_t sigma, scls, rcls, ccls, gapA, gapB, minc, maxc, bandoff, rowinfo, anc, cre_start, cre, crow, rowarc,
         am_score, D, topM, res, tok, tq, segs, groups, dw, gbc, dwn, inner, sscore, rect, am_rect,
-        litems, blkrows, quad_start;
+        litems, blkrows, quad_start, arcs4, lefts, row_start, row_arcs, am_lr, am_b, inner_a, inner_b, stackable, am_pos,
+        cursor, gcursor;
 };
 
 // One chunk of an lcg_align_pairs call: pairs [q0, q0 + nq) of the batch.
@@ -664,14 +799,15 @@ struct Chunk {
 // (sankoff_fill_kernel). An estimate of the three fill times from the pairs'
 // sizes; the constants are fits to measured fills on a GB300. Matrix cells:
 // 2 (n + m) per arc match within 30 % over 60-500 nt. One warp per group fills
-// 90 cells/ns, lane per group 130 (32 groups) or 170 (64); a lane item of a pair
-// is serial, its longest one takes 2.2 us per quad and 50 ns per arc match, of
-// which a launch ends with three quarters (a third more with 64 groups), and
-// the row sweep of one group a sixth of that. So single pairs and small batches
-// go to one warp per group (one 400 x 400 pair: 3.1 ms against 9.6 ms), batches
-// to lanes (28 profile pairs of 80-300: 5.0 -> 4.6 ms with 32 groups, 5.9 with
-// 64; 66 pairs of 60-300 nt: 8.9 -> 7.3 and 7.2 ms; 276 pairs of 60-400 nt in
-// two chunks: 126 -> 82 and 64 ms).
+// 80 cells/ns, lane per group 130 (32 groups) or 170 (64). A lane item is
+// serial: the longest one of a pair takes 2.2 us per quad and 50 ns per arc
+// match, and a launch ends with six tenths of that (64 groups: 1.4 times), where
+// the row sweep of one group takes a sixth. So single pairs and small batches go
+// to one warp per group (one 400 x 400 pair: 3.1 ms against 9.6 ms), batches to
+// lanes (fill of 28 profile pairs of 80-300 columns: 5.0 -> 4.7 ms with 32
+// groups, 5.9 with 64; 45 stacking pairs of 100-300 nt: 8.6 -> 6.7, 7.4 with 64;
+// 66 pairs of 60-300 nt: 8.9 -> 7.4 with either; 276 pairs of 60-400 nt in two
+// chunks: 126 -> 82, 64 with 64).
 int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg_align_opts *opts) {
     if (e->counting || opts->struct_local) return 0;
     if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) == 64 ? 64 : std::atoi(v) == 32 ? 32 : 0;
@@ -685,8 +821,18 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
         longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
     }
     if (opts->no_lonely_pairs) cells /= 50;  // few arc matches have a stacked partner
-    const double warp = cells / 90 + longest / 6, l32 = cells / 130 + 0.75 * longest, l64 = cells / 170 + longest;
+    const double warp = cells / 80 + longest / 6, l32 = cells / 130 + 0.6 * longest, l64 = cells / 170 + 1.4 * longest;
     return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
+}
+
+// Whether the device makes the index structures of a chunk: from 2,000 arc
+// matches on its two launches (10 us) cost less than the host's 30 ns per arc
+// match (one 60 x 60 pair: 500 arc matches, 15 us on the host).
+bool index_on_device(const lcg_pair_tables *pairs, int npairs) {
+    if (const char *v = std::getenv("LCG_DEVICE_INDEX")) return v[0] != '0';
+    long long am = 0;
+    for (int q = 0; q < npairs; ++q) am += std::max(pairs[q].num_arcmatches, 0);
+    return am >= 2000;
 }
 
 // pairs per chunk: one chunk for small batches, else up to 8 chunks of at
@@ -817,6 +963,13 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         return o;
     };
     size_t off_pairs = take(up, sizeof(PairDev) * npairs);
+    int index_lefts = -1, index_n = 0;  // -1: no pair's index structures are made on the device
+    for (auto &p : prep)
+        if (p.device_index) {
+            index_lefts = std::max(index_lefts, (int)p.lefts.size());
+            index_n = std::max(index_n, p.n);
+        }
+    const size_t off_index = index_lefts >= 0 ? take(up, sizeof(IndexPair) * npairs) : 0;
     // the pairs filled lane per group and the others, each with a queue of
     // (pair, item) work items and a launch of its own
     std::vector<int> of[2];
@@ -839,7 +992,9 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         PairOff &o = off[q];
         o.gbc = take(up, 4ull * (p.m + 1));
         o.groups = take(up, sizeof(GroupItem) * p.groups.size());
-        o.dw = take(up, sizeof(int4) * std::max<size_t>(p.dw.size(), 1));
+        // what the device makes itself is laid out behind the upload, below
+        const bool dev = p.device_index;
+        o.dw = dev ? 0 : take(up, sizeof(int4) * std::max<size_t>(p.dw.size(), 1));
         o.dwn = p.inner.empty() ? 0 : take(up, sizeof(int2) * std::max<size_t>(p.dwn.size(), 1));
         o.inner = p.inner.empty() ? 0 : take(up, sizeof(int2) * p.inner.size());
         o.sscore = p.sscore.empty() ? 0 : take(up, 4ull * p.sscore.size());
@@ -856,12 +1011,23 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         o.rowinfo = take(up, 16ull * (p.n + 2));
         o.anc = t.match_lo ? take(up, 4ull * (2 * (p.n + 1) + 2 * (p.n + 1) + 2 * (p.m + 1))) : 0;
         o.cre_start = take(up, 4ull * p.cre_start.size());
-        o.cre = take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
-        o.crow = take(up, 4ull * std::max<size_t>(p.crow.size(), 4));
+        o.cre = dev ? 0 : take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
+        o.crow = dev ? 0 : take(up, 4ull * std::max<size_t>(p.crow.size(), 4));
         o.rowarc = take(up, 4ull * p.rowarc.size());
         o.am_score = take(up, 4ull * std::max(t.num_arcmatches, 1));
-        o.D = take(up, 4ull * std::max(p.num_pos, 1));
-        o.am_rect = keep ? take(up, 8ull * p.am_rect.size()) : 0;
+        o.D = dev ? 0 : take(up, 4ull * std::max(p.num_pos, 1));
+        o.am_rect = keep && !dev ? take(up, 8ull * p.am_rect.size()) : 0;
+        if (dev) {
+            o.arcs4 = take(up, 16ull * std::max<size_t>(p.arcs4.size(), 1));
+            o.lefts = take(up, 16ull * std::max<size_t>(p.lefts.size(), 1));
+            o.row_start = take(up, 4ull * p.row_start.size());
+            o.row_arcs = take(up, 4ull * p.row_arcs.size());
+            o.am_lr = take(up, 4ull * p.am_lr.size());
+            o.am_b = take(up, 4ull * p.am_b.size());
+            o.inner_a = take(up, 4ull * p.inner_a.size());
+            o.inner_b = take(up, 4ull * p.inner_b.size());
+            o.stackable = take(up, p.am_b.size());
+        }
         o.litems = take(up, sizeof(LaneItem) * p.litems.size());
         o.blkrows = take(up, sizeof(int4) * p.blkrows.size());
         o.quad_start = take(up, 4ull * p.quad_start.size());
@@ -882,6 +1048,21 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         const auto &p = prep[q];
         PairOff &o = off[q];
         o.tq = take(dev_only, 16ull * p.tq_cap);
+        if (p.device_index) {
+            const size_t na = (size_t)std::max(pairs[q].num_arcmatches, 1), npos = (size_t)std::max(p.num_pos, 1);
+            o.dw = take(dev_only, sizeof(int4) * std::max(p.num_dw, 1));
+            if (p.flags & PF_STACK) {
+                o.dwn = take(dev_only, sizeof(int2) * std::max(p.num_dw, 1));
+                o.inner = take(dev_only, sizeof(int2) * na);
+            }
+            o.cre = take(dev_only, 16 * npos);
+            o.crow = take(dev_only, 8 * npos);
+            o.D = take(dev_only, 4 * npos);
+            o.am_rect = keep ? take(dev_only, 8 * na) : 0;
+            o.am_pos = take(dev_only, 4 * na);
+            o.cursor = take(dev_only, 4ull * p.bandcells);
+            o.gcursor = take(dev_only, 4ull * p.groups.size());
+        }
         o.topM = take(dev_only, 4ull * (p.n + 1) * (p.m + 1));
         const size_t rect_bytes = (p.flags & PF_LANES) ? 4ull * p.lane_groups * std::max<long long>(p.lane_lines, 1)
                                                        : (size_t)rect_bytes_per_cell * std::max<long long>(p.rect_cells, 1);
@@ -969,7 +1150,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         if (!p.cre.empty()) std::memcpy(H + o.cre, p.cre.data(), 4ull * p.cre.size());
         if (!p.crow.empty()) std::memcpy(H + o.crow, p.crow.data(), 4ull * p.crow.size());
         std::memcpy(H + o.rowarc, p.rowarc.data(), 4ull * p.rowarc.size());
-        if (p.num_pos) std::memcpy(H + o.D, p.Dinit.data(), 4ull * p.num_pos);
+        if (!p.Dinit.empty()) std::memcpy(H + o.D, p.Dinit.data(), 4ull * p.num_pos);
         if (t.num_arcmatches) {
             std::memcpy(H + o.am_score, t.am_score, 4ull * t.num_arcmatches);
         }
@@ -983,7 +1164,30 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         if (!p.dwn.empty()) std::memcpy(H + o.dwn, p.dwn.data(), sizeof(int2) * p.dwn.size());
         if (!p.inner.empty()) std::memcpy(H + o.inner, p.inner.data(), sizeof(int2) * p.inner.size());
         if (!p.sscore.empty()) std::memcpy(H + o.sscore, p.sscore.data(), 4ull * p.sscore.size());
-        if (keep) std::memcpy(H + o.am_rect, p.am_rect.data(), 8ull * p.am_rect.size());
+        if (keep && !p.device_index) std::memcpy(H + o.am_rect, p.am_rect.data(), 8ull * p.am_rect.size());
+        if (index_lefts >= 0) {
+            IndexPair &X = ((IndexPair *)(H + off_index))[q];
+            std::memset(&X, 0, sizeof X);
+            if (p.device_index) {
+                auto put = [&](size_t at, const void *src, size_t bytes) {
+                    if (bytes) std::memcpy(H + at, src, bytes);
+                    return Dv + at;
+                };
+                X.arcs = (const int4 *)put(o.arcs4, p.arcs4.data(), 16ull * p.arcs4.size());
+                X.lefts = (const int4 *)put(o.lefts, p.lefts.data(), 16ull * p.lefts.size());
+                X.nlefts = (int)p.lefts.size();
+                X.row_start = (const int *)put(o.row_start, p.row_start.data(), 4ull * p.row_start.size());
+                X.row_arcs = (const int *)put(o.row_arcs, p.row_arcs.data(), 4ull * p.row_arcs.size());
+                X.am_lr = (const int *)put(o.am_lr, p.am_lr.data(), 4ull * p.am_lr.size());
+                X.am_b = (const int *)put(o.am_b, p.am_b.data(), 4ull * p.am_b.size());
+                X.inner_a = (const int *)put(o.inner_a, p.inner_a.data(), 4ull * p.inner_a.size());
+                X.inner_b = (const int *)put(o.inner_b, p.inner_b.data(), 4ull * p.inner_b.size());
+                X.am_stackable = (const unsigned char *)put(o.stackable, t.am_stackable, p.am_b.size());
+                X.am_pos = (int *)(Dv + o.am_pos);
+                X.cursor = (int *)(Dv + o.cursor);
+                X.gcursor = (int *)(Dv + o.gcursor);
+            }
+        }
         PairDev &d = hp[q];
         std::memset(&d, 0, sizeof d);
         d.n = p.n;
@@ -1050,8 +1254,8 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             d.blkrows = (const int4 *)(Dv + o.blkrows);
         }
         d.dw = (const int4 *)(Dv + o.dw);
-        d.dwn = p.inner.empty() ? nullptr : (const int2 *)(Dv + o.dwn);
-        d.inner = p.inner.empty() ? nullptr : (const int2 *)(Dv + o.inner);
+        d.dwn = o.dwn ? (const int2 *)(Dv + o.dwn) : nullptr;
+        d.inner = o.inner ? (const int2 *)(Dv + o.inner) : nullptr;
         d.am_sscore = p.sscore.empty() ? nullptr : (const int *)(Dv + o.sscore);
     });
     *pack_ms += ms_between(tp0, std::chrono::steady_clock::now());
@@ -1133,7 +1337,8 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         key = {(long long)(uintptr_t)Dv, (long long)(uintptr_t)H, (long long)(uintptr_t)scratch, (long long)down_begin,
                (long long)down_end, (long long)off_ctrl, (long long)off_pairs, (long long)off_queue, (long long)nitems[0],
                blocks, sw, rb, stride, fast, e->counting, sl, sl_fast, keep, opts->do_trace, npairs,
-               (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lfast, lgroups};
+               (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lfast, lgroups,
+               (long long)off_index, index_n, index_lefts};
         if (s.graph->exec && s.graph->key == key) {
             CUDA_TRY(cudaGraphLaunch(s.graph->exec, st));
             ++e->last_graph_replays;
@@ -1181,6 +1386,9 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     CUDA_TRY_CAP(record(s.ev0));
     unsigned long long *counters = e->counting ? (unsigned long long *)(Dv + off_ctrl + 16) : nullptr;
     c.launches = 0;
+    if (index_lefts >= 0)
+        CUDA_TRY_CAP(launch_index((const PairDev *)(Dv + off_pairs), (const IndexPair *)(Dv + off_index), npairs,
+                                  index_n, index_lefts, st));
     if (!of[1].empty()) {
         CUDA_TRY_CAP(launch_lane_fill(lgroups, (const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_lqueue),
                                       (int)nitems[1], scratch, lslot, lqslot, rb, lfast,
@@ -1560,7 +1768,8 @@ static lcg_status align_impl(lcg_engine e, const lcg_pair_tables *pairs, int32_t
         next.clear();
         next.resize(nq);
         const int lanes = lane_width(e, pairs + q0, nq, opts);
-        lcg_host::parallel_for(nq, [&](int q) { prep_pair(pairs[q0 + q], *opts, next[q], lanes); });
+        const bool dev = index_on_device(pairs + q0, nq);
+        lcg_host::parallel_for(nq, [&](int q) { prep_pair(pairs[q0 + q], *opts, next[q], lanes, dev); });
         t_prep += ms_between(a, clk::now());
         for (int q = 0; q < nq && rc == LCG_OK; ++q)
             if (next[q].code != LCG_OK)
@@ -1760,7 +1969,8 @@ lcg_status lcg_align_kbest(lcg_engine e, const lcg_pair_tables *pairs, int32_t n
     c.kbest = true;
     c.prep.resize(npairs);
     const int lanes = lane_width(e, pairs, npairs, opts);
-    lcg_host::parallel_for(npairs, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q], lanes); });
+    const bool dev = index_on_device(pairs, npairs);
+    lcg_host::parallel_for(npairs, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q], lanes, dev); });
     for (int q = 0; q < npairs; ++q)
         if (c.prep[q].code != LCG_OK) return fail(c.prep[q].code, "pair " + std::to_string(q) + ": " + c.prep[q].err);
     const Slot sl0 = slot_of(e, 0);

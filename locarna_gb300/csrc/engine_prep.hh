@@ -57,6 +57,17 @@ struct Prep {
     std::vector<int> quad_start;
     int lane_groups = 0;
     long long lane_slot = 0, lane_lines = 0;
+    // Index structures made on the device (index_kernels.cu; then cre, crow,
+    // am_pos, am_ends, Dinit, dw, dwn, inner and am_rect stay empty here): per
+    // arc of A (l, r, first and past its last arc match), the arcs of A by right
+    // end (row_start[i] .. row_start[i + 1] of row_arcs), per left end of A (first
+    // and past its last arc, first and past its last group), per arc match the
+    // ends of its arc of B (l | r << 16); with stacking per arc match its arc of
+    // B and per arc the next inner one (l + 1, r - 1) or -1
+    bool device_index = false;
+    std::vector<int4> arcs4, lefts;
+    std::vector<int> row_start, row_arcs, am_lr, am_b, inner_a, inner_b;
+    int num_dw = 0;
     int token_cap = 0, tq_cap = 0;
     long long cells = 0;                         // M cells of all groups + top level
     std::string err;
@@ -66,7 +77,10 @@ struct Prep {
 // Validate one pair's tables and build its derived structures; on error
 // p.code / p.err describe it. lanes: groups per item of the
 // lane-per-group fill where the pair allows it (then p.flags has PF_LANES), 0: none.
-lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes = 0);
+// device_index: leave what is made per arc match to the device where the pair
+// allows it (then p.device_index).
+lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes = 0,
+                     bool device_index = false);
 
 void set_error(const std::string &msg);
 
