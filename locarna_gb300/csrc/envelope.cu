@@ -2,7 +2,12 @@
 // TraceController (trace_controller.cc:565-597) from the PFGotoh forward and
 // reverse partition functions (edge_probs.icc:76-162) and the edge
 // probabilities of PFTraceProbs (edge_probs.icc:212-268), for a batch of
-// pairs, one warp per pair.
+// pairs, one block per pair (four warps per direction).
+//
+// 166 pairs of 60-400 nt take 5.0 ms and 0.3 ms for the weights; one warp per
+// pair, four pairs per block, took 29.3 ms (FP64 issue of the 42 SMs it used),
+// one warp per block with the weights kept for the reverse pass 18.3 ms (the
+// row's chain of dependent FP64 operations).
 //
 // The reference evaluates the recursions in long double (locarna) or double
 // (locarna_p) without scaling. Here every matrix row is kept in FP64 scaled by
@@ -32,7 +37,9 @@
 
 namespace {
 
-constexpr int ENV_WARPS = 4;  // warps (pairs) per block
+constexpr int ENV_SIDE = 128;             // threads per direction
+constexpr int ENV_THREADS = 2 * ENV_SIDE;  // forward and reverse pass of one pair
+constexpr int ENV_ROW_SMEM = 96 * 1024;    // at most this much shared memory for rows, else they stay in HBM
 
 struct EnvDev {
     int n, m;
@@ -40,9 +47,9 @@ struct EnvDev {
     const double *sdA, *suA, *sdB, *suB;
     const int *minc, *maxc;
     int *newmin, *newmax, *flag;
-    double *fz;   // forward rows: (n+1) x [zM | zA | zB] x (m+1)
-    int *fexp;    // forward row exponents
-    double *rz;   // reverse rows, two alternating: 2 x [zM | zA | zB] x (m+1)
+    double *fz, *rz;    // forward and reverse rows: (n+1) x [zM | zA | zB] x (m+1)
+    int *fexp, *rexp;   // their exponents
+    double *wt;         // match weights, (n+1) x (m+1)
 };
 
 struct EnvConst {
@@ -95,151 +102,257 @@ __device__ __forceinline__ int band_hi(const EnvDev &P, int i) {
     return REV ? P.m - P.minc[P.n - i] : P.maxc[i];
 }
 
-// Boltzmann weight of the StralScore match (stral_score.cc:29-60) at (i, j)
-// of direction REV; the reverse object mirrors both sequences and swaps the
-// up/down probabilities, which leaves sqrt(dA dB) + sqrt(uA uB) unchanged.
-template <bool REV>
+// Boltzmann weight of the StralScore match (stral_score.cc:29-60) at (i, j).
+// The reverse pass's object mirrors both sequences and swaps the up/down
+// probabilities, which leaves sqrt(dA dB) + sqrt(uA uB) unchanged.
 __device__ __forceinline__ double match_weight(const EnvDev &P, const EnvConst &C, int i, int j) {
-    const int ia = REV ? P.n + 1 - i : i, jb = REV ? P.m + 1 - j : j;
-    const int a = P.ca[ia], b = P.cb[jb];
+    const int a = P.ca[i], b = P.cb[j];
     const double seq = (a >= 0 && b >= 0) ? C.score[a * 4 + b] : 0.0;
-    const double s = C.sw * (P.sdA[ia] * P.sdB[jb] + P.suA[ia] * P.suB[jb]) + seq;
+    const double s = C.sw * (P.sdA[i] * P.sdB[j] + P.suA[i] * P.suB[j]) + seq;
     return exp(s * C.itemp);
 }
 
-// Row 0 of direction REV (PFGotoh::pf_gotoh initialisation, edge_probs.icc:
-// 89-117): zM(0,0) = 1 (global) / 0 (local); zB(0,j) = g_open g_ext^j along
-// the band; +1 on zB(0,j) with free end gaps at the start of B.
-template <bool REV>
-__device__ void env_row0(const EnvDev &P, const EnvConst &C, double *row, int fe) {
-    const int lane = threadIdx.x & 31;
-    const int m1 = P.m + 1;
-    const int lo0 = band_lo<REV>(P, 0), hi0 = band_hi<REV>(P, 0);
-    const bool chain = lo0 <= 1;
-    for (int j = lane; j <= P.m; j += 32) {
-        double zb = 0.0;
-        if (j >= 1) {
-            if (chain && j <= hi0) zb = C.go * C.ge * pow(C.ge, (double)(j - 1));
-            if (fe & LCG_FREE_LEFT_1) zb += 1.0;
-        }
-        row[j] = (j == 0 && lo0 == 0 && !C.local) ? 1.0 : 0.0;
-        row[m1 + j] = 0.0;
-        row[2 * m1 + j] = zb;
-    }
+// The weights of every cell that a pass reads: cells of the band (forward) and
+// those one step down and right of one (reverse). One warp per row; the exp
+// evaluations are most of the envelope's FP64 operations, of which an SM issues
+// two a clock, so they are spread over all SMs and done once for both passes.
+__global__ void __launch_bounds__(256) env_weights_kernel(const EnvDev *__restrict__ pairs, EnvConst C) {
+    const EnvDev &P = pairs[blockIdx.x];
+    const int i = blockIdx.y * 8 + (threadIdx.x >> 5) + 1;
+    if (i > P.n) return;
+    const int lo = max(1, min(P.minc[i], P.minc[i - 1] + 1)), hi = min(P.m, max(P.maxc[i], P.maxc[i - 1] + 1));
+    double *const w = P.wt + (size_t)i * (P.m + 1);
+    for (int j = lo + (threadIdx.x & 31); j <= hi; j += 32) w[j] = match_weight(P, C, i, j);
 }
 
-// Row i >= 1 of direction REV from row i-1 (`prev`, scaled by 2^-eprev) into
-// `cur` in the same scale (edge_probs.icc:118-161); returns the row maximum
-// and, through zsum, the sum of zM over the row.
-template <bool REV>
-__device__ double env_row(const EnvDev &P, const EnvConst &C, int i, const double *prev, double *cur, int eprev,
-                          int fe, double *zsum) {
+// Constants of a warp's gap chains: g_ext^1, 2, 4, 8, 16 and g_ext^(lane+1)
+struct EnvPow {
+    double p[5], lane;
+};
+__device__ __forceinline__ EnvPow env_pow(double ge) {
+    EnvPow w;
+    double x = ge, y = ge;
     const int lane = threadIdx.x & 31;
-    const int m1 = P.m + 1;
-    const int lo = band_lo<REV>(P, i), hi = band_hi<REV>(P, i);
-    const int j0 = max(lo, 1), j1 = min(hi, P.m);
-    // column 0: zA(i,0) = g_open g_ext^i while the band holds column 0 (from
-    // row 1 on), +1 with free end gaps at the start of A
-    double col0 = 0.0;
-    if (band_lo<REV>(P, 1) == 0 && lo == 0) col0 = C.go * C.ge * pow(C.ge, (double)(i - 1));
-    if (fe & LCG_FREE_LEFT_2) col0 += 1.0;
-    col0 = ldexp(col0, -eprev);
-    const double locw = C.local ? ldexp(1.0, -eprev) : 0.0;
-    const double gog = C.go * C.ge;
-    double carryB = 0.0, carryMA = 0.0;  // zB(i, base-1) and zM + zA at (i, base-1)
-    double rmax = 0.0, rsum = 0.0;
-    for (int base = 0; base <= P.m; base += 32) {
-        const int j = base + lane;
-        const bool act = j <= P.m;
-        const bool inb = act && j >= j0 && j <= j1;
-        double zm = 0.0, za = (j == 0) ? col0 : 0.0;
-        if (inb) {
-            const double w = match_weight<REV>(P, C, i, j);
-            const double pm1 = prev[j - 1] + prev[m1 + j - 1] + prev[2 * m1 + j - 1];
-            zm = pm1 * w + w * locw;
-            za = prev[m1 + j] * C.ge + prev[j] * gog + prev[2 * m1 + j] * gog;
-        }
-        // zB(j) = g_ext zB(j-1) + (zM + zA)(j-1) g_open g_ext inside the band,
-        // 0 outside: a first-order linear recurrence, scanned over the lanes
-        double ma = zm + za;
-        double mal = __shfl_up_sync(0xffffffffu, ma, 1);
-        if (lane == 0) mal = carryMA;
-        double a = inb ? C.ge : 0.0;
-        double b = inb ? mal * gog : 0.0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const double a2 = __shfl_up_sync(0xffffffffu, a, off);
-            const double b2 = __shfl_up_sync(0xffffffffu, b, off);
-            if (lane >= off) {
-                b = a * b2 + b;
-                a = a * a2;
-            }
-        }
-        const double zb = a * carryB + b;
-        if (act) {
-            cur[j] = zm;
-            cur[m1 + j] = za;
-            cur[2 * m1 + j] = zb;
-            rmax = fmax(rmax, fmax(zm, fmax(za, zb)));
-            rsum += zm;
-        }
-        carryB = __shfl_sync(0xffffffffu, zb, 31);
-        carryMA = __shfl_sync(0xffffffffu, ma, 31);
+    for (int k = 0; k < 5; ++k) {
+        w.p[k] = x;
+        if (lane >> k & 1) y *= x;
+        x *= x;
     }
-    *zsum = warp_sum(rsum);
-    return warp_max(rmax);
+    w.lane = y;
+    return w;
 }
 
-// scale a row by 2^-d (exact)
-__device__ void env_scale(double *row, int m1, int d) {
-    if (d == 0) return;
-    const int lane = threadIdx.x & 31;
-    for (int k = lane; k < 3 * m1; k += 32) row[k] = ldexp(row[k], -d);
-}
+// what the four warps of a direction exchange
+struct EnvShare {
+    double a[2][4], t[2][4];  // gap-chain totals of a warp's 32 columns, by pass parity
+    double sum[4], top[4];
+    int hmax[4];
+};
 
-__device__ __forceinline__ int exp_of(double v) { return v > 0.0 ? ilogb(v) : 0; }
+constexpr int ENV_RANGE = 128;
 
-__global__ void __launch_bounds__(ENV_WARPS * 32) envelope_kernel(const EnvDev *__restrict__ pairs, int npairs,
-                                                                    EnvConst C) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = blockIdx.x * ENV_WARPS + warp;
-    if (q >= npairs) return;
-    const EnvDev &P = pairs[q];
+// One direction of the partition function (PFGotoh::pf_gotoh, edge_probs.icc:
+// 76-162) by 128 threads: rows in order, 128 columns at a time. The gap chain
+// of a row is a linear recurrence T(j) = a(j) T(j-1) + c(j): a scan inside each
+// warp (constant factors where its 32 columns are all in the band), the warps'
+// totals combined through shared memory. Rows are kept in HBM for the edge
+// probabilities and, where they fit, two of them in shared memory. A row that
+// has left 2^-ENV_RANGE .. 2^ENV_RANGE is scaled back to 1 .. 2 by a power of
+// two (exact); zexp holds the exponents. Returns the flag (2: values that the
+// reference's float type would not hold); local alignment: *zloc, the sum of zM.
+template <bool REV>
+__device__ int env_pass(const EnvDev &P, const EnvConst &C, double *rows, EnvShare &sh, XAcc *zloc) {
+    const int tid = threadIdx.x & (ENV_SIDE - 1), lane = tid & 31, sub = tid >> 5;
     const int n = P.n, m = P.m, m1 = m + 1;
     const size_t rowsz = 3 * (size_t)m1;
-    int flag = 0;
-
-    // ---- forward: every row kept
-    env_row0<false>(P, C, P.fz, C.fe);
-    if (lane == 0) P.fexp[0] = 0;
-    __syncwarp();
-    int e = 0;
-    XAcc zloc{0.0, 0};
-    if (C.local) {
-        double s = 0.0;
-        for (int j = lane; j <= m; j += 32) s += P.fz[j];
-        xadd(zloc, warp_sum(s), 0);
+    double *const z = REV ? P.rz : P.fz;
+    int *const zexp = REV ? P.rexp : P.fexp;
+    const int fe = REV ? C.rfe : C.fe;
+    const EnvPow W = env_pow(C.ge);
+    const double gog = C.go * C.ge;
+    auto sync = [] { asm volatile("bar.sync %0, %1;" ::"r"(REV ? 2 : 1), "n"(ENV_SIDE) : "memory"); };
+    // row i's values: zM, zA, zB
+    auto row = [&](int i) { return rows ? rows + (size_t)(i & 1) * rowsz : z + (size_t)i * rowsz; };
+    int flag = 0, e = 0;
+    {
+        // row 0 (edge_probs.icc:89-117): zM(0,0) = 1 (global) / 0 (local);
+        // zB(0,j) = g_open g_ext^j along the band; +1 on zB(0,j) with free end
+        // gaps at the start of B
+        double *const r = row(0);
+        const int lo0 = band_lo<REV>(P, 0), hi0 = band_hi<REV>(P, 0);
+        const bool chain = lo0 <= 1;
+        for (int j = tid; j <= m; j += ENV_SIDE) {
+            const double zm = (j == 0 && lo0 == 0 && !C.local) ? 1.0 : 0.0;
+            double zb = 0.0;
+            if (j >= 1) {
+                if (chain && j <= hi0) zb = C.go * C.ge * pow(C.ge, (double)(j - 1));
+                if (fe & LCG_FREE_LEFT_1) zb += 1.0;
+            }
+            r[j] = zm;
+            r[m1 + j] = 0.0;
+            r[2 * m1 + j] = zb;
+            if (rows) {
+                z[j] = zm;
+                z[m1 + j] = 0.0;
+                z[2 * m1 + j] = zb;
+            }
+        }
+        if (tid == 0) zexp[0] = 0;
     }
+    sync();
     for (int i = 1; i <= n; ++i) {
-        double *cur = P.fz + (size_t)i * rowsz;
-        double zs = 0.0;
-        const double mx = env_row<false>(P, C, i, cur - rowsz, cur, e, C.fe, &zs);
-        if (C.local) xadd(zloc, zs, e);
-        __syncwarp();
-        const int d = exp_of(mx);
-        env_scale(cur, m1, d);
-        e += d;
-        if (e + 2 > C.exp_limit) flag = 2;
-        if (lane == 0) P.fexp[i] = e;
-        __syncwarp();
+        const double *const prev = row(i - 1);
+        double *const cur = row(i), *const out = z + (size_t)i * rowsz;
+        const int lo = band_lo<REV>(P, i), hi = band_hi<REV>(P, i);
+        const int j0 = max(lo, 1), j1 = min(hi, m);
+        // column 0: zA(i,0) = g_open g_ext^i while the band holds column 0 (from
+        // row 1 on), +1 with free end gaps at the start of A
+        double col0 = 0.0;
+        if (tid == 0) {
+            if (band_lo<REV>(P, 1) == 0 && lo == 0) col0 = C.go * C.ge * pow(C.ge, (double)(i - 1));
+            if (fe & LCG_FREE_LEFT_2) col0 += 1.0;
+            col0 = ldexp(col0, -e);
+        }
+        const double locw = C.local ? ldexp(1.0, -e) : 0.0;
+        const double *const w = P.wt + (size_t)(REV ? n + 1 - i : i) * m1;
+        double carry = 0.0, rsum = 0.0;  // T of the column before the pass
+        int hmax = 0, par = 0;
+        for (int base = 0; base <= m; base += ENV_SIDE, par ^= 1) {
+            const int j = base + tid;
+            const bool act = j <= m, inb = act && j >= j0 && j <= j1;
+            double zm = 0.0, za = col0;  // (zero but for column 0)
+            col0 = 0.0;
+            if (inb) {
+                const double wj = w[REV ? m + 1 - j : j];
+                const double pm1 = prev[j - 1] + prev[m1 + j - 1] + prev[2 * m1 + j - 1];
+                zm = C.local ? pm1 * wj + wj * locw : pm1 * wj;
+                za = prev[m1 + j] * C.ge + (prev[j] + prev[2 * m1 + j]) * gog;
+            }
+            // zB(j) = T(j-1) inside the band, 0 outside; T(j) = g_ext zB(j) + (zM + zA)(j) g_open g_ext
+            double t = (zm + za) * gog, a;
+            const int c0 = base + 32 * sub;
+            if (c0 >= j0 && c0 + 31 <= j1) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const double t2 = __shfl_up_sync(0xffffffffu, t, 1 << k);
+                    if (lane >= 1 << k) t = W.p[k] * t2 + t;
+                }
+                a = W.lane;
+            } else {
+                a = inb ? C.ge : 0.0;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const double a2 = __shfl_up_sync(0xffffffffu, a, off);
+                    const double t2 = __shfl_up_sync(0xffffffffu, t, off);
+                    if (lane >= off) {
+                        t = a * t2 + t;
+                        a = a * a2;
+                    }
+                }
+            }
+            if (lane == 31) {
+                sh.a[par][sub] = a;
+                sh.t[par][sub] = t;
+            }
+            sync();
+            double c = carry;
+            for (int s = 0; s < 4; ++s) {
+                if (s == sub) c = carry;
+                carry = sh.a[par][s] * carry + sh.t[par][s];
+            }
+            t = a * c + t;
+            double zb = __shfl_up_sync(0xffffffffu, t, 1);
+            if (lane == 0) zb = c;
+            if (!inb) zb = 0.0;
+            if (act) {
+                cur[j] = zm;
+                cur[m1 + j] = za;
+                cur[2 * m1 + j] = zb;
+                if (rows) {
+                    out[j] = zm;
+                    out[m1 + j] = za;
+                    out[2 * m1 + j] = zb;
+                }
+                // no value is negative: their order is that of the high words
+                hmax = max(hmax, max(__double2hiint(zm), max(__double2hiint(za), __double2hiint(zb))));
+                if (C.local) rsum += zm;
+            }
+        }
+        // the row's largest value and, local, its sum
+        hmax = __reduce_max_sync(0xffffffffu, hmax);
+        if (C.local) rsum = warp_sum(rsum);
+        if (lane == 0) {
+            sh.hmax[sub] = hmax;
+            sh.sum[sub] = rsum;
+        }
+        sync();
+        hmax = max(max(sh.hmax[0], sh.hmax[1]), max(sh.hmax[2], sh.hmax[3]));
+        if (C.local && zloc) xadd(*zloc, sh.sum[0] + sh.sum[1] + sh.sum[2] + sh.sum[3], e);
+        int d = (hmax >> 20) - 1023;
+        if (hmax < 1 << 20) {  // zeros, or below the normal range
+            double mx = 0.0;
+            for (int k = tid; k < 3 * m1; k += ENV_SIDE) mx = fmax(mx, cur[k]);
+            mx = warp_max(mx);
+            if (lane == 0) sh.top[sub] = mx;
+            sync();
+            mx = fmax(fmax(sh.top[0], sh.top[1]), fmax(sh.top[2], sh.top[3]));
+            d = mx > 0.0 ? ilogb(mx) : 0;
+        }
+        if (e + d + 2 > C.exp_limit) flag = 2;
+        if (d > ENV_RANGE || d < -ENV_RANGE) {
+            for (int k = tid; k < 3 * m1; k += ENV_SIDE) {
+                const double v = ldexp(cur[k], -d);
+                cur[k] = v;
+                if (rows) out[k] = v;
+            }
+            e += d;
+            sync();
+        }
+        if (tid == 0) zexp[i] = e;
     }
-    // total (edge_probs.icc:220-236)
+    return flag;
+}
+
+// One pair per block: forward and reverse pass side by side, then the edge
+// probabilities (PFTraceProbs, edge_probs.icc:212-268) and row thresholds, a
+// warp per row. Bound by FP64 issue and, for a pair alone, by the rows' chain of
+// dependent FP64 operations (about 2,500 clocks a row of 400).
+__global__ void __launch_bounds__(ENV_THREADS) envelope_kernel(const EnvDev *__restrict__ pairs, EnvConst C,
+                                                               size_t row_smem) {
+    extern __shared__ double env_smem[];
+    __shared__ EnvShare share[2];
+    __shared__ XAcc zloc_s;
+    __shared__ int flags[3];
+    const EnvDev &P = pairs[blockIdx.x];
+    const int n = P.n, m = P.m, m1 = m + 1;
+    const size_t rowsz = 3 * (size_t)m1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool rev = threadIdx.x >= ENV_SIDE;
+    const bool shared_rows = 4 * rowsz * sizeof(double) <= row_smem;
+    if (threadIdx.x == 0) flags[2] = 0;
+    if (rev) {
+        const int f = env_pass<true>(P, C, shared_rows ? env_smem + 2 * rowsz : nullptr, share[1], nullptr);
+        if (threadIdx.x == ENV_SIDE) flags[1] = f;
+    } else {
+        XAcc zloc{0.0, 0};  // (zM of row 0 is 0 in local alignment)
+        const int f = env_pass<false>(P, C, shared_rows ? env_smem : nullptr, share[0], &zloc);
+        if (threadIdx.x == 0) {
+            flags[0] = f;
+            zloc_s = zloc;
+        }
+    }
+    __syncthreads();
+    // total (edge_probs.icc:220-236), every warp for itself
+    const XAcc zloc = zloc_s;
+    int flag = max(flags[0], flags[1]);
     XAcc z{0.0, 0};
     if (C.local) {
         xadd(z, 1.0, 0);
         xadd(z, zloc.v, zloc.e);
     } else {
         const double *rn = P.fz + (size_t)n * rowsz;
+        const int e = P.fexp[n];
         xadd(z, rn[m] + rn[m1 + m] + rn[2 * m1 + m], e);
         if (C.fe & LCG_FREE_LEFT_2)
             for (int i = 0; i <= n; ++i) xadd(z, P.fz[(size_t)i * rowsz + m1 + m], P.fexp[i]);
@@ -251,61 +364,49 @@ __global__ void __launch_bounds__(ENV_WARPS * 32) envelope_kernel(const EnvDev *
     }
     if (z.v == 0.0 || z.e + 2 > C.exp_limit || z.e < -C.exp_limit) flag = 2;
     const double zinv = z.v > 0.0 ? 1.0 / z.v : 0.0;
-
-    // ---- reverse, combined row by row with the stored forward rows
-    int er = 0;
+    const double gopen_inv = 1.0 / C.gopen1;
     const double thr_hi = C.min_prob * (1.0 + C.mu), thr_lo = C.min_prob * (1.0 - C.mu);
-    for (int r = 0; r <= n; ++r) {
-        double *cur = P.rz + (size_t)(r & 1) * rowsz;
-        if (r == 0) {
-            env_row0<true>(P, C, cur, C.rfe);
-        } else {
-            double zs = 0.0;
-            const double mx = env_row<true>(P, C, r, P.rz + (size_t)((r - 1) & 1) * rowsz, cur, er, C.rfe, &zs);
-            __syncwarp();
-            const int d = exp_of(mx);
-            env_scale(cur, m1, d);
-            er += d;
-            if (er + 2 > C.exp_limit) flag = 2;
-        }
-        __syncwarp();
-        // edge probabilities of forward row i = n - r (edge_probs.icc:238-262)
-        // and the row's threshold (trace_controller.cc:568-579)
-        const int i = n - r;
-        const double *f = P.fz + (size_t)i * rowsz;
-        const int ef = P.fexp[i];
+    int unsure = 0;
+    for (int i = warp; i <= n; i += ENV_THREADS / 32) {
+        // edge probabilities of forward row i with reverse row n - i
+        // (edge_probs.icc:238-262) and the row's threshold
+        // (trace_controller.cc:568-579)
+        const double *f = P.fz + (size_t)i * rowsz, *cur = P.rz + (size_t)(n - i) * rowsz;
+        const int er = P.rexp[n - i], k = P.fexp[i] + er - z.e;
         const double locs = C.local ? ldexp(1.0, -er) : 0.0;
         const int lo = P.minc[i], hi = P.maxc[i];
         int nmin = hi, nmax = lo, umin = INT_MAX, umax = INT_MIN;
+        // p = zij / z 2^k is compared as zij / z with the thresholds 2^-k, which
+        // is exact while those stay in the normal range
+        const bool direct = k > -900 && k < 900;
+        const double t_hi = direct ? ldexp(thr_hi, -k) : thr_hi, t_lo = direct ? ldexp(thr_lo, -k) : thr_lo;
         for (int j = max(lo, 0) + lane; j <= min(hi, m); j += 32) {
             const int jr = m - j;
             const double rM = cur[jr], rA = cur[m1 + jr], rB = cur[2 * m1 + jr];
-            const double zij = f[j] * (rM + rA + rB + locs) + f[m1 + j] * (rM + rA / C.gopen1 + rB) +
-                               f[2 * m1 + j] * (rM + rA + rB / C.gopen1);
-            const double p = ldexp(zij * zinv, ef + er - z.e);
-            if (p >= thr_hi) {
+            const double zij = f[j] * (rM + rA + rB + locs) + f[m1 + j] * (rM + rA * gopen_inv + rB) +
+                               f[2 * m1 + j] * (rM + rA + rB * gopen_inv);
+            const double p = direct ? zij * zinv : ldexp(zij * zinv, k);
+            if (p >= t_hi) {
                 nmin = min(nmin, j);
                 nmax = max(nmax, j);
-            } else if (p >= thr_lo) {
+            } else if (p >= t_lo) {
                 umin = min(umin, j);
                 umax = max(umax, j);
             }
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            nmin = min(nmin, __shfl_xor_sync(0xffffffffu, nmin, off));
-            nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, off));
-            umin = min(umin, __shfl_xor_sync(0xffffffffu, umin, off));
-            umax = max(umax, __shfl_xor_sync(0xffffffffu, umax, off));
-        }
-        if (umin < nmin || umax > nmax) flag = flag ? flag : 1;
+        nmin = __reduce_min_sync(0xffffffffu, nmin);
+        nmax = __reduce_max_sync(0xffffffffu, nmax);
+        umin = __reduce_min_sync(0xffffffffu, umin);
+        umax = __reduce_max_sync(0xffffffffu, umax);
+        if (umin < nmin || umax > nmax) unsure = 1;
         if (lane == 0) {
             P.newmin[i] = nmin;
             P.newmax[i] = nmax;
         }
-        __syncwarp();
     }
-    if (lane == 0) *P.flag = flag;
+    if (lane == 0 && unsure) flags[2] = 1;  // (any writer writes the same)
+    __syncthreads();
+    if (threadIdx.x == 0) *P.flag = flag ? flag : flags[2];
 }
 
 size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -358,12 +459,12 @@ static EnvConst make_const(const Params &Pm) {
 
 static size_t wave_end(const PairIn *in, int q0, int npairs) {
     // waves of pairs whose forward rows fit a device budget
-    const size_t budget = (size_t)6 << 30;
+    const size_t budget = (size_t)16 << 30;
     size_t fz_bytes = 0;
     int q1 = q0;
     for (; q1 < npairs; ++q1) {
         const size_t n1 = (size_t)in[q1].n + 1, m1 = (size_t)in[q1].m + 1;
-        const size_t f = 8 * (3 * n1 * m1 + 6 * m1) + 4 * n1;
+        const size_t f = 8 * 7 * n1 * m1 + 8 * n1;
         if (q1 > q0 && fz_bytes + f > budget) break;
         fz_bytes += f;
     }
@@ -459,7 +560,7 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
     dev_off.resize(nq);
     for (int k = 0; k < nq; ++k) {
         const size_t n1 = (size_t)in[q0 + k].n + 1, m1 = (size_t)in[q0 + k].m + 1;
-        dev_off[k] = take(ds, 8 * (3 * n1 * m1 + 6 * m1) + 4 * n1);
+        dev_off[k] = take(ds, 8 * 7 * n1 * m1 + 8 * n1);
     }
     // the buffers are reused only after the previous computation ended
     // (compute waits; a pending one is ended before the next begins)
@@ -485,7 +586,13 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
     }
     char *H = eng->env_host, *D = eng->env_dev;
     EnvDev *hp = (EnvDev *)(H + o_pairs);
-    for (int k = 0; k < nq; ++k) {
+    // the largest pairs first: they take longest, and blocks start in this order
+    std::vector<int> order(nq);
+    for (int k = 0; k < nq; ++k) order[k] = k;
+    auto area = [&](int k) { return (long long)in[q0 + k].n * in[q0 + k].m; };
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return area(x) > area(y); });
+    for (int r = 0; r < nq; ++r) {
+        const int k = order[r];
         const PairIn &p = in[q0 + k];
         const int n1 = p.n + 1, m1 = p.m + 1;
         char *h = H + in_off[k];
@@ -501,7 +608,7 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
         signed char *ca = (signed char *)(suB + m1), *cb = ca + n1;
         std::memcpy(ca, p.ca, n1);
         std::memcpy(cb, p.cb, m1);
-        EnvDev &v = hp[k];
+        EnvDev &v = hp[r];
         v.n = p.n;
         v.m = p.m;
         v.minc = (const int *)d;
@@ -519,7 +626,9 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
         char *dd = D + dev_off[k];
         v.fz = (double *)dd;
         v.rz = v.fz + 3ull * n1 * m1;
-        v.fexp = (int *)(v.rz + 6ull * m1);
+        v.wt = v.rz + 3ull * n1 * m1;
+        v.fexp = (int *)(v.wt + (size_t)n1 * m1);
+        v.rexp = v.fexp + n1;
     }
     cudaStream_t st = eng->stream;
     auto fail_cuda = [&](cudaError_t x, const char *what) {
@@ -529,8 +638,16 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
     };
     if ((ce = cudaMemcpyAsync(D, H, out_begin, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return fail_cuda(ce, "envelope upload");
-    const int blocks = (nq + ENV_WARPS - 1) / ENV_WARPS;
-    envelope_kernel<<<blocks, ENV_WARPS * 32, 0, st>>>((const EnvDev *)(D + o_pairs), nq, C);
+    int max_n = 1, max_m = 1;
+    for (int k = 0; k < nq; ++k) {
+        max_n = std::max(max_n, in[q0 + k].n);
+        max_m = std::max(max_m, in[q0 + k].m);
+    }
+    env_weights_kernel<<<dim3(nq, (max_n + 7) / 8), 256, 0, st>>>((const EnvDev *)(D + o_pairs), C);
+    const size_t smem = std::min<size_t>(ENV_ROW_SMEM, 4 * 3 * sizeof(double) * (size_t)(max_m + 1));
+    if ((ce = cudaFuncSetAttribute(envelope_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return fail_cuda(ce, "envelope launch");
+    envelope_kernel<<<nq, ENV_THREADS, smem, st>>>((const EnvDev *)(D + o_pairs), C, smem);
     if ((ce = cudaGetLastError()) != cudaSuccess) return fail_cuda(ce, "envelope launch");
     if ((ce = cudaMemcpyAsync(H + out_begin, D + out_begin, out_end - out_begin, cudaMemcpyDeviceToHost, st)) !=
         cudaSuccess)
