@@ -233,8 +233,11 @@ lcg_status lcg_engine_set_graphs(lcg_engine eng, int32_t on);
  * group's rectangle instead of recomputing it (the reference recomputes too,
  * trace_arcmatch, aligner.cc:967-1028); the results are the same. Single
  * pairs and small batches; not with --noLP. bytes = 0 always recomputes;
- * bytes < 0 restores the default budgets, 4 GiB for plain chunks and 32 GiB
- * for structure-local chunks (a 400 x 400 nt pair takes ~25 GB).
+ * bytes < 0 restores the default budgets, 4 GiB for plain chunks, 16 GiB for
+ * batches filled lane per group (whose storage holds whole band rows of 32 or
+ * 64 groups) and 32 GiB for structure-local chunks (a 400 x 400 nt pair takes
+ * ~25 GB). Where the device has not that much memory left, the chunk
+ * recomputes.
  * LocARNA-P (lcg_pf_forward / lcg_pf_backward) keeps the groups' M (and E, F
  * for the gap gradients) from the forward for the backward pass under the
  * same budget, by default in FP64 only (4 GiB; in FP32 the backward's

@@ -793,6 +793,7 @@ struct Chunk {
     // and the L2 budget of a pair wave in MB (0 = default)
     int bps = 0;
     double wave_mb = 0;
+    bool no_keep = false;  // the kept rectangles did not fit the device's memory
 };
 
 // Groups per item of the lane-per-group fill for a chunk, 0: one warp per group
@@ -943,9 +944,13 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     const long long rect_bytes_per_cell = opts->struct_local ? 32 : 4;
     bool keep;
     {
+        bool lanes = false;
+        for (auto &p : prep) lanes = lanes || (p.flags & PF_LANES);
         const long long budget = e->rect_budget >= 0 ? e->rect_budget
-                                                     : (opts->struct_local ? RECT_BUDGET_SL : RECT_BUDGET_PLAIN);
-        keep = budget > 0;
+                                 : opts->struct_local ? RECT_BUDGET_SL
+                                 : lanes              ? RECT_BUDGET_LANES
+                                                      : RECT_BUDGET_PLAIN;
+        keep = budget > 0 && !c.no_keep;
         double bytes = 0;
         for (auto &p : prep) {
             const bool ln = p.flags & PF_LANES;
@@ -1082,8 +1087,14 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         if (*s.d_arena) cudaFree(*s.d_arena);
         *s.d_arena = nullptr;
         *s.arena_cap = 0;
-        size_t cap = total + total / 4;
-        if (cudaMalloc(s.d_arena, cap) != cudaSuccess) return fail(LCG_ERR_NOMEM, "device arena allocation failed");
+        const size_t cap = total + std::min<size_t>(total / 4, (size_t)1 << 30);
+        if (cudaMalloc(s.d_arena, cap) != cudaSuccess) {
+            cudaGetLastError();
+            *s.d_arena = nullptr;
+            if (!keep) return fail(LCG_ERR_NOMEM, "device arena allocation failed");
+            c.no_keep = true;  // without the kept rectangles
+            return chunk_launch(e, s, all, opts, c, pack_ms);
+        }
         *s.arena_cap = cap;
     }
     if (down_end > *s.stage_cap) {
@@ -1786,6 +1797,7 @@ static lcg_status align_impl(lcg_engine e, const lcg_pair_tables *pairs, int32_t
         c.nq = nq;
         c.bps = plan[k].bps;
         c.wave_mb = plan[k].wave_mb;
+        c.no_keep = false;
         rc = chunk_launch(e, s, pairs, opts, c, &t_pack);
     }
     // the chunks still in flight, in batch order; after an error only wait

@@ -45,6 +45,9 @@ struct lcg_buffer_set {
 // structure-local chunks, whose rectangles hold eight state matrices
 constexpr long long RECT_BUDGET_PLAIN = 4ll << 30;
 constexpr long long RECT_BUDGET_SL = 32ll << 30;
+// chunks filled lane per group, whose item storages would be as large in the
+// warps' slots (45 stacking pairs of 100-300 nt, 4.5 GB: traceback 2.6 -> 0.2 ms)
+constexpr long long RECT_BUDGET_LANES = 16ll << 30;
 
 struct lcg_engine_s {
     int device = 0;

@@ -88,19 +88,20 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
     Walker w(P);
     int nseg = 0;
     int qhead = 0;
-    if (lane == 0) {
-        if (!(sel.flags & TRACE_KEEP_MIN)) {
-            P.res[R_MINI] = 1;
-            P.res[R_MINJ] = 1;
-        }
+    if (lane == 0 && !(sel.flags & TRACE_KEEP_MIN)) {
+        P.res[R_MINI] = 1;
+        P.res[R_MINJ] = 1;
+    }
+    __syncwarp();
+    {
         const int sA = sel.rst ? sel.rst[pair].x : 1, sB = sel.rst ? sel.rst[pair].y : 1;
         walk<false>(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), P.m + 1, sA - 1, sB - 1, P.res[R_MAXI],
              P.res[R_MAXJ], true, status, lam);
-        P.segs[nseg++] = make_int4(-1, 0, w.ntok, 0);
+        if (lane == 0) P.segs[0] = make_int4(-1, 0, w.ntok, 0);
+        nseg = 1;
     }
     if (sel.flags & TRACE_TOP_ONLY) return;
-    int qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
-    while (qhead < qtail) {
+    while (qhead < w.qtail) {
         int4 qe = make_int4(-1, 0, 0, 0);
         if (lane == 0 && qhead < P.tq_cap) qe = P.tq[qhead];
         const int k = __shfl_sync(0xffffffffu, qe.x, 0), kaux = __shfl_sync(0xffffffffu, qe.y, 0);
@@ -110,15 +111,16 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         const int4 ends = trace_ends(lefts, rights);  // a.l, a.r, b.l, b.r
         if (lefts & TQ_CHAIN) {
             if (lane == 0) trace_chain(w, k, kaux, ends, nseg, status);
-            __syncwarp();
-            qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
+            w.share();
+            nseg = __shfl_sync(0xffffffffu, nseg, 0);
             continue;
         }
         if ((P.flags & (PF_STACK | PF_NOLP)) == PF_STACK) {
             int stacked = 0;
             if (lane == 0) stacked = trace_stack(w, k, kaux, ends, nseg);
             if (__shfl_sync(0xffffffffu, stacked, 0)) {
-                qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
+                w.share();
+                nseg = __shfl_sync(0xffffffffu, nseg, 0);
                 continue;
             }
         }
@@ -138,15 +140,12 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
                                            true, true, false, status, (volatile int *)&dummy_abort, nullptr);
         }
         __syncwarp();
-        if (lane == 0) {
-            const int start = w.ntok;
-            if (kept && lanes) walk<true>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
-            else walk<false>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
-            if (nseg < P.tq_cap + 1) P.segs[nseg] = make_int4(k, start, w.ntok, 0);
-            ++nseg;
-        }
+        const int start = w.ntok;
+        if (kept && lanes) walk<true>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
+        else walk<false>(w, Mw, pw, ends.x, ends.z, ends.y - 1, ends.w - 1, false, status);
+        if (lane == 0 && nseg < P.tq_cap + 1) P.segs[nseg] = make_int4(k, start, w.ntok, 0);
+        ++nseg;
         __syncwarp();
-        qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
     }
     if (lane == 0) {
         P.res[R_NTOK] = w.ntok;

@@ -699,45 +699,54 @@ __global__ void __launch_bounds__(SL_FILL_WARPS * 32)
 
 // ---------------------------------------------------------------- traceback
 
-// trace_in_arcmatch (aligner.cc:1233-1343) as a loop over (state, i, j);
-// M of state s is Mg + s*mstride (the top level has only state NO_NO).
+// trace_in_arcmatch (aligner.cc:1233-1343) as a loop over (state, i, j), by a
+// whole warp; M of state s is Mg + s*mstride (the top level has only state
+// NO_NO).
 static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long mstride, int pitch,
                                             int al, int bl, int state, int i, int j, bool tl,
                                             int *status, int lam = 0) {
     const PairDev &P = w.P;
-    const int tlam = tl ? lam : 0;  // top level of normalized / penalized alignment
     const bool local = P.flags & PF_SEQU_LOCAL;
     const int fe = P.free_endgaps;
-    const int go = P.go, X = P.excl;
+    const int X = P.excl, lane = threadIdx.x & 31;
 #define MS(s, x, y) Mg[(long long)(s) * mstride + (long long)((x) - al) * pitch + ((y) - bl)]
+    // cells above (left of) (i, j) in `state` that hold the same value, up to 32
+    auto run_up = [&](int Mij) {
+        const unsigned no = __ballot_sync(0xffffffffu, !(i - lane > al && MS(state, i - lane - 1, j) == Mij));
+        return no ? __ffs(no) - 1 : 32;
+    };
+    auto run_left = [&](int Mij) {
+        const unsigned no = __ballot_sync(0xffffffffu, !(j - lane > bl && MS(state, i, j - lane - 1) == Mij));
+        return no ? __ffs(no) - 1 : 32;
+    };
     for (int guard = 0; guard < 8 * (P.n + P.m + 4); ++guard) {
         const int Mij = MS(state, i, j);
         if (tl && local && Mij == 0) {
-            P.res[R_MINI] = i;
-            P.res[R_MINJ] = j;
+            if (lane == 0) {
+                P.res[R_MINI] = i;
+                P.res[R_MINJ] = j;
+            }
             return;
         }
         if (i <= al) {
             if (state == S_NO_NO || state == S_OP_NO || state == S_X_NO)
-                if (!(tl && (local || (fe & 1))))
-                    for (int k = j; k > bl; --k) w.emit(-1, k);
+                if (!(tl && (local || (fe & 1)))) w.emit_run(max(j - bl, 0), -1, 0, j, 1);
             return;
         }
         if (j <= bl) {
             if (state == S_NO_NO || state == S_NO_OP || state == S_NO_X)
-                if (!(tl && (local || (fe & 4))))
-                    for (int k = i; k > al; --k) w.emit(k, -1);
+                if (!(tl && (local || (fe & 4)))) w.emit_run(max(i - al, 0), i, 1, -1, 0);
             return;
         }
         bool noex = false;
         switch (state) {
         case S_NO_NO: noex = true; break;
         case S_OP_NO:
-            if (Mij == MS(state, i - 1, j)) { --i; continue; }
+            if (const int r = run_up(Mij)) { i -= r; continue; }
             if (Mij == MS(S_NO_NO, i, j)) { state = S_NO_NO; continue; }
             return;
         case S_NO_OP:
-            if (Mij == MS(state, i, j - 1)) { --j; continue; }
+            if (const int r = run_left(Mij)) { j -= r; continue; }
             if (Mij == MS(S_NO_NO, i, j)) { state = S_NO_NO; continue; }
             return;
         case S_NO_X:
@@ -745,7 +754,7 @@ static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long 
             noex = true;
             break;
         case S_OP_X:
-            if (Mij == MS(state, i - 1, j)) { --i; continue; }
+            if (const int r = run_up(Mij)) { i -= r; continue; }
             if (Mij == MS(S_NO_X, i, j)) { state = S_NO_X; continue; }
             return;
         case S_X_NO:
@@ -753,7 +762,7 @@ static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long 
             noex = true;
             break;
         case S_X_OP:
-            if (Mij == MS(state, i, j - 1)) { --j; continue; }
+            if (const int r = run_left(Mij)) { j -= r; continue; }
             if (Mij == MS(S_X_NO, i, j)) { state = S_X_NO; continue; }
             return;
         case S_X_X:
@@ -763,74 +772,12 @@ static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long 
             break;
         }
         if (!noex) return;
-        // trace_noex (aligner.cc:1082-1229) in `state`
-        if (a_match(P, i, j) && w.valid(i - 1, j - 1) &&
-            Mij == MS(state, i - 1, j - 1) + sigma_at(P, i, j) - 2 * tlam) {
-            w.emit(i, j);
-            --i;
-            --j;
-            continue;
-        }
-        bool found = false;
-        if (go == 0) {
-            if (a_del(P, i, j) && w.valid(i - 1, j) && Mij == MS(state, i - 1, j) + P.gapA[i] - tlam) {
-                w.emit(i, -1);
-                --i;
-                continue;
-            }
-            if (a_ins(P, i, j) && w.valid(i, j - 1) && Mij == MS(state, i, j - 1) + P.gapB[j] - tlam) {
-                w.emit(-1, j);
-                --j;
-                continue;
-            }
-        } else {
-            int gap = go;
-            for (int k = 1; i >= al + k && a_del(P, i - k + 1, j); ++k) {
-                if (!w.valid(i - k, j)) break;
-                gap += P.gapA[i - k + 1] - tlam;
-                if (Mij == MS(state, i - k, j) + gap) {
-                    for (int l = 1; l <= k; ++l) w.emit(i - l + 1, -1);
-                    i -= k;
-                    found = true;
-                    break;
-                }
-            }
-            if (found) continue;
-            gap = go;
-            for (int k = 1; j >= bl + k && a_ins(P, i, j - k + 1); ++k) {
-                if (!w.valid(i, j - k)) break;
-                gap += P.gapB[j - k + 1] - tlam;
-                if (Mij == MS(state, i, j - k) + gap) {
-                    for (int l = 1; l <= k; ++l) w.emit(-1, j - l + 1);
-                    j -= k;
-                    found = true;
-                    break;
-                }
-            }
-            if (found) continue;
-        }
-        if (!(a_match(P, i, j) && w.valid(i - 1, j - 1))) return;
-        const int cell = P.bandoff[i] + j - P.min_col[i];
-        for (int q = P.cre_start[cell]; q < P.cre_end[cell]; ++q) {
-            const int4 ent = P.cre[q];
-            const int alq = (ent.y & 0xffff) + 1, blq = (ent.y >> 16) + 1;
-            if (alq <= al || blq <= bl || !w.valid(alq - 1, blq - 1)) continue;
-            if (Mij == MS(state, alq - 1, blq - 1) + P.D[ent.x] - tlam * ((i - alq + 1) + (j - blq + 1))) {
-                w.emit(i, j);
-                w.emit(-2, ent.w);
-                w.emit(alq, blq);
-                if (w.qtail < P.tq_cap) P.tq[w.qtail] = trace_entry(P, ent.w, ent.x, alq, i, blq, j);
-                else w.ok = false;
-                ++w.qtail;
-                i = alq - 1;
-                j = blq - 1;
-                found = true;
-                break;
-            }
-        }
-        if (!found) return;
+        // trace_noex in `state`; the states with an exclusion open are looked
+        // at before every diagonal step
+        auto M = [&](int x, int y) { return MS(state, x, y); };
+        if (!walk_noex(w, M, al, bl, i, j, Mij, tl ? lam : 0, tl && local, state == S_NO_NO ? 32 : 1)) return;
     }
-    atomicOr(status, ST_INTERNAL);
+    if (lane == 0) atomicOr(status, ST_INTERNAL);
 #undef MS
 }
 
@@ -855,19 +802,20 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
     Walker w(P);
     int nseg = 0;
     int qhead = 0;
-    if (lane == 0) {
-        if (!(sel.flags & TRACE_KEEP_MIN)) {
-            P.res[R_MINI] = 1;
-            P.res[R_MINJ] = 1;
-        }
+    if (lane == 0 && !(sel.flags & TRACE_KEEP_MIN)) {
+        P.res[R_MINI] = 1;
+        P.res[R_MINJ] = 1;
+    }
+    __syncwarp();
+    {
         const int sA = sel.rst ? sel.rst[pair].x : 1, sB = sel.rst ? sel.rst[pair].y : 1;
         walk_sl(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), 0, P.m + 1, sA - 1, sB - 1, S_NO_NO,
                 P.res[R_MAXI], P.res[R_MAXJ], true, status, lam);
-        P.segs[nseg++] = make_int4(-1, 0, w.ntok, 0);
+        if (lane == 0) P.segs[0] = make_int4(-1, 0, w.ntok, 0);
+        nseg = 1;
     }
     if (sel.flags & TRACE_TOP_ONLY) return;
-    int qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
-    while (qhead < qtail) {
+    while (qhead < w.qtail) {
         int4 qe = make_int4(-1, 0, 0, 0);
         if (lane == 0 && qhead < P.tq_cap) qe = P.tq[qhead];
         const int k = __shfl_sync(0xffffffffu, qe.x, 0), kpos = __shfl_sync(0xffffffffu, qe.y, 0);
@@ -877,15 +825,16 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         const int4 ends = trace_ends(lefts, rights);  // a.l, a.r, b.l, b.r
         if (lefts & TQ_CHAIN) {
             if (lane == 0) trace_chain(w, k, kpos, ends, nseg, status);
-            __syncwarp();
-            qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
+            w.share();
+            nseg = __shfl_sync(0xffffffffu, nseg, 0);
             continue;
         }
         if ((P.flags & (PF_STACK | PF_NOLP)) == PF_STACK) {
             int stacked = 0;
             if (lane == 0) stacked = trace_stack(w, k, kpos, ends, nseg);
             if (__shfl_sync(0xffffffffu, stacked, 0)) {
-                qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
+                w.share();
+                nseg = __shfl_sync(0xffffffffu, nseg, 0);
                 continue;
             }
         }
@@ -907,27 +856,24 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
                                           nullptr, 0, status, (volatile int *)&dummy_abort);
         }
         __syncwarp();
-        if (lane == 0) {
-            // trace_arcmatch, struct-local branch (aligner.cc:1014-1026): first
-            // non-open state whose value explains D(am); for the inner arc
-            // match of a no-lonely-pairs stack (aligner.cc:1062-1074) the
-            // queue entry carries D(outer) - score(outer) - score(am)
-            const int ar = ends.y, br = ends.w;
-            const long long o = (long long)(ar - 1 - ends.x) * pw + (br - 1 - ends.z);
-            const bool nolp = P.flags & PF_NOLP;
-            const int dv = nolp ? kpos : P.D[kpos], sc = nolp ? 0 : P.am_score[k];
-            const int start = w.ntok;
-            for (int s2 = 0; s2 < 4; ++s2) {
-                if (dv == Mw[s2 * ms + o] + sc) {
-                    walk_sl(w, Mw, ms, pw, ends.x, ends.z, s2, ar - 1, br - 1, false, status);
-                    break;
-                }
+        // trace_arcmatch, struct-local branch (aligner.cc:1014-1026): first
+        // non-open state whose value explains D(am); for the inner arc
+        // match of a no-lonely-pairs stack (aligner.cc:1062-1074) the
+        // queue entry carries D(outer) - score(outer) - score(am)
+        const int ar = ends.y, br = ends.w;
+        const long long o = (long long)(ar - 1 - ends.x) * pw + (br - 1 - ends.z);
+        const bool nolp = P.flags & PF_NOLP;
+        const int dv = nolp ? kpos : P.D[kpos], sc = nolp ? 0 : P.am_score[k];
+        const int start = w.ntok;
+        for (int s2 = 0; s2 < 4; ++s2) {
+            if (dv == Mw[s2 * ms + o] + sc) {
+                walk_sl(w, Mw, ms, pw, ends.x, ends.z, s2, ar - 1, br - 1, false, status);
+                break;
             }
-            if (nseg < P.tq_cap + 1) P.segs[nseg] = make_int4(k, start, w.ntok, 0);
-            ++nseg;
         }
+        if (lane == 0 && nseg < P.tq_cap + 1) P.segs[nseg] = make_int4(k, start, w.ntok, 0);
+        ++nseg;
         __syncwarp();
-        qtail = __shfl_sync(0xffffffffu, w.qtail, 0);
     }
     if (lane == 0) {
         P.res[R_NTOK] = w.ntok;
