@@ -505,22 +505,30 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
     }
     if (!p.device_index) p.Dinit.assign(p.num_pos, NEG);
     std::vector<int> ks;
-    // band cells of rows [r0, r1) inside columns [A, B], in O(log n) from
-    // prefix sums (min_col and max_col are nondecreasing)
+    // band cells of rows [r0, r1) inside columns [A, B], from prefix sums and,
+    // per column, the rows whose band starts (ends) left of it (min_col and
+    // max_col are nondecreasing)
     std::vector<long long> psmin(n + 2, 0), psmax(n + 2, 0);
     for (int i = 0; i <= n; ++i) {
         psmin[i + 1] = psmin[i] + p.min_col[i];
         psmax[i + 1] = psmax[i] + p.max_col[i];
     }
+    std::vector<int> begun(m + 2, 0), ended(m + 3, 0);  // rows with min_col <= j, rows with max_col < j
+    for (int j = 0, r = 0; j <= m + 1; ++j) {
+        while (r <= n && p.min_col[r] <= j) ++r;
+        begun[j] = r;
+    }
+    for (int j = 0, r = 0; j <= m + 2; ++j) {
+        while (r <= n && p.max_col[r] < j) ++r;
+        ended[j] = r;
+    }
     auto rect_cells = [&](int r0, int r1, int A, int B) -> long long {
         if (r0 >= r1 || A > B) return 0;
-        const int *mn = p.min_col.data(), *mx = p.max_col.data();
         // rows whose band lies left of A (max_col < A) or right of B (min_col > B) are empty
-        const int u = (int)(std::lower_bound(mx + r0, mx + r1, A) - mx);
-        const int v = (int)(std::upper_bound(mn + r0, mn + r1, B) - mn);
+        const int u = std::min(std::max(ended[A], r0), r1), v = std::min(std::max(begun[B], r0), r1);
         if (u >= v) return 0;
-        const int x = (int)(std::upper_bound(mx + u, mx + v, B) - mx);  // rows [u,x): max_col <= B
-        const int y = (int)(std::upper_bound(mn + u, mn + v, A) - mn);  // rows [u,y): min_col <= A
+        const int x = std::min(std::max(ended[B + 1], u), v);  // rows [u,x): max_col <= B
+        const int y = std::min(std::max(begun[A], u), v);      // rows [u,y): min_col <= A
         const long long shi = (psmax[x] - psmax[u]) + (long long)B * (v - x);
         const long long slo = (long long)A * (y - u) + (psmin[v] - psmin[y]);
         return shi - slo + (v - u);

@@ -322,6 +322,9 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         d.gA = (const T *)(Dv + L0.gA);
         d.gB = (const T *)(Dv + L0.gB);
         d.o = (T)ow;
+        d.gu = hgB[1];
+        for (int j = 2; j <= m && d.gu > T(0); ++j)
+            if (hgB[j] != hgB[1]) d.gu = T(0);
         d.inv_s = (T)(1.0 / pf_scale);
         d.arcf = (T)(pf_scale / (c2 * c2));
         d.w = (const T *)(Dv + L0.w);

@@ -69,6 +69,34 @@ __device__ __forceinline__ T pf_wait(const T *p, int *status, volatile int *abor
     return v;
 }
 
+// The gap chains' factors of a pair whose columns all have the same gap weight
+// g (single sequences): g^1, 2, 4, 8, 16 for the warp scans and g^(lane+1),
+// g^(32-lane) for their carries. FP64 arithmetic is what bounds the FP64
+// passes (an SM issues two FP64 operations a clock), and the scan with constant
+// factors takes 5 multiply-adds a cell instead of 10.
+template <typename T>
+struct PFPow {
+    T p[5];
+};
+template <typename T>
+__device__ __forceinline__ PFPow<T> pf_pow(T g) {
+    PFPow<T> w;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        w.p[k] = g;
+        g *= g;
+    }
+    return w;
+}
+template <typename T>
+__device__ __forceinline__ T pf_power(const PFPow<T> &w, int n) {  // g^n, 1 <= n <= 32
+    T x = T(1);
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        if (n >> k & 1) x *= w.p[k];
+    return n == 32 ? w.p[4] * w.p[4] : x;
+}
+
 extern __shared__ unsigned char pf_smem_raw[];
 
 // Shared-memory rows per warp (T each), ring buffers of rb entries (a
@@ -115,6 +143,9 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
     const int lane = threadIdx.x & 31;
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
+    const bool uni = P.gu > T(0);
+    const PFPow<T> W = pf_pow(P.gu);
+    const T guo = P.gu * o, wl = pf_power(W, lane + 1);
 #define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
     // E and the arc-term sums start at zero; the cell sweep puts zero back
     // into every arc-term column it reads, so no row needs a clearing pass
@@ -178,8 +209,8 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
         const int2 ra = P.rowarc[i];
         const int minc = ri.x;
         const int lo = max(bl + 1, minc), hi = min(br - 1, ri.y);
-        const T gAi = P.gA[i];
-        // ---- arc-match terms of row i into Ar[lo..hi]: two batches of 32
+        const T gAi = P.gA[i], gAo = gAi * o;
+        // ---- arc-match terms of row i into Ar[lo..hi] (without the factor s): two batches of 32
         // entries per step, their loads issued together
         bool rowarcs = false;
         for (int e0 = ra.x; e0 < ra.y; e0 += 64) {
@@ -214,7 +245,7 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
                 if (ok[u]) {
                     const int e = e0 + 32 * u + lane;
                     if (WAIT && pf_not_ready(dv[u])) dv[u] = pf_wait(P.D + e, status, abort_flag);
-                    atomicAdd(&R.Ar[RG(en[u].y)], mv[u] * dv[u] * arcf);
+                    atomicAdd(&R.Ar[RG(en[u].y)], mv[u] * dv[u]);
                     if (COUNTU) atomicAdd(P.cnt + e, 1);
                 }
             }
@@ -247,38 +278,49 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
             const bool act = j <= hi;
             T X = T(0), Ei = T(0), g = T(0);
             if (act) {
-                Ei = R.E[RG(j)] * gAi + R.Np[RG(j)] * gAi * o;
+                Ei = R.E[RG(j)] * gAi + R.Np[RG(j)] * gAo;
                 X = R.Mp[RG(j - 1)] * bmrow[j];
                 if (rowarcs) {
-                    X += R.Ar[RG(j)];
+                    X += R.Ar[RG(j)] * arcf;
                     R.Ar[RG(j)] = T(0);
                 }
-                g = P.gB[j];
+                if (!uni) g = P.gB[j];
             }
             // F(j) = gB(j) F(j-1) + gB(j) o Q(j-1): linear warp scan
             const T Q = X + Ei;
             T Qp = __shfl_up_sync(0xffffffffu, Q, 1);
             if (lane == 0) Qp = Qc;
-            T a = T(1), b = T(0);
-            if (act) {
-                a = g;
-                b = g * o * Qp;
-            }
+            T F;
+            if (uni) {
+                T b = Qp * guo;  // (past the row's end: zeros and what no one reads)
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const T a1 = __shfl_up_sync(0xffffffffu, a, off);
-                const T b1 = __shfl_up_sync(0xffffffffu, b, off);
-                if (lane >= off) {
-                    b = a * b1 + b;
-                    a = a * a1;
+                for (int k = 0; k < 5; ++k) {
+                    const T b1 = __shfl_up_sync(0xffffffffu, b, 1 << k);
+                    if (lane >= 1 << k) b += W.p[k] * b1;
                 }
+                F = wl * Fc + b;
+            } else {
+                T a = T(1), b = T(0);
+                if (act) {
+                    a = g;
+                    b = g * o * Qp;
+                }
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const T a1 = __shfl_up_sync(0xffffffffu, a, off);
+                    const T b1 = __shfl_up_sync(0xffffffffu, b, off);
+                    if (lane >= off) {
+                        b = a * b1 + b;
+                        a = a * a1;
+                    }
+                }
+                F = a * Fc + b;
             }
-            const T F = a * Fc + b;
             if (act) {
-                const T M = X + Ei + F;
+                const T N = X + F, M = N + Ei;
                 R.E[RG(j)] = Ei;
                 R.Mc[RG(j)] = M;
-                R.Nc[RG(j)] = X + F;
+                R.Nc[RG(j)] = N;
                 Mg[roff + j] = M;
                 if (SAVE && SAVEEF) {
                     Eg[roff + j] = Ei;
@@ -400,6 +442,9 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
     const int lane = threadIdx.x & 31;
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
+    const bool uni = P.gu > T(0);
+    const PFPow<T> W = pf_pow(P.gu);
+    const T guo = P.gu * o, wr = pf_power(W, 32 - lane);
     T *const Eb = R.E;
     T *const Xb = R.Ar;
     // diagonal adjoint contributions X_bar(i,j) bm(i,j) to M_bar(i-1,j-1):
@@ -434,6 +479,8 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
         const int lo = max(bl + 1, minc), hi = min(br - 1, ri.y);
         const T gAi = P.gA[i];
         const T gAn = (i + 1 < ar) ? P.gA[i + 1] : T(0);
+        const T gAo = gAi * o, gAno = gAn * o;
+        T opnE = T(0);  // GRADS: the row's vertical gap openings without their weight
         // seeds: dZ'/dD(am) w(am) into M(ar-1, br-1) once every use of D(am)
         // has been back-propagated
         while (dwp >= 0) {
@@ -487,7 +534,7 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
                 Mbar = ld_cg(Mb + roff + c) + Dc[RG(j)];
                 Dc[RG(j)] = T(0);
                 Ebn = Eb[RG(j)];  // E_bar(i+1, j)
-                g = P.gB[j];
+                if (!uni) g = P.gB[j];
                 if (GRADS) {
                     Ev = Eg[roff + c];
                     Fv = Fg[roff + c];
@@ -497,10 +544,11 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
                 Mup = Mg[roff - pitch + c];
                 bmj = bmrow[j];
             }
-            T gn = __shfl_down_sync(0xffffffffu, g, 1);  // gB(j+1); 0 past the row's end
+            T gn = T(0);  // gB(j+1); 0 past the row's end
+            if (!uni) gn = __shfl_down_sync(0xffffffffu, g, 1);
             T Ml = __shfl_up_sync(0xffffffffu, Mv, 1), Fl = __shfl_up_sync(0xffffffffu, Fv, 1);
             T Md = __shfl_up_sync(0xffffffffu, Mup, 1);
-            if (lane == 31 && act) gn = (j + 1 <= hi) ? P.gB[j + 1] : T(0);
+            if (!uni && lane == 31 && act) gn = (j + 1 <= hi) ? P.gB[j + 1] : T(0);
             if (lane == 0 && act) {
                 if (GRADS) {
                     Ml = Mg[roff + c - 1];
@@ -508,49 +556,64 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
                 }
                 Md = Mg[roff - pitch + c - 1];
             }
-            const T Nbar = act ? Ebn * gAn * o : T(0);  // N(i,j) feeds E(i+1,j)
+            const T Nbar = Ebn * gAno;  // N(i,j) feeds E(i+1,j); 0 past the row's end
+            const T MN = Mbar + Nbar;
             // F_bar(j) = gB(j+1) F_bar(j+1) + (M_bar + N_bar)(j), right to left
-            T a = T(1), b = T(0);
-            if (act) {
-                a = gn;
-                b = Mbar + Nbar;
-            }
+            T Fb;
+            if (uni) {
+                T b = MN;
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const T a2 = __shfl_down_sync(0xffffffffu, a, off);
-                const T b2 = __shfl_down_sync(0xffffffffu, b, off);
-                if (lane + off < 32) {
-                    b = a * b2 + b;
-                    a = a * a2;
+                for (int k = 0; k < 5; ++k) {
+                    const T b2 = __shfl_down_sync(0xffffffffu, b, 1 << k);
+                    if (lane + (1 << k) < 32) b += W.p[k] * b2;
                 }
+                Fb = wr * Fbc + b;
+            } else {
+                T a = T(1), b = T(0);
+                if (act) {
+                    a = gn;
+                    b = MN;
+                }
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const T a2 = __shfl_down_sync(0xffffffffu, a, off);
+                    const T b2 = __shfl_down_sync(0xffffffffu, b, off);
+                    if (lane + off < 32) {
+                        b = a * b2 + b;
+                        a = a * a2;
+                    }
+                }
+                Fb = a * Fbc + b;
             }
-            const T Fb = a * Fbc + b;
             T Fbr = __shfl_down_sync(0xffffffffu, Fb, 1);  // F_bar(i, j+1)
             if (lane == 31) Fbr = Fbc;
             if (act) {
-                const T Qbar = Fbr * gn * o;
-                const T Ebar = Mbar + Qbar + Ebn * gAn;
-                const T Xbar = Mbar + Nbar + Qbar;
+                const T Qbar = uni ? Fbr * guo : Fbr * gn * o;
+                const T Ebar = Mbar + (Qbar + Ebn * gAn);
+                const T Xbar = MN + Qbar;
                 Eb[RG(j)] = Ebar;
                 Xb[RG(j)] = Xbar;
                 // gap derivatives: E(i,j) = gA(i) (E(i-1,j) + N(i-1,j) o)
                 if (GRADS) {
                     ext += (double)(Ebar * Ev + Fb * Fv);
-                    opn += (double)(Ebar * (Mup - Eup) * gAi * o + Fb * (Ml - Fl) * g * o);
+                    opnE += Ebar * (Mup - Eup);
+                    opn += (double)(Fb * (Ml - Fl) * (uni ? guo : g * o));
                 }
                 // diagonal
+                const T Xd = Xbar * bmj;
                 if (j - 1 >= dlo && j - 1 <= dhi)
-                    Dn[RG(j - 1)] = Xbar * bmj;
+                    Dn[RG(j - 1)] = Xd;
                 else
-                    atomicAdd(Mb + roff - pitch + c - 1, Xbar * bmj);
-                atomicAdd(P.bmacc + cb + j, (double)(Xbar * Md * bmj));
+                    atomicAdd(Mb + roff - pitch + c - 1, Xd);
+                atomicAdd(P.bmacc + cb + j, (double)(Xd * Md));
                 // E(i,j) reads N(i-1,j) = M(i-1,j) - E(i-1,j); F(i,j) reads Q(i,j-1)
                 if (i - 1 == al || rup.x > j || rup.y < j)
-                    atomicAdd(Mb + roff - pitch + c, Ebar * gAi * o);
-                if (j == lo) atomicAdd(Mb + roff + c - 1, Fb * g * o);
+                    atomicAdd(Mb + roff - pitch + c, Ebar * gAo);
+                if (j == lo) atomicAdd(Mb + roff + c - 1, Fb * (uni ? guo : g * o));
             }
             Fbc = __shfl_sync(0xffffffffu, Fb, 0);
         }
+        if (GRADS) opn += (double)opnE * gAo;
         __syncwarp();
         // arc terms of row i: M_bar(corner) += X_bar D s', D_bar(am) += X_bar M(corner) s'
         // (two batches of 32 entries per step, loads issued together). The
@@ -602,8 +665,9 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (ok[u]) {
-                    atomicAdd(Mb + co[u], xb[u] * dv[u] * arcf);
-                    if (!TRUNC) atomicAdd(P.Dbar + e0 + 32 * u + lane, (double)(xb[u] * mv[u] * arcf));
+                    const T xs = xb[u] * arcf;
+                    atomicAdd(Mb + co[u], xs * dv[u]);
+                    if (!TRUNC) atomicAdd(P.Dbar + e0 + 32 * u + lane, (double)(xs * mv[u]));
                 }
             }
 #pragma unroll
