@@ -1079,6 +1079,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         o.topM = take(dev_only, 4ull * (p.n + 1) * (p.m + 1));
         const size_t rect_bytes = (p.flags & PF_LANES) ? 4ull * p.lane_groups * std::max<long long>(p.lane_lines, 1)
                                                        : (size_t)rect_bytes_per_cell * std::max<long long>(p.rect_cells, 1);
+        dev_only = align_up(dev_only, 256);  // whole lines of an item's storage
         o.rect = keep ? take(dev_only, rect_bytes) : 0;
     }
     // normalized / penalized alignment: per pair its penalty, the selected

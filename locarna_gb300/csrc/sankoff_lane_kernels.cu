@@ -139,9 +139,13 @@ __device__ __forceinline__ bool lane_inside(int cell0, int b0, int4 en) {
     return en.z >> 5 >= cell0 && en.y >> 16 >= b0;  // (a corner outside the band has cell 0)
 }
 
-// D of the copied entries (NOT_READY where still to be written), loads in flight on return
+// D of the copied entries (NOT_READY where still to be written), loads in
+// flight on return. At 32 groups an item the lines of their terms (store: line
+// 0) are sent for as well: 24 pairs of 80-130 nt 3.59 -> 3.43 ms, 12 of
+// 180-220 nt 6.53 -> 6.18; at 64 groups 9 pairs of 300-400 nt took 23.2 -> 23.3.
 template <int GW>
-__device__ __forceinline__ void lane_fetch_d(int sb, int raw, int cell0, int n, int (&d)[LaneShape<GW>::STEPS]) {
+__device__ __forceinline__ void lane_fetch_d(int sb, const int *store, int raw, int cell0, int n,
+                                             int (&d)[LaneShape<GW>::STEPS]) {
     const int lane = threadIdx.x & 31;
     const int *const D = lc_ptr<const int>(sb + LaneShape<GW>::CTX, LC_D);
     const int b0 = lc_int(sb + LaneShape<GW>::CTX, LC_B0);
@@ -150,7 +154,11 @@ __device__ __forceinline__ void lane_fetch_d(int sb, int raw, int cell0, int n, 
         d[k] = NEG;
         if (32 * k + lane < n) {
             const int4 en = *(const int4 *)&lcg_smem[raw + 4 * (32 * k + lane)];
-            if (lane_inside(cell0, b0, en)) d[k] = ld_volatile(D + en.x);
+            if (lane_inside(cell0, b0, en)) {
+                d[k] = ld_volatile(D + en.x);
+                if (GW == 1)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(store + ((en.z >> 5) - cell0) * 32));
+            }
         }
     }
 }
@@ -393,7 +401,7 @@ __device__ __forceinline__ void lane_group(const PairDev &P, const LaneItem &it,
     {
         const int4 w = lane_quad<GW>(sb, 0);
         if (w.x < 0) return;
-        lane_fetch_d<GW>(sb, sb + LaneShape<GW>::RAW, cell0, w.w, d);
+        lane_fetch_d<GW>(sb, store, sb + LaneShape<GW>::RAW, cell0, w.w, d);
         row_data(w.y);
     }
     int Mup[8][GW], V[8][GW];  // M and vertical-gap state max(E, M + go) of the row above
@@ -473,7 +481,7 @@ __device__ __forceinline__ void lane_group(const PairDev &P, const LaneItem &it,
         asm volatile("cp.async.wait_all;" ::: "memory");
         {
             const int4 x = lane_quad<GW>(sb, t + 1);
-            lane_fetch_d<GW>(sb, sb + LaneShape<GW>::RAW + (~t & 1) * 4 * LaneShape<GW>::ENTRIES, cell0, x.w, d);
+            lane_fetch_d<GW>(sb, store, sb + LaneShape<GW>::RAW + (~t & 1) * 4 * LaneShape<GW>::ENTRIES, cell0, x.w, d);
             row_data(x.x < 0 ? q : x.y);
         }
         __syncwarp();
