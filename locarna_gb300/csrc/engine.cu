@@ -1348,9 +1348,11 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     // ---- transfer + launch + transfer
     cudaStream_t st = s.st;
     // Without host steps between the launches (not normalized / penalized /
-    // k-best), the chunk's device work is one CUDA graph: captured from the
-    // stream on first use, replayed while the launch parameters (buffers,
-    // sizes, grid) stay the same, updated in place otherwise.
+    // k-best), the chunk's device work is one CUDA graph, replayed while the
+    // launch parameters (buffers, sizes, grid) stay the same. With new ones the
+    // work goes to the stream as it is and the graph is recorded behind it, for
+    // the calls to come, while the device is busy: recording and updating it
+    // first cost a new 60-nt pair 18 of 205 us and a 150-nt one 15 of 505.
     const bool use_graph = e->graphs && !modv && !c.kbest;
     std::vector<long long> key;
     if (use_graph) {
@@ -1375,68 +1377,13 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             e->last_d2h += 64 + (long long)(down_end - down_begin);
             return LCG_OK;
         }
-        CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     }
-    // timing events: inside a capture an event record becomes a graph node
-    // only when it is marked external
-    auto record = [&](cudaEvent_t ev) {
-        return use_graph ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal) : cudaEventRecord(ev, st);
-    };
-    // an error inside the capture ends it before returning
-    auto end_capture = [&]() {
-        if (!use_graph) return;
-        cudaGraph_t g = nullptr;
-        cudaStreamEndCapture(st, &g);
-        if (g) cudaGraphDestroy(g);
-    };
-#undef CUDA_TRY_CAP
-#define CUDA_TRY_CAP(call)                                                                      \
-    do {                                                                                        \
-        cudaError_t _e = (call);                                                                \
-        if (_e != cudaSuccess) {                                                                \
-            end_capture();                                                                      \
-            return fail(LCG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e));      \
-        }                                                                                       \
-    } while (0)
-    CUDA_TRY_CAP(cudaMemcpyAsync(Dv, H, down_begin, cudaMemcpyHostToDevice, st));
-    CUDA_TRY_CAP(cudaMemsetAsync(Dv + down_begin, 0, down_end - down_begin, st));
+    if (sl && e->counting) return fail(LCG_ERR_UNSUPPORTED, "work counting covers the plain mode only");
     unsigned int *qhead = (unsigned int *)(Dv + off_ctrl);
     int *status = (int *)(Dv + off_ctrl + 4);
     int *abort_flag = (int *)(Dv + off_ctrl + 8);
-    CUDA_TRY_CAP(record(s.ev0));
     unsigned long long *counters = e->counting ? (unsigned long long *)(Dv + off_ctrl + 16) : nullptr;
-    c.launches = 0;
-    if (index_lefts >= 0)
-        CUDA_TRY_CAP(launch_index((const PairDev *)(Dv + off_pairs), (const IndexPair *)(Dv + off_index), npairs,
-                                  index_n, index_lefts, st));
-    if (!of[1].empty()) {
-        CUDA_TRY_CAP(launch_lane_fill(lgroups, (const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_lqueue),
-                                      (int)nitems[1], scratch, lslot, lqslot, rb, lfast,
-                                      (unsigned int *)(Dv + off_ctrl + 32), status, abort_flag, lblocks, st));
-        ++c.launches;
-    }
-    if (sl) {
-        if (counters) {
-            end_capture();
-            return fail(LCG_ERR_UNSUPPORTED, "work counting covers the plain mode only");
-        }
-        CUDA_TRY_CAP(launch_sl_fill((const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_queue),
-                                (int)nitems[0], scratch, stride, sw, rb, sl_fast, keep, qhead,
-                                status, abort_flag, blocks, st));
-        ++c.launches;
-    } else if (!of[0].empty()) {
-        CUDA_TRY_CAP(launch_fill((const PairDev *)(Dv + off_pairs), (const int2 *)(Dv + off_queue),
-                             (int)nitems[0], scratch, stride, sw, rb, fast, qhead,
-                             status, abort_flag, blocks, st, counters));
-        ++c.launches;
-    }
-    CUDA_TRY_CAP(record(s.ev1));
-    TraceSel sel;
-    if (modv) {
-        lcg_status ms = mod_top_levels(opts, c, (const PairDev *)(Dv + off_pairs), (int *)(Dv + off_mod), npairs,
-                                       scratch, stride, sw, rb, sl, status, st, &sel);
-        if (ms != LCG_OK) return ms;
-    }
+    const PairDev *const d_pairs = (const PairDev *)(Dv + off_pairs);
     c.off_pairs = off_pairs;
     c.off_mod = off_mod;
     c.sw = sw;
@@ -1444,24 +1391,67 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     c.stride = stride;
     c.sl = sl;
     c.scratch = scratch;
-    if ((opts->do_trace || modv) && !c.kbest) {
-        if (sl)
-            CUDA_TRY_CAP(launch_sl_trace((const PairDev *)(Dv + off_pairs), npairs, scratch, stride, sw, rb,
-                                     sl_fast, status, st, sel));
-        else
-            CUDA_TRY_CAP(launch_trace((const PairDev *)(Dv + off_pairs), npairs, scratch, stride, sw, rb, status,
-                                  st, sel));
-        ++c.launches;
-    }
-    CUDA_TRY_CAP(record(s.ev2));
-    CUDA_TRY_CAP(cudaMemcpyAsync(H + off_ctrl, Dv + off_ctrl, 64, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY_CAP(cudaMemcpyAsync(H + down_begin, Dv + down_begin, down_end - down_begin, cudaMemcpyDeviceToHost, st));
+    // the chunk's device work onto the stream; into a capture its timing events
+    // go as external records, which alone become nodes of the graph
+    auto enqueue = [&](bool captured) -> lcg_status {
+        auto record = [&](cudaEvent_t ev) {
+            return captured ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal) : cudaEventRecord(ev, st);
+        };
+        CUDA_TRY(cudaMemcpyAsync(Dv, H, down_begin, cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemsetAsync(Dv + down_begin, 0, down_end - down_begin, st));
+        CUDA_TRY(record(s.ev0));
+        c.launches = 0;
+        if (index_lefts >= 0)
+            CUDA_TRY(launch_index(d_pairs, (const IndexPair *)(Dv + off_index), npairs, index_n, index_lefts, st));
+        if (!of[1].empty()) {
+            CUDA_TRY(launch_lane_fill(lgroups, d_pairs, (const int2 *)(Dv + off_lqueue), (int)nitems[1], scratch,
+                                      lslot, lqslot, rb, lfast, (unsigned int *)(Dv + off_ctrl + 32), status,
+                                      abort_flag, lblocks, st));
+            ++c.launches;
+        }
+        if (sl) {
+            CUDA_TRY(launch_sl_fill(d_pairs, (const int2 *)(Dv + off_queue), (int)nitems[0], scratch, stride, sw, rb,
+                                    sl_fast, keep, qhead, status, abort_flag, blocks, st));
+            ++c.launches;
+        } else if (!of[0].empty()) {
+            CUDA_TRY(launch_fill(d_pairs, (const int2 *)(Dv + off_queue), (int)nitems[0], scratch, stride, sw, rb,
+                                 fast, qhead, status, abort_flag, blocks, st, counters));
+            ++c.launches;
+        }
+        CUDA_TRY(record(s.ev1));
+        TraceSel sel;
+        if (modv) {
+            lcg_status ms = mod_top_levels(opts, c, d_pairs, (int *)(Dv + off_mod), npairs, scratch, stride, sw, rb,
+                                           sl, status, st, &sel);
+            if (ms != LCG_OK) return ms;
+        }
+        if ((opts->do_trace || modv) && !c.kbest) {
+            if (sl)
+                CUDA_TRY(launch_sl_trace(d_pairs, npairs, scratch, stride, sw, rb, sl_fast, status, st, sel));
+            else
+                CUDA_TRY(launch_trace(d_pairs, npairs, scratch, stride, sw, rb, status, st, sel));
+            ++c.launches;
+        }
+        CUDA_TRY(record(s.ev2));
+        CUDA_TRY(cudaMemcpyAsync(H + off_ctrl, Dv + off_ctrl, 64, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaMemcpyAsync(H + down_begin, Dv + down_begin, down_end - down_begin, cudaMemcpyDeviceToHost, st));
+        return LCG_OK;
+    };
+    const lcg_status es = enqueue(false);
+    if (es != LCG_OK) return es;
+    c.in_flight = true;
     if (use_graph) {
-        cudaGraph_t g = nullptr;
-        CUDA_TRY(cudaStreamEndCapture(st, &g));
-        // the set's graph updated in place, or instantiated again when the
-        // update is refused
+        // recorded, then the set's graph updated in place, or instantiated
+        // again when the update is refused
         lcg_graph_cache &gc = *s.graph;
+        cudaGraph_t g = nullptr;
+        CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        const lcg_status cs = enqueue(true);  // an error inside the capture ends it before returning
+        const cudaError_t ce = cudaStreamEndCapture(st, &g);
+        if (cs != LCG_OK || ce != cudaSuccess) {
+            if (g) cudaGraphDestroy(g);
+            return cs != LCG_OK ? cs : fail(LCG_ERR_CUDA, std::string("cudaStreamEndCapture: ") + cudaGetErrorString(ce));
+        }
         cudaGraphExecUpdateResultInfo info;
         if (!gc.exec || cudaGraphExecUpdate(gc.exec, g, &info) != cudaSuccess) {
             cudaGetLastError();  // a refused update leaves the runtime's last error set: clear it
@@ -1476,10 +1466,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         cudaGraphDestroy(g);
         gc.key = key;
         ++e->last_graph_captures;
-        CUDA_TRY(cudaGraphLaunch(gc.exec, st));
     }
-#undef CUDA_TRY_CAP
-    c.in_flight = true;
     e->last_h2d += (long long)down_begin;
     e->last_d2h += 64 + (long long)(down_end - down_begin);
     return LCG_OK;
