@@ -42,7 +42,7 @@ size_t up16(size_t x) { return (x + 15) / 16 * 16; }
 
 struct PFLayout {
     int n, m, na, npos, bandcells;  // npos: D entries (arc matches with a band cell as right ends)
-    size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, w, D, Dbar, cnt, bmacc, res, topM, rect;
+    size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, w, D, Dbar, cnt, bmacc, res, topM, topE, topF, rect;
     double log_c_total;  // (n+m) log c
 };
 
@@ -145,7 +145,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     size_t nitems = 0;
     int sw = 0, rows_max = 1, span = 2;
     for (auto &p : prep) {
-        nitems += p.groups.size();
+        nitems += p.groups.size() - 1;  // the top levels apart
         sw = std::max(sw, std::max(p.width_max + 1, p.m + 2));
         rows_max = std::max(rows_max, std::max(p.rows_max + 1, p.n + 1));
         // widest column range two consecutive band rows cover (plus the
@@ -196,7 +196,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     // reading the kept rectangle from DRAM (200-nt pair: backward 3.37 ms
     // recomputing, 3.60 ms kept; FP64 7.51 against 6.06 ms).
     const int rect_states = o->gap_gradients ? 3 : 1;
-    bool keep;
+    bool keep, top_ef;
     {
         const long long budget =
             e->rect_budget >= 0 ? e->rect_budget : (sizeof(T) == 8 ? RECT_BUDGET_PLAIN : 0);
@@ -207,7 +207,18 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
             cells += p.rect_cells;
         }
         keep = keep && (double)cells * rect_states * sizeof(T) <= (double)budget;
+        // E and F of the top levels, for the gap gradients
+        const double top_budget = (double)(e->rect_budget >= 0 ? e->rect_budget : RECT_BUDGET_PLAIN);
+        double top = 0;
+        for (auto &p : prep) top += 2.0 * sizeof(T) * (p.n + 1) * (p.m + 1);
+        top_ef = o->gap_gradients && (keep || top <= top_budget);
     }
+    if (top_ef)
+        for (int q = 0; q < npairs; ++q) {
+            PFLayout &L = S->lay[q];
+            L.topE = take(up, sizeof(T) * (L.n + 1) * (L.m + 1));
+            L.topF = take(up, sizeof(T) * (L.n + 1) * (L.m + 1));
+        }
     for (int q = 0; q < npairs; ++q)
         S->lay[q].rect = keep ? take(up, sizeof(T) * rect_states * std::max<long long>(prep[q].rect_cells, 1)) : 0;
     const size_t total = up;
@@ -237,7 +248,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         // against 8 MB ones: FP32 backward 335 -> 283 ms, FP64 841 -> 655 ms,
         // while the forward slows from 74 to 82 ms)
         std::vector<size_t> ng(npairs);
-        for (int q = 0; q < npairs; ++q) ng[q] = prep[q].groups.size();
+        for (int q = 0; q < npairs; ++q) ng[q] = prep[q].groups.size() - 1;
         auto bytes = [&](int q) {
             return (12.0 + 3.0 * sizeof(T)) * prep[q].num_pos + 3.0 * sizeof(T) * prep[q].bandcells;
         };
@@ -332,6 +343,8 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         d.Dbar = (double *)(Dv + L.Dbar);
         d.cnt = (int *)(Dv + L.cnt);
         d.topM = (T *)(Dv + L.topM);
+        d.topE = top_ef ? (T *)(Dv + L.topE) : nullptr;
+        d.topF = top_ef ? (T *)(Dv + L.topF) : nullptr;
         d.bmacc = (double *)(Dv + L.bmacc);
         d.res = (double *)(Dv + L.res);
         d.rect = keep ? (T *)(Dv + L.rect) : nullptr;
@@ -361,10 +374,11 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     unsigned int *qhead = (unsigned int *)(Dv + S->off_ctrl);
     int *status = (int *)(Dv + S->off_ctrl + 4);
     int *abort_flag = (int *)(Dv + S->off_ctrl + 8);
+    unsigned int *topq = (unsigned int *)(Dv + S->off_ctrl + 12);
     PF_TRY(cudaEventRecord(e->ev0, st));
-    PF_TRY(pf_launch_fwd<T>(Dv + S->off_pairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
-                            S->d_scratch, stride, sw, rb, qhead, status, abort_flag, e->sms * bf, true, st,
-                            keep ? rect_states : 0));
+    PF_TRY(pf_launch_fwd<T>(Dv + S->off_pairs, npairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
+                            S->d_scratch, stride, sw, rb, qhead, topq, status, abort_flag, e->sms * bf, st,
+                            keep ? rect_states : 0, top_ef));
     PF_TRY(cudaEventRecord(e->ev1, st));
     PF_TRY(cudaMemcpyAsync(H + S->off_ctrl, Dv + S->off_ctrl, 64, cudaMemcpyDeviceToHost, st));
     for (int q = 0; q < npairs; ++q)
@@ -406,10 +420,11 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
     unsigned int *qhead = (unsigned int *)(Dv + S->off_ctrl);
     int *status = (int *)(Dv + S->off_ctrl + 4);
     int *abort_flag = (int *)(Dv + S->off_ctrl + 8);
+    unsigned int *topq = (unsigned int *)(Dv + S->off_ctrl + 12);
     PF_TRY(cudaEventRecord(e->ev1, st));
-    PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
-                             S->d_scratch, S->stride, S->sw, S->rb, qhead, status, abort_flag, e->sms * bb, st, 0.0,
-                             S->gap_gradients));
+    PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, S->npairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
+                             S->d_scratch, S->stride, S->sw, S->rb, qhead, topq, status, abort_flag, e->sms * bb, st,
+                             0.0, S->gap_gradients));
     PF_TRY(cudaEventRecord(e->ev2, st));
     PF_TRY(cudaMemcpyAsync(H + S->off_ctrl, Dv + S->off_ctrl, 64, cudaMemcpyDeviceToHost, st));
     PF_TRY(cudaMemcpyAsync(H + S->out_begin, Dv + S->out_begin, S->out_end - S->out_begin, cudaMemcpyDeviceToHost, st));
@@ -483,9 +498,9 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
         for (int q = 0; q < S->npairs; ++q)
             PF_TRY(cudaMemsetAsync(Dv + S->lay[q].bmacc, 0, sizeof(double) * std::max(S->lay[q].bandcells, 1), st));
         PF_TRY(cudaMemsetAsync(Dv + S->off_ctrl, 0, 64, st));
-        PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
-                                 S->d_scratch, S->stride, S->sw, S->rb, qhead, status, abort_flag, e->sms * bb, st,
-                                 std::sqrt(S->min_am_prob)));
+        PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, S->npairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
+                                 S->d_scratch, S->stride, S->sw, S->rb, qhead, topq, status, abort_flag, e->sms * bb,
+                                 st, std::sqrt(S->min_am_prob)));
         PF_TRY(cudaEventRecord(e->ev2, st));
         for (int q = 0; q < S->npairs; ++q)
             PF_TRY(cudaMemcpyAsync(H + S->lay[q].bmacc, Dv + S->lay[q].bmacc,

@@ -28,10 +28,12 @@ struct PFPair {
     T *D;                  // NOT_READY pattern until written
     double *Dbar;          // dZ'/dD (backward), accumulated in FP64
     int *cnt;              // number of uses still to be back-propagated
-    T *topM;               // (n+1)(m+1)
+    // the top level, (n+1)(m+1) each, with zeros around the band: M, and E and F
+    // (nullptr: not kept; only the gap gradients read them)
+    T *topM, *topE, *topF;
     double *bmacc;         // per band cell (row offset rowinfo.w): sum of X_bar M(i-1,j-1) bm, FP64
     double *res;           // [0] log Z', [1] gap-extension uses, [2] gap-opening uses
-    const GroupItem *groups;  // left-end groups (work items) in dependency order, top level last
+    const GroupItem *groups;  // left-end groups (work items) in dependency order (then the top level)
     const int4 *dw;           // D writes: (D index, ar-1, br-1, -), by group, ar ascending
     // Kept group rectangles (nullptr: the backward recomputes them): the
     // forward writes group g's M (rect_states 1) or M, E, F (3; the gap
@@ -42,21 +44,20 @@ struct PFPair {
     int rect_states;
 };
 
-
-
+// queue: (pair, group) work items in dependency-respecting order, the top
+// levels apart (topq counts those taken); keep_states: 0, or the pairs'
+// PFPair::rect_states (rectangles kept); top_ef: PFPair::topE and topF are set
 template <typename T>
-// queue: (pair, group) work items in dependency-respecting order;
-// keep_states: 0, or the pairs' PFPair::rect_states (rectangles kept)
-cudaError_t pf_launch_fwd(const void *pairs, const int2 *queue, int nitems, void *scratch,
-                          long long stride, int pitch, int rb, unsigned int *qhead, int *status, int *abort_flag,
-                          int blocks, bool count_uses, cudaStream_t st, int keep_states = 0);
+cudaError_t pf_launch_fwd(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
+                          long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq, int *status,
+                          int *abort_flag, int blocks, cudaStream_t st, int keep_states, bool top_ef);
 // theta > 0: the truncated base-match pass (min_am_prob = theta^2) after a
 // full backward pass; theta = 0: the full adjoint pass, with the gap counts
 // (the indel / indel-opening gradients) when grads
 template <typename T>
-cudaError_t pf_launch_back(const void *pairs, const int2 *queue, int nitems, void *scratch,
-                           long long stride, int pitch, int rb, unsigned int *qhead, int *status, int *abort_flag,
-                           int blocks, cudaStream_t st, double theta = 0.0, bool grads = true);
+cudaError_t pf_launch_back(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
+                           long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq, int *status,
+                           int *abort_flag, int blocks, cudaStream_t st, double theta = 0.0, bool grads = true);
 // rb: ring size of the shared-memory rows (a power of two above the span of
 // any two consecutive band rows)
 template <typename T>

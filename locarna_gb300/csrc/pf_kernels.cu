@@ -370,13 +370,176 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
 #undef RG
 }
 
+// ---- top levels: a whole block per pair
+//
+// A pair's top level is the last to finish in the forward pass and the first to
+// go in the backward, where every group waits for it; it is the widest sweep
+// and has the longest entry lists. By one warp a row of a 200-nt pair took 6.5 us
+// forward and 13 us backward, 4.0 of the backward's 4.7 ms. A block spreads the
+// row's columns and entries over its threads, and the backward reads what the
+// forward kept: backward 4.7 -> 3.6 ms (top level 4.0 -> 1.6), forward 2.1 -> 1.9
+// (the top level now after the groups, 1.2 ms); the truncated pass over ten pairs
+// of 80-240 nt, which is little else, 2.1 -> 0.9. A row costs 6 to 8 us still:
+// some 20 FP64 operations a column at 2 a clock per SM, L2 latency of M_bar and
+// of the entries, and the fence before the counters. Scans with constant
+// factors, entries loaded a row ahead and longer naps of the waiting warps
+// changed nothing.
+
+// The recurrence x -> a x + b over the block's threads, in thread order, from
+// the value c before the first one (the same in all threads): c becomes the
+// value after the last thread, the result is the value before this thread and
+// *own the one after it. sm: 2 PF_WARPS values, not the ones of the last call.
+template <typename T>
+__device__ __forceinline__ T pf_block_scan(T a, T b, T &c, T *own, T *sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const T a1 = __shfl_up_sync(0xffffffffu, a, off);
+        const T b1 = __shfl_up_sync(0xffffffffu, b, off);
+        if (lane >= off) {
+            b = a * b1 + b;
+            a = a * a1;
+        }
+    }
+    if (lane == 31) {
+        sm[2 * warp] = a;
+        sm[2 * warp + 1] = b;
+    }
+    __syncthreads();
+    T before = c;
+#pragma unroll
+    for (int w = 0; w < PF_WARPS; ++w) {
+        if (w == warp) before = c;
+        c = sm[2 * w] * c + sm[2 * w + 1];
+    }
+    *own = a * before + b;
+    const T left = __shfl_up_sync(0xffffffffu, *own, 1);
+    return lane == 0 ? before : left;
+}
+
+// The forward sweep of a pair's top level (pf_group_sweep<SAVE> over all rows
+// and columns) by a block: M to P.topM, with EF also E and F to Eg and Fg.
+template <typename T, bool WAIT, bool COUNTU, bool EF>
+__device__ __noinline__ void pf_top_sweep(const PFPair<T> &P, T *__restrict__ Eg, T *__restrict__ Fg, PFRows<T> R, T (*sm)[2 * PF_WARPS],
+                             int *status, volatile int *abort_flag) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    constexpr int NT = PF_WARPS * 32;
+    const int n = P.n, m = P.m, pitch = m + 1;
+    const T o = P.o, arcf = P.arcf;
+    T *const Mg = P.topM;
+#define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
+    for (int c = tid; c < R.rb; c += NT) R.E[c] = R.Ar[c] = T(0);
+    auto put = [&](size_t at, T M, T E, T F) {
+        Mg[at] = M;
+        if (EF) {
+            Eg[at] = E;
+            Fg[at] = F;
+        }
+    };
+    int bf = 0;
+    {
+        // row 0: M(0,0) = 1/s, M(0,j) = (o/s) prod gB
+        const int L0 = P.rowinfo[0].y + 1;
+        T c = o * P.inv_s;
+        for (int base = 1; base < L0; base += NT, bf ^= 1) {
+            const int j = base + tid;
+            T v;
+            pf_block_scan<T>(j < L0 ? P.gB[j] : T(1), T(0), c, &v, sm[bf]);
+            if (j < L0) {
+                R.Mp[RG(j)] = R.Np[RG(j)] = v;
+                put(j, v, T(0), T(0));
+            }
+        }
+        if (tid == 0) {
+            R.Mp[0] = R.Np[0] = P.inv_s;
+            put(0, P.inv_s, T(0), T(0));
+        }
+        for (int j = L0 + tid; j <= P.rowinfo[1].y; j += NT) {
+            R.Mp[RG(j)] = R.Np[RG(j)] = T(0);
+            put(j, T(0), T(0), T(0));
+        }
+    }
+    T colval = o * P.inv_s;
+    for (int i = 1; i <= n; ++i) {
+        __syncthreads();  // the row above, its entry sums cleared
+        const int4 ri = P.rowinfo[i];
+        const int2 ra = P.rowarc[i];
+        const int lo = max(1, ri.x), hi = ri.y;
+        const T gAi = P.gA[i], gAo = gAi * o;
+        const size_t row = (size_t)i * pitch;
+        for (int e = ra.x + tid; e < ra.y; e += NT) {
+            const int2 en = P.crow[e];
+            if (en.y < lo || en.y > hi) continue;
+            T dv = pf_ld(P.D + e);
+            const T mv = Mg[(size_t)(en.x & 0xffff) * pitch + (en.x >> 16)];
+            if (WAIT && pf_not_ready(dv)) dv = pf_wait(P.D + e, status, abort_flag);
+            atomicAdd(&R.Ar[RG(en.y)], mv * dv);
+            if (COUNTU) atomicAdd(P.cnt + e, 1);
+        }
+        T B = T(0);
+        if (ri.x <= 0) B = colval *= gAi;
+        if (tid == 0) {
+            R.Mc[RG(lo - 1)] = R.Nc[RG(lo - 1)] = B;
+            put(row + lo - 1, B, T(0), T(0));
+        }
+        __syncthreads();
+        // F(j+1) = gB(j+1) (F(j) + o Q(j)): the value before thread j is F(j)
+        T Fc = P.gB[min(lo, m)] * o * B;
+        for (int base = lo; base <= hi; base += NT, bf ^= 1) {
+            const int j = base + tid;
+            const bool act = j <= hi;
+            T X = T(0), Ei = T(0), a = T(1), b = T(0), own;
+            if (act) {
+                Ei = R.E[RG(j)] * gAi + R.Np[RG(j)] * gAo;
+                X = R.Mp[RG(j - 1)] * P.bm[row + j];
+                if (ra.x < ra.y) {
+                    X += R.Ar[RG(j)] * arcf;
+                    R.Ar[RG(j)] = T(0);
+                }
+                a = j < m ? P.gB[j + 1] : T(0);
+                b = a * o * (X + Ei);
+            }
+            const T F = pf_block_scan<T>(a, b, Fc, &own, sm[bf]);
+            if (act) {
+                const T N = X + F, M = N + Ei;
+                R.E[RG(j)] = Ei;
+                R.Mc[RG(j)] = M;
+                R.Nc[RG(j)] = N;
+                put(row + j, M, Ei, F);
+            }
+        }
+        if (i < n)
+            // columns entering the band with row i+1 start from zero
+            for (int j = max(hi + 1, 1) + tid; j <= P.rowinfo[i + 1].y; j += NT) {
+                R.Mc[RG(j)] = R.Nc[RG(j)] = R.E[RG(j)] = T(0);
+                put(row + j, T(0), T(0), T(0));
+            }
+        T *t;
+        t = R.Mp; R.Mp = R.Mc; R.Mc = t;
+        t = R.Np; R.Np = R.Nc; R.Nc = t;
+    }
+    __syncthreads();
+#undef RG
+}
+
+// the next pair whose top level this block takes (npairs: none left)
+__device__ __forceinline__ int pf_next_top(unsigned int *topq, int npairs, volatile int *abort_flag) {
+    __shared__ int next;
+    __syncthreads();
+    if (threadIdx.x == 0) next = *abort_flag ? npairs : min((int)atomicAdd(topq, 1u), npairs);
+    __syncthreads();
+    return next;
+}
+
 // KEEP: 0, or the pairs' rect_states (the groups' rectangles are kept for
-// the backward pass, M alone or M, E and F)
-template <typename T, bool COUNTU, int KEEP = 0>
+// the backward pass, M alone or M, E and F); EF: E and F of the top levels too.
+// The groups go warp by warp, then the top levels block by block: a top level
+// waits for groups, all of which have been taken by then.
+template <typename T, int KEEP, bool EF>
 __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
-    pf_fwd_kernel(const PFPair<T> *__restrict__ pairs, const int2 *__restrict__ queue, int nitems,
+    pf_fwd_kernel(const PFPair<T> *__restrict__ pairs, int npairs, const int2 *__restrict__ queue, int nitems,
                   T *scratch, long long stride, int pitch, int rb,
-                  unsigned int *qhead, int *status, int *abort_ptr) {
+                  unsigned int *qhead, unsigned int *topq, int *status, int *abort_ptr) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     PFRows<T> R = pf_rows<T>(warp, rb);
     T *Mg = scratch + ((long long)blockIdx.x * PF_WARPS + warp) * stride;
@@ -389,27 +552,24 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
         const int2 qi = queue[idx];  // (pair, group)
         const PFPair<T> &P = pairs[qi.x];
         const GroupItem it = P.groups[qi.y];
-        if (it.top) {
-            pf_group_sweep<T, true, false, COUNTU, false>(P, 0, P.n + 1, 0, P.m + 1, P.topM, nullptr, nullptr,
-                                                          P.m + 1, R, nullptr, 0, status, abort_flag);
-            __syncwarp();
-            if (lane == 0) {
-                const T z = P.topM[(size_t)P.n * (P.m + 1) + P.m];
-                P.res[0] = log((double)z);
-            }
-        } else if (KEEP > 0 && P.rect && it.rect_off >= 0) {
+        if (KEEP > 0 && P.rect && it.rect_off >= 0) {
             const int w = it.br - it.bl;
             const size_t sz = (size_t)(it.ar - it.al) * w;
             T *Mk = P.rect + (size_t)KEEP * it.rect_off;
-            pf_group_sweep<T, true, true, COUNTU, true, KEEP == 3>(P, it.al, it.ar, it.bl, it.br, Mk, Mk + sz,
-                                                                   Mk + 2 * sz, w, R, P.dw + it.dw_start,
-                                                                   it.dw_count, status, abort_flag);
+            pf_group_sweep<T, true, true, true, true, KEEP == 3>(P, it.al, it.ar, it.bl, it.br, Mk, Mk + sz,
+                                                                 Mk + 2 * sz, w, R, P.dw + it.dw_start, it.dw_count,
+                                                                 status, abort_flag);
         } else {
-            pf_group_sweep<T, true, true, COUNTU, false>(P, it.al, it.ar, it.bl, it.br, Mg, nullptr, nullptr,
-                                                         pitch, R, P.dw + it.dw_start, it.dw_count, status,
-                                                         abort_flag);
+            pf_group_sweep<T, true, true, true, false>(P, it.al, it.ar, it.bl, it.br, Mg, nullptr, nullptr, pitch, R,
+                                                       P.dw + it.dw_start, it.dw_count, status, abort_flag);
         }
         __syncwarp();
+    }
+    __shared__ T sm[2][2 * PF_WARPS];
+    for (int q; (q = pf_next_top(topq, npairs, abort_flag)) < npairs;) {
+        const PFPair<T> &P = pairs[q];
+        pf_top_sweep<T, true, true, EF>(P, P.topE, P.topF, pf_rows<T>(0, rb), sm, status, abort_flag);
+        if (threadIdx.x == 0) P.res[0] = log((double)P.topM[(size_t)P.n * (P.m + 1) + P.m]);
     }
 }
 
@@ -422,8 +582,7 @@ __device__ __forceinline__ T ld_cg(const T *p) { return __ldcg(p); }
 // them or as pf_group_sweep<SAVE> recomputed them. Mb (same layout as Mg)
 // accumulates dZ'/dM for every cell of the rectangle, boundaries included.
 // Seeds: the group's own D
-// entries (dZ'/dD(am) w(am) into M(ar-1,br-1)) or, for the top level,
-// dZ'/dM(n,m) = 1. Propagates into D_bar of nested arc matches, the per-pair
+// entries (dZ'/dD(am) w(am) into M(ar-1,br-1)). Propagates into D_bar of nested arc matches, the per-pair
 // base-match accumulator and the gap counts. Rows bottom-up, chunks right to
 // left; E_bar of the row below lives in the E ring, the row's X_bar in Ar.
 // TRUNC: the base-match sums of compute_basematch_probabilities with a
@@ -434,7 +593,7 @@ __device__ __forceinline__ T ld_cg(const T *p) { return __ldcg(p); }
 // gap counts (ext_acc / open_acc) are accumulated, which reads E and F;
 // without, only M of the recomputed rectangle is read.
 template <typename T, bool TRUNC = false, bool GRADS = true>
-__device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br, bool top,
+__device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br,
                               const T *__restrict__ Mg, const T *__restrict__ Eg, const T *__restrict__ Fg,
                               T *__restrict__ Mb, int pitch, PFRows<T> R, const int4 *__restrict__ dw, int ndw,
                               int *status, volatile int *abort_flag, double *ext_acc, double *open_acc,
@@ -467,8 +626,6 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
         Dn[c] = T(0);
         Dc[c] = T(0);
     }
-    __syncwarp();
-    if (top && lane == 0) Mb[(size_t)(P.n - al) * pitch + (P.m - bl)] = T(1);
     __syncwarp();
     double ext = 0.0, opn = 0.0;
     int dwp = ndw - 1;  // D entries by ar descending
@@ -714,16 +871,164 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
     }
 }
 
+// pf_group_back of a pair's top level, by a block: dZ'/dM(n,m) = 1 is the
+// seed, all entries of a row are inside, and the row's columns go to the threads
+// from right to left. Mg, Eg, Fg as pf_top_sweep wrote them.
+template <typename T, bool TRUNC, bool GRADS>
+__device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict__ Mg, const T *__restrict__ Eg,
+                            const T *__restrict__ Fg, T *__restrict__ Mb, PFRows<T> R, T (*sm)[2 * PF_WARPS],
+                            double *ext_acc, double *open_acc) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NT = PF_WARPS * 32;
+    const int n = P.n, m = P.m, pitch = m + 1;
+    const T o = P.o, arcf = P.arcf;
+    T *const Eb = R.E, *const Xb = R.Ar;
+    T *Dn = R.Mp, *Dc = R.Mc;  // diagonal contributions, as in pf_group_back
+#define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
+    for (int i = warp; i <= n; i += PF_WARPS) {
+        const int hi = max(P.rowinfo[i].y, i < n ? P.rowinfo[i + 1].y : 0);
+        for (int j = max(0, P.rowinfo[i].x - 1) + lane; j <= hi; j += 32) Mb[(size_t)i * pitch + j] = T(0);
+        if (lane == 0) Mb[(size_t)i * pitch] = T(0);
+    }
+    for (int c = tid; c < R.rb; c += NT) Eb[c] = Dn[c] = Dc[c] = T(0);
+    __syncthreads();
+    if (tid == 0) Mb[(size_t)n * pitch + m] = T(1);
+    double ext = 0.0, opn = 0.0;
+    int bf = 0;
+    for (int i = n; i > 0; --i) {
+        __syncthreads();  // M_bar and the rings as row i+1 left them
+        const int4 ri = P.rowinfo[i], rup = P.rowinfo[i - 1];
+        const int2 ra = P.rowarc[i];
+        const int lo = max(1, ri.x), hi = ri.y;
+        const T gAi = P.gA[i], gAn = i < n ? P.gA[i + 1] : T(0);
+        const T gAo = gAi * o, gAno = gAn * o;
+        const size_t row = (size_t)i * pitch;
+        const int cb = ri.w - ri.x;
+        const int dlo = i > 1 ? max(1, rup.x) : INT_MAX, dhi = rup.y;
+        // the thread's first entry, loaded ahead of the cells
+        const int e0 = ra.x + tid;
+        int2 en = make_int2(0, 0);
+        T dv = T(0), mv = T(0);
+        if (e0 < ra.y) {
+            en = P.crow[e0];
+            dv = P.D[e0];
+            mv = Mg[(size_t)(en.x & 0xffff) * pitch + (en.x >> 16)];
+        }
+        T Fbc = T(0);
+        T opnE = T(0);
+        for (int top = hi; top >= lo; top -= NT, bf ^= 1) {
+            const int j = top - tid;
+            const bool act = j >= lo;
+            const size_t c = row + j;
+            T Mbar = T(0), Ebn = T(0), gn = T(0), bmj = T(0), Md = T(0), own;
+            if (act) {
+                Mbar = ld_cg(Mb + c) + Dc[RG(j)];
+                Dc[RG(j)] = T(0);
+                Ebn = Eb[RG(j)];
+                gn = j < hi ? P.gB[j + 1] : T(0);
+                bmj = P.bm[c];
+                Md = Mg[c - pitch - 1];
+            }
+            const T MN = Mbar + Ebn * gAno;
+            // F_bar(j) = gB(j+1) F_bar(j+1) + (M_bar + N_bar)(j)
+            const T Fbr = pf_block_scan<T>(act ? gn : T(1), MN, Fbc, &own, sm[bf]);
+            const T Fb = own;
+            if (act) {
+                const T Qbar = Fbr * gn * o;
+                const T Ebar = Mbar + (Qbar + Ebn * gAn);
+                const T Xbar = MN + Qbar;
+                Eb[RG(j)] = Ebar;
+                Xb[RG(j)] = Xbar;
+                if (GRADS) {
+                    ext += (double)(Ebar * Eg[c] + Fb * Fg[c]);
+                    opnE += Ebar * (Mg[c - pitch] - Eg[c - pitch]);
+                    opn += (double)(Fb * (Mg[c - 1] - Fg[c - 1]) * (P.gB[j] * o));
+                }
+                const T Xd = Xbar * bmj;
+                if (j - 1 >= dlo && j - 1 <= dhi)
+                    Dn[RG(j - 1)] = Xd;
+                else
+                    atomicAdd(Mb + c - pitch - 1, Xd);
+                atomicAdd(P.bmacc + cb + j, (double)(Xd * Md));
+                if (i == 1 || rup.x > j || rup.y < j) atomicAdd(Mb + c - pitch, Ebar * gAo);
+                if (j == lo) atomicAdd(Mb + c - 1, Fb * (P.gB[j] * o));
+            }
+        }
+        if (GRADS) opn += (double)opnE * gAo;
+        __syncthreads();
+        for (int e = e0; e < ra.y; e += NT) {
+            if (e != e0) {
+                en = P.crow[e];
+                dv = P.D[e];
+                mv = Mg[(size_t)(en.x & 0xffff) * pitch + (en.x >> 16)];
+            }
+            if (en.y < lo || en.y > hi) continue;
+            const T xs = Xb[RG(en.y)] * arcf;
+            atomicAdd(Mb + (size_t)(en.x & 0xffff) * pitch + (en.x >> 16), xs * dv);
+            if (!TRUNC) atomicAdd(P.Dbar + e, (double)(xs * mv));
+        }
+        if (!TRUNC && e0 < ra.y) {
+            __threadfence();  // the D_bar updates are visible before the counters drop
+            for (int e = e0; e < ra.y; e += NT) {
+                const int j = e == e0 && ra.y - e0 <= NT ? en.y : P.crow[e].y;
+                if (j >= lo && j <= hi) atomicSub(P.cnt + e, 1);
+            }
+        }
+        // E_bar of row i at columns row i-1 has but row i does not is zero
+        if (i > 1)
+            for (int j = max(1, rup.x) + tid; j < lo; j += NT) Eb[RG(j)] = T(0);
+        T *const dt = Dn;
+        Dn = Dc;
+        Dc = dt;
+    }
+    __syncthreads();
+#undef RG
+    if (TRUNC || !GRADS) return;
+    for (int j = 1 + tid; j <= P.rowinfo[0].y; j += NT) {
+        const T v = ld_cg(Mb + j) * Mg[j];
+        ext += (double)v * j;
+        opn += (double)v;
+    }
+    for (int i = 1 + tid; i <= n; i += NT) {
+        if (P.rowinfo[i].x > 0) continue;
+        const T v = ld_cg(Mb + (size_t)i * pitch) * Mg[(size_t)i * pitch];
+        ext += (double)v * i;
+        opn += (double)v;
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        ext += __shfl_xor_sync(0xffffffffu, ext, off);
+        opn += __shfl_xor_sync(0xffffffffu, opn, off);
+    }
+    if (lane == 0) {
+        atomicAdd(ext_acc, ext);
+        atomicAdd(open_acc, opn);
+    }
+}
+
 template <typename T, bool TRUNC, bool GRADS>
 __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
-    pf_back_kernel(const PFPair<T> *__restrict__ pairs, const int2 *__restrict__ queue, int nitems,
+    pf_back_kernel(const PFPair<T> *__restrict__ pairs, int npairs, const int2 *__restrict__ queue, int nitems,
                    T *scratch, long long stride, int pitch, int rb,
-                   unsigned int *qhead, int *status, int *abort_ptr, double theta) {
+                   unsigned int *qhead, unsigned int *topq, int *status, int *abort_ptr, double theta) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int *abort_flag = abort_ptr;
+    // the top levels first: every group waits for its pair's
+    {
+        __shared__ T sm[2][2 * PF_WARPS];
+        T *const Eg = scratch + (long long)blockIdx.x * PF_WARPS * stride * 4, *const Fg = Eg + stride;
+        for (int q; (q = pf_next_top(topq, npairs, abort_flag)) < npairs;) {
+            const PFPair<T> &P = pairs[q];
+            const PFRows<T> R = pf_rows<T>(0, rb);
+            const bool again = GRADS && !P.topE;  // E and F not kept by the forward pass
+            if (again) pf_top_sweep<T, false, false, true>(P, Eg, Fg, R, sm, status, abort_flag);
+            pf_top_back<T, TRUNC, GRADS>(P, P.topM, again ? Eg : P.topE, again ? Fg : P.topF, Fg + stride, R, sm,
+                                         P.res + 1, P.res + 2);
+        }
+    }
     PFRows<T> R = pf_rows<T>(warp, rb);
     T *Mg = scratch + ((long long)blockIdx.x * PF_WARPS + warp) * stride * 4;
     T *Eg = Mg + stride, *Fg = Eg + stride, *Mb = Fg + stride;
-    volatile int *abort_flag = abort_ptr;
     while (true) {
         int idx = 0;
         if (lane == 0) idx = (int)atomicAdd(qhead, 1u);
@@ -733,12 +1038,11 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
         const int2 qi = queue[nitems - 1 - idx];
         const PFPair<T> &P = pairs[qi.x];
         const GroupItem it = P.groups[qi.y];
-        const int al = it.top ? 0 : it.al, ar = it.top ? P.n + 1 : it.ar;
-        const int bl = it.top ? 0 : it.bl, br = it.top ? P.m + 1 : it.br;
+        const int al = it.al, ar = it.ar, bl = it.bl, br = it.br;
         // TRUNC: theta Z' (scaled frame); a group none of whose arc matches
         // passes the threshold contributes nothing
         const double theta_z = TRUNC ? theta * exp(P.res[0]) : 0.0;
-        if (TRUNC && !it.top) {
+        if (TRUNC) {
             bool any = false;
             for (int k = lane; k < it.dw_count && !any; k += 32) {
                 const int pos = P.dw[it.dw_start + k].x;
@@ -750,7 +1054,7 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
         // into the warp's slot (the adjoint rectangle Mb takes the same pitch)
         const T *Mw = Mg, *Ew = Eg, *Fw = Fg;
         int pw = pitch;
-        if (!it.top && P.rect && it.rect_off >= 0 && (!GRADS || P.rect_states == 3)) {
+        if (P.rect && it.rect_off >= 0 && (!GRADS || P.rect_states == 3)) {
             pw = br - bl;
             const size_t sz = (size_t)(ar - al) * pw;
             Mw = P.rect + (size_t)P.rect_states * it.rect_off;
@@ -761,9 +1065,8 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
                                                                 0, status, abort_flag);
         }
         __syncwarp();
-        pf_group_back<T, TRUNC, GRADS>(P, al, ar, bl, br, it.top != 0, Mw, Ew, Fw, Mb, pw, R,
-                                it.top ? nullptr : P.dw + it.dw_start, it.top ? 0 : it.dw_count, status, abort_flag,
-                                P.res + 1, P.res + 2, theta_z);
+        pf_group_back<T, TRUNC, GRADS>(P, al, ar, bl, br, Mw, Ew, Fw, Mb, pw, R, P.dw + it.dw_start, it.dw_count,
+                                       status, abort_flag, P.res + 1, P.res + 2, theta_z);
         __syncwarp();
     }
 }
@@ -776,30 +1079,18 @@ static size_t pf_smem(int rb) {
 }
 
 template <typename T>
-cudaError_t pf_launch_fwd(const void *pairs, const int2 *queue, int nitems, void *scratch,
-                          long long stride, int pitch, int rb, unsigned int *qhead, int *status, int *abort_flag,
-                          int blocks, bool count_uses, cudaStream_t st, int keep_states) {
+cudaError_t pf_launch_fwd(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
+                          long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq, int *status,
+                          int *abort_flag, int blocks, cudaStream_t st, int keep_states, bool top_ef) {
     const size_t smem = pf_smem<T>(rb);
-    cudaError_t e;
-    if (count_uses && keep_states > 0) {
-        auto k = keep_states == 3 ? pf_fwd_kernel<T, true, 3> : pf_fwd_kernel<T, true, 1>;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k<<<blocks, PF_WARPS * 32, smem, st>>>((const PFPair<T> *)pairs, queue, nitems, (T *)scratch, stride, pitch,
-                                               rb, qhead, status, abort_flag);
-    } else if (count_uses) {
-        e = cudaFuncSetAttribute(pf_fwd_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        pf_fwd_kernel<T, true><<<blocks, PF_WARPS * 32, smem, st>>>(
-            (const PFPair<T> *)pairs, queue, nitems, (T *)scratch, stride, pitch, rb, qhead,
-            status, abort_flag);
-    } else {
-        e = cudaFuncSetAttribute(pf_fwd_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        pf_fwd_kernel<T, false><<<blocks, PF_WARPS * 32, smem, st>>>(
-            (const PFPair<T> *)pairs, queue, nitems, (T *)scratch, stride, pitch, rb, qhead,
-            status, abort_flag);
-    }
+    auto k = keep_states == 3   ? pf_fwd_kernel<T, 3, true>
+             : keep_states == 1 ? pf_fwd_kernel<T, 1, false>
+             : top_ef           ? pf_fwd_kernel<T, 0, true>
+                                : pf_fwd_kernel<T, 0, false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<blocks, PF_WARPS * 32, smem, st>>>((const PFPair<T> *)pairs, npairs, queue, nitems, (T *)scratch, stride,
+                                           pitch, rb, qhead, topq, status, abort_flag);
     return cudaGetLastError();
 }
 
@@ -825,38 +1116,39 @@ static cudaError_t pf_cap_blocks(K kernel, const char *var, size_t smem, int *bl
 template <typename T>
 cudaError_t pf_fwd_occupancy(int rb, int *blocks_per_sm) {
     const size_t smem = pf_smem<T>(rb);
-    cudaError_t e = cudaFuncSetAttribute(pf_fwd_kernel<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(pf_fwd_kernel<T, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pf_fwd_kernel<T, true>, PF_WARPS * 32, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pf_fwd_kernel<T, 0, true>, PF_WARPS * 32, smem);
     if (e != cudaSuccess) return e;
-    return pf_cap_blocks(pf_fwd_kernel<T, true>, "LCG_PF_FWD_BPS", smem, blocks_per_sm);
+    return pf_cap_blocks(pf_fwd_kernel<T, 0, true>, "LCG_PF_FWD_BPS", smem, blocks_per_sm);
 }
 
 template <typename T, bool TRUNC, bool GRADS>
-static cudaError_t pf_launch_back_k(const void *pairs, const int2 *queue, int nitems, void *scratch, long long stride,
-                                    int pitch, int rb, unsigned int *qhead, int *status, int *abort_flag, int blocks,
-                                    cudaStream_t st, double theta) {
+static cudaError_t pf_launch_back_k(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
+                                    long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq,
+                                    int *status, int *abort_flag, int blocks, cudaStream_t st, double theta) {
     const size_t smem = pf_smem<T>(rb);
     cudaError_t e = cudaFuncSetAttribute(pf_back_kernel<T, TRUNC, GRADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
     pf_back_kernel<T, TRUNC, GRADS><<<blocks, PF_WARPS * 32, smem, st>>>(
-        (const PFPair<T> *)pairs, queue, nitems, (T *)scratch, stride, pitch, rb, qhead, status, abort_flag, theta);
+        (const PFPair<T> *)pairs, npairs, queue, nitems, (T *)scratch, stride, pitch, rb, qhead, topq, status,
+        abort_flag, theta);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t pf_launch_back(const void *pairs, const int2 *queue, int nitems, void *scratch,
-                           long long stride, int pitch, int rb, unsigned int *qhead, int *status, int *abort_flag,
-                           int blocks, cudaStream_t st, double theta, bool grads) {
+cudaError_t pf_launch_back(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
+                           long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq, int *status,
+                           int *abort_flag, int blocks, cudaStream_t st, double theta, bool grads) {
     if (theta > 0.0)
-        return pf_launch_back_k<T, true, false>(pairs, queue, nitems, scratch, stride, pitch, rb, qhead, status,
-                                                abort_flag, blocks, st, theta);
+        return pf_launch_back_k<T, true, false>(pairs, npairs, queue, nitems, scratch, stride, pitch, rb, qhead, topq,
+                                             status, abort_flag, blocks, st, theta);
     if (grads)
-        return pf_launch_back_k<T, false, true>(pairs, queue, nitems, scratch, stride, pitch, rb, qhead, status,
-                                                abort_flag, blocks, st, 0.0);
-    return pf_launch_back_k<T, false, false>(pairs, queue, nitems, scratch, stride, pitch, rb, qhead, status,
-                                             abort_flag, blocks, st, 0.0);
+        return pf_launch_back_k<T, false, true>(pairs, npairs, queue, nitems, scratch, stride, pitch, rb, qhead, topq,
+                                             status, abort_flag, blocks, st, 0.0);
+    return pf_launch_back_k<T, false, false>(pairs, npairs, queue, nitems, scratch, stride, pitch, rb, qhead, topq,
+                                             status, abort_flag, blocks, st, 0.0);
 }
 
 template <typename T>
@@ -873,16 +1165,18 @@ cudaError_t pf_back_occupancy(int rb, int *blocks_per_sm) {
 
 int pf_warps_per_block() { return PF_WARPS; }
 
-template cudaError_t pf_launch_fwd<double>(const void *, const int2 *, int, void *, long long, int,
-                                           int, unsigned int *, int *, int *, int, bool, cudaStream_t, int);
-template cudaError_t pf_launch_fwd<float>(const void *, const int2 *, int, void *, long long, int,
-                                          int, unsigned int *, int *, int *, int, bool, cudaStream_t, int);
+template cudaError_t pf_launch_fwd<double>(const void *, int, const int2 *, int, void *, long long, int, int,
+                                           unsigned int *, unsigned int *, int *, int *, int, cudaStream_t, int, bool);
+template cudaError_t pf_launch_fwd<float>(const void *, int, const int2 *, int, void *, long long, int, int,
+                                          unsigned int *, unsigned int *, int *, int *, int, cudaStream_t, int, bool);
 template cudaError_t pf_fwd_occupancy<double>(int, int *);
 template cudaError_t pf_fwd_occupancy<float>(int, int *);
-template cudaError_t pf_launch_back<double>(const void *, const int2 *, int, void *, long long, int,
-                                            int, unsigned int *, int *, int *, int, cudaStream_t, double, bool);
-template cudaError_t pf_launch_back<float>(const void *, const int2 *, int, void *, long long, int,
-                                           int, unsigned int *, int *, int *, int, cudaStream_t, double, bool);
+template cudaError_t pf_launch_back<double>(const void *, int, const int2 *, int, void *, long long, int, int,
+                                            unsigned int *, unsigned int *, int *, int *, int, cudaStream_t, double,
+                                            bool);
+template cudaError_t pf_launch_back<float>(const void *, int, const int2 *, int, void *, long long, int, int,
+                                           unsigned int *, unsigned int *, int *, int *, int, cudaStream_t, double,
+                                           bool);
 template cudaError_t pf_back_occupancy<double>(int, int *);
 template cudaError_t pf_back_occupancy<float>(int, int *);
 
