@@ -28,7 +28,7 @@ GENCODE = "-gencode=arch=compute_103a,code=sm_103a"
 EXTRA_DEFS = os.environ.get("LCG_NVCC_DEFS", "").split()
 
 CUDA_SOURCES = ["engine.cu", "index_kernels.cu", "sankoff_kernels.cu", "sankoff_lane_kernels.cu", "sankoff_sl_kernels.cu", "noalloc.cu",
-                "pf_kernels.cu", "engine_pf.cu", "envelope.cu"]
+                "pf_kernels.cu", "pf_lane_kernels.cu", "engine_pf.cu", "envelope.cu"]
 PROBE_SOURCE = "microbench.cu"  # the measurement probe, a library of its own
 HOST_SOURCES = ["host_prep.cpp"]  # C++ host-only translation units
 

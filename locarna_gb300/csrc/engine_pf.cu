@@ -38,11 +38,15 @@ lcg_status pf_fail(lcg_status c, const std::string &m) {
         if (_e != cudaSuccess) return pf_fail(LCG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
     } while (0)
 
+// at most this much scratch for the slots of a lane-per-group launch
+constexpr long long PF_LANE_SCRATCH_BYTES = 24ll << 30;
+
 size_t up16(size_t x) { return (x + 15) / 16 * 16; }
 
 struct PFLayout {
     int n, m, na, npos, bandcells;  // npos: D entries (arc matches with a band cell as right ends)
     size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, w, D, Dbar, cnt, bmacc, res, topM, topE, topF, rect;
+    size_t litems, cre, blkrows, quad_start;  // lane per group
     double log_c_total;  // (n+m) log c
 };
 
@@ -65,6 +69,8 @@ struct PFState {
     double temperature = 300.0;
     double min_am_prob = 0.0;  // > 0: base-match probabilities truncated as AlignerP computes them
     bool gap_gradients = true;  // the backward pass accumulates the gap counts
+    bool lanes = false;  // the batch is swept lane per group (pf_lane_kernels.cu)
+    PFLaneScratch lane_scratch;
     std::vector<double> log_z;
     std::vector<std::vector<int>> am_pos;  // per pair: D position of each arc match
 };
@@ -118,6 +124,31 @@ double seq_log_pf(const lcg_pair_tables &t, const std::vector<double> &bm, const
     return logscale + std::log(std::max(Mp[m], 1e-300));
 }
 
+// Whether an FP32 batch is swept lane per group (pf_lane_kernels.cu). An
+// estimate of both times from the pairs' sizes, with lane_width's measures (cells
+// and the longest item's time, engine.cu); the constants are fits to forward and
+// backward together on a GB300: one warp per group 10 cells/ns and half the
+// longest item, lane per group 50 cells/ns and four times the longest, whose quads
+// go one after the other behind the waits for their uses. Single pairs stay with
+// one warp per group (200 nt: 3.4 ms against 9.2, 400 nt: 36 against 57), as do
+// 6 pairs of 100-180 nt (2.3 against 4.3); 66 pairs of 70-110 nt take 5.7 ms
+// instead of 6.2, 28 of 160-200 nt 14 instead of 26, 10 of 250-330 nt 36 instead of
+// 65 and 21 of 80-500 nt 72 instead of 152.
+bool pf_lanes(const lcg_pair_tables *pairs, int npairs, const lcg_pf_opts *o) {
+    if (o->gap_gradients) return false;  // the adjoint of the gap weights reads E and F
+    if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) >= 32;
+    double cells = 0, longest = 0;
+    for (int q = 0; q < npairs; ++q) {
+        const lcg_pair_tables &t = pairs[q];
+        if (t.len_a < 1 || !t.min_col || !t.max_col) return false;
+        double band = 0;
+        for (int i = 0; i <= t.len_a; ++i) band += t.max_col[i] - t.min_col[i] + 1;
+        cells += 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
+        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
+    }
+    return cells / 10 + 0.5 * longest > cells / 50 + 4 * longest;
+}
+
 template <typename T>
 lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, int npairs, const lcg_pf_opts *o,
                         const lcg_pf_grad_spec *specs, double *log_z) {
@@ -125,7 +156,19 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     const double pf_scale = o->pf_scale > 0 ? o->pf_scale : 1.0;
     lcg_align_opts ao{0, 0, 0, 0};
     std::vector<lcg_host::Prep> prep(npairs);
-    lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q]); });
+    bool lanes = sizeof(T) == 4 && pf_lanes(pairs, npairs, o);
+    lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], lanes ? 32 : 0); });
+    if (lanes) {
+        // all pairs or none: a pair whose band is too wide keeps the batch off it
+        bool all = true;
+        for (auto &p : prep) all = all && (p.code != LCG_OK || (p.flags & PF_LANES));
+        if (!all) {
+            lanes = false;
+            prep.assign(npairs, lcg_host::Prep());
+            lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q]); });
+        }
+    }
+    S->lanes = lanes;
     bool need_spec = false;
     for (int k = 2; k < 19; ++k) need_spec |= o->param_delta[k] != 0.0;
     if (need_spec && !specs) return pf_fail(LCG_ERR_ARG, "param_delta[2..18] needs grad specs");
@@ -145,7 +188,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     size_t nitems = 0;
     int sw = 0, rows_max = 1, span = 2;
     for (auto &p : prep) {
-        nitems += p.groups.size() - 1;  // the top levels apart
+        nitems += lanes ? p.litems.size() : p.groups.size() - 1;  // the top levels apart
         sw = std::max(sw, std::max(p.width_max + 1, p.m + 2));
         rows_max = std::max(rows_max, std::max(p.rows_max + 1, p.n + 1));
         // widest column range two consecutive band rows cover (plus the
@@ -169,6 +212,12 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         L.rowarc = take(up, 4ull * p.rowarc.size());
         L.groups = take(up, sizeof(GroupItem) * p.groups.size());
         L.dw = take(up, sizeof(int4) * std::max<size_t>(p.dw.size(), 1));
+        if (lanes) {
+            L.litems = take(up, sizeof(LaneItem) * std::max<size_t>(p.litems.size(), 1));
+            L.cre = take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
+            L.blkrows = take(up, sizeof(int4) * p.blkrows.size());
+            L.quad_start = take(up, 4ull * p.quad_start.size());
+        }
         L.bm = take(up, sizeof(T) * (p.n + 1) * (p.m + 1));
         L.gA = take(up, sizeof(T) * (p.n + 1));
         L.gB = take(up, sizeof(T) * (p.m + 1));
@@ -191,20 +240,23 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     // the gap gradients, E and F) to a rectangle of its own and the backward
     // reads them instead of recomputing the groups, when the pairs'
     // rectangles fit the engine's budget (lcg_engine_set_rect_budget) -
-    // single pairs and small batches. By default FP64 only: an FP32
-    // recomputation into the warp's slot, read back from L2, is faster than
-    // reading the kept rectangle from DRAM (200-nt pair: backward 3.37 ms
-    // recomputing, 3.60 ms kept; FP64 7.51 against 6.06 ms).
+    // single pairs and small batches. One warp per group: by default FP64
+    // only, as an FP32 recomputation into the warp's slot, read back from L2,
+    // is faster than reading the kept rectangle from DRAM (200-nt pair:
+    // backward 3.37 ms recomputing, 3.60 ms kept; FP64 7.51 against 6.06 ms).
+    // Lane per group: kept (21 pairs of 80-500 nt: 46 ms, recomputing 89).
     const int rect_states = o->gap_gradients ? 3 : 1;
     bool keep, top_ef;
     {
         const long long budget =
-            e->rect_budget >= 0 ? e->rect_budget : (sizeof(T) == 8 ? RECT_BUDGET_PLAIN : 0);
+            e->rect_budget >= 0 ? e->rect_budget
+                                : (lanes ? RECT_BUDGET_LANES : sizeof(T) == 8 ? RECT_BUDGET_PLAIN : 0);
         keep = budget > 0;
         long long cells = 0;
         for (auto &p : prep) {
-            if (p.rect_cells < 0) keep = false;
-            cells += p.rect_cells;
+            const long long c = lanes ? p.lane_lines : p.rect_cells;
+            if (c < 0) keep = false;
+            cells += lanes ? 32 * c : c;
         }
         keep = keep && (double)cells * rect_states * sizeof(T) <= (double)budget;
         // E and F of the top levels, for the gap gradients
@@ -219,15 +271,33 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
             L.topE = take(up, sizeof(T) * (L.n + 1) * (L.m + 1));
             L.topF = take(up, sizeof(T) * (L.n + 1) * (L.m + 1));
         }
-    for (int q = 0; q < npairs; ++q)
-        S->lay[q].rect = keep ? take(up, sizeof(T) * rect_states * std::max<long long>(prep[q].rect_cells, 1)) : 0;
-    const size_t total = up;
+    const size_t bare = up;
+    for (int q = 0; q < npairs; ++q) {
+        if (keep) {
+            up = (up + 255) / 256 * 256;  // whole lines
+            const long long cells = lanes ? 32 * prep[q].lane_lines : prep[q].rect_cells;
+            S->lay[q].rect = take(up, sizeof(T) * rect_states * std::max<long long>(cells, 1));
+        }
+    }
+    size_t total = up;
     if (total > S->cap) {
         if (S->d_arena) cudaFree(S->d_arena);
         S->d_arena = nullptr;
         S->cap = 0;
-        if (cudaMalloc(&S->d_arena, total + total / 4) != cudaSuccess) return pf_fail(LCG_ERR_NOMEM, "PF device arena allocation failed");
-        S->cap = total + total / 4;
+        // with room to grow, else without, else without the kept rectangles
+        for (size_t bytes : {total + total / 4, total, bare}) {
+            if (cudaMalloc(&S->d_arena, bytes) == cudaSuccess) {
+                S->cap = bytes;
+                break;
+            }
+            cudaGetLastError();
+            S->d_arena = nullptr;
+        }
+        if (!S->d_arena) return pf_fail(LCG_ERR_NOMEM, "PF device arena allocation failed");
+        if (S->cap < total) {
+            keep = false;
+            total = bare;
+        }
     }
     if (out_end > S->hcap) {
         if (S->h_stage) cudaFreeHost(S->h_stage);
@@ -248,16 +318,16 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         // against 8 MB ones: FP32 backward 335 -> 283 ms, FP64 841 -> 655 ms,
         // while the forward slows from 74 to 82 ms)
         std::vector<size_t> ng(npairs);
-        for (int q = 0; q < npairs; ++q) ng[q] = prep[q].groups.size() - 1;
+        for (int q = 0; q < npairs; ++q) ng[q] = lanes ? prep[q].litems.size() : prep[q].groups.size() - 1;
         auto bytes = [&](int q) {
             return (12.0 + 3.0 * sizeof(T)) * prep[q].num_pos + 3.0 * sizeof(T) * prep[q].bandcells;
         };
         auto pfor = [](int n, auto fn) { lcg_host::parallel_for(n, fn); };
-        lcg_host::queue_order(ng, bytes, (int2 *)(H + S->off_queue), pfor);
+        lcg_host::queue_order(ng, bytes, (int2 *)(H + S->off_queue), pfor, lanes ? 1e15 : 0.0);
         const char *v = std::getenv("LCG_PF_BACK_WAVE_MB");
         const double back_mb = v ? std::atof(v) : 256.0;
         lcg_host::queue_order(ng, bytes, (int2 *)(H + S->off_queue_back), pfor,
-                              (back_mb > 0 ? back_mb : 1e9) * 1048576.0);
+                              lanes ? 1e15 : (back_mb > 0 ? back_mb : 1e9) * 1048576.0);
     }
     std::memset(H + S->off_ctrl, 0, 64);
     // per pair: Boltzmann weights, scale factor and packed tables (disjoint
@@ -293,6 +363,12 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         std::memcpy(H + L0.groups, p.groups.data(), sizeof(GroupItem) * p.groups.size());
         if (!p.dw.empty()) std::memcpy(H + L0.dw, p.dw.data(), sizeof(int4) * p.dw.size());
         std::memcpy(H + L0.rowarc, p.rowarc.data(), 4ull * p.rowarc.size());
+        if (lanes) {
+            if (!p.litems.empty()) std::memcpy(H + L0.litems, p.litems.data(), sizeof(LaneItem) * p.litems.size());
+            if (!p.cre.empty()) std::memcpy(H + L0.cre, p.cre.data(), 4ull * p.cre.size());
+            std::memcpy(H + L0.blkrows, p.blkrows.data(), sizeof(int4) * p.blkrows.size());
+            std::memcpy(H + L0.quad_start, p.quad_start.data(), 4ull * p.quad_start.size());
+        }
         T *hbm = (T *)(H + L0.bm);
         for (size_t k = 0; k < bm.size(); ++k) hbm[k] = (T)(bm[k] / c2);
         T *hgA = (T *)(H + L0.gA);
@@ -349,25 +425,60 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         d.res = (double *)(Dv + L.res);
         d.rect = keep ? (T *)(Dv + L.rect) : nullptr;
         d.rect_states = rect_states;
+        if (lanes) {
+            d.litems = (const LaneItem *)(Dv + L0.litems);
+            d.cre = (const int4 *)(Dv + L0.cre);
+            d.blkrows = (const int4 *)(Dv + L0.blkrows);
+            d.quad_start = (const int *)(Dv + L0.quad_start);
+        }
     };
     lcg_host::parallel_for(npairs, pack);
     // scratch: forward one rectangle per warp, backward four
     int bf = 0, bb = 0;
     const int rb = lcg_host::ring_size(span);
-    PF_TRY(pf_fwd_occupancy<T>(rb, &bf));
-    PF_TRY(pf_back_occupancy<T>(rb, &bb));
-    if (bf < 1 || bb < 1) return pf_fail(LCG_ERR_UNSUPPORTED, "PF kernels do not fit on an SM");
     const long long stride = (long long)rows_max * sw;
-    const size_t fwd_slots = (size_t)e->sms * bf * pf_warps_per_block();
-    const size_t back_slots = (size_t)e->sms * bb * pf_warps_per_block() * 4;
-    const size_t need = std::max(fwd_slots, back_slots) * (size_t)stride * sizeof(T);
+    size_t need;
+    if (lanes) {
+        PF_TRY(pf_lane_occupancy(rb, &bf));
+        if (bf < 1) return pf_fail(LCG_ERR_UNSUPPORTED, "PF kernels do not fit on an SM");
+        long long slot = 0, rows = 0, top = 0;
+        for (auto &p : prep) {
+            slot = std::max(slot, 32 * p.lane_slot);
+            rows = std::max(rows, 64ll * (p.n + 8));
+            top = std::max(top, (long long)(p.n + 1) * (p.m + 1));
+        }
+        PFLaneScratch &s = S->lane_scratch;
+        s.slot = keep ? 0 : slot;
+        s.back_slot = slot;
+        s.warp = s.slot + s.back_slot + rows;
+        s.block = (std::max(pf_warps_per_block() * s.warp, top) + 31) / 32 * 32;
+        // no more blocks than items, and a bounded amount of scratch
+        const long long want = std::max<long long>(npairs, (long long)(nitems + pf_warps_per_block() - 1) / pf_warps_per_block());
+        s.blocks = (int)std::max(1ll, std::min({(long long)e->sms * bf, want, PF_LANE_SCRATCH_BYTES / 4 / s.block}));
+        need = (size_t)s.blocks * (size_t)s.block * sizeof(T);
+    } else {
+        PF_TRY(pf_fwd_occupancy<T>(rb, &bf));
+        PF_TRY(pf_back_occupancy<T>(rb, &bb));
+        if (bf < 1 || bb < 1) return pf_fail(LCG_ERR_UNSUPPORTED, "PF kernels do not fit on an SM");
+        const size_t fwd_slots = (size_t)e->sms * bf * pf_warps_per_block();
+        const size_t back_slots = (size_t)e->sms * bb * pf_warps_per_block() * 4;
+        need = std::max(fwd_slots, back_slots) * (size_t)stride * sizeof(T);
+    }
     if (need > S->scratch_cap) {
         if (S->d_scratch) cudaFree(S->d_scratch);
         S->d_scratch = nullptr;
         S->scratch_cap = 0;
-        if (cudaMalloc(&S->d_scratch, need) != cudaSuccess) return pf_fail(LCG_ERR_NOMEM, "PF scratch allocation failed");
+        // with little memory left, a lane launch takes fewer blocks
+        while (cudaMalloc(&S->d_scratch, need) != cudaSuccess) {
+            cudaGetLastError();
+            S->d_scratch = nullptr;
+            if (!lanes || S->lane_scratch.blocks <= 1) return pf_fail(LCG_ERR_NOMEM, "PF scratch allocation failed");
+            S->lane_scratch.blocks /= 2;
+            need = (size_t)S->lane_scratch.blocks * (size_t)S->lane_scratch.block * sizeof(T);
+        }
         S->scratch_cap = need;
     }
+    S->lane_scratch.base = S->d_scratch;
     cudaStream_t st = e->stream;
     PF_TRY(cudaMemcpyAsync(Dv, H, zero_begin, cudaMemcpyHostToDevice, st));
     PF_TRY(cudaMemsetAsync(Dv + zero_begin, 0, out_end - zero_begin, st));
@@ -376,9 +487,13 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     int *abort_flag = (int *)(Dv + S->off_ctrl + 8);
     unsigned int *topq = (unsigned int *)(Dv + S->off_ctrl + 12);
     PF_TRY(cudaEventRecord(e->ev0, st));
-    PF_TRY(pf_launch_fwd<T>(Dv + S->off_pairs, npairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
-                            S->d_scratch, stride, sw, rb, qhead, topq, status, abort_flag, e->sms * bf, st,
-                            keep ? rect_states : 0, top_ef));
+    if (lanes)
+        PF_TRY(pf_launch_lane_fwd(Dv + S->off_pairs, npairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
+                                  S->lane_scratch, rb, qhead, topq, status, abort_flag, st));
+    else
+        PF_TRY(pf_launch_fwd<T>(Dv + S->off_pairs, npairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
+                                S->d_scratch, stride, sw, rb, qhead, topq, status, abort_flag, e->sms * bf, st,
+                                keep ? rect_states : 0, top_ef));
     PF_TRY(cudaEventRecord(e->ev1, st));
     PF_TRY(cudaMemcpyAsync(H + S->off_ctrl, Dv + S->off_ctrl, 64, cudaMemcpyDeviceToHost, st));
     for (int q = 0; q < npairs; ++q)
@@ -415,16 +530,22 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
     char *H = S->h_stage, *Dv = S->d_arena;
     cudaStream_t st = e->stream;
     int bb = 0;
-    PF_TRY(pf_back_occupancy<T>(S->rb, &bb));
+    if (!S->lanes) PF_TRY(pf_back_occupancy<T>(S->rb, &bb));
     PF_TRY(cudaMemsetAsync(Dv + S->off_ctrl, 0, 64, st));
     unsigned int *qhead = (unsigned int *)(Dv + S->off_ctrl);
     int *status = (int *)(Dv + S->off_ctrl + 4);
     int *abort_flag = (int *)(Dv + S->off_ctrl + 8);
     unsigned int *topq = (unsigned int *)(Dv + S->off_ctrl + 12);
     PF_TRY(cudaEventRecord(e->ev1, st));
-    PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, S->npairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
-                             S->d_scratch, S->stride, S->sw, S->rb, qhead, topq, status, abort_flag, e->sms * bb, st,
-                             0.0, S->gap_gradients));
+    auto launch = [&](double theta) {
+        const int2 *const queue = (const int2 *)(Dv + S->off_queue_back);
+        if (S->lanes)
+            return pf_launch_lane_back(Dv + S->off_pairs, S->npairs, queue, (int)S->nitems, S->lane_scratch, S->rb, qhead,
+                                       topq, status, abort_flag, st, theta);
+        return pf_launch_back<T>(Dv + S->off_pairs, S->npairs, queue, (int)S->nitems, S->d_scratch, S->stride, S->sw,
+                                 S->rb, qhead, topq, status, abort_flag, e->sms * bb, st, theta, S->gap_gradients);
+    };
+    PF_TRY(launch(0.0));
     PF_TRY(cudaEventRecord(e->ev2, st));
     PF_TRY(cudaMemcpyAsync(H + S->off_ctrl, Dv + S->off_ctrl, 64, cudaMemcpyDeviceToHost, st));
     PF_TRY(cudaMemcpyAsync(H + S->out_begin, Dv + S->out_begin, S->out_end - S->out_begin, cudaMemcpyDeviceToHost, st));
@@ -498,9 +619,7 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
         for (int q = 0; q < S->npairs; ++q)
             PF_TRY(cudaMemsetAsync(Dv + S->lay[q].bmacc, 0, sizeof(double) * std::max(S->lay[q].bandcells, 1), st));
         PF_TRY(cudaMemsetAsync(Dv + S->off_ctrl, 0, 64, st));
-        PF_TRY(pf_launch_back<T>(Dv + S->off_pairs, S->npairs, (const int2 *)(Dv + S->off_queue_back), (int)S->nitems,
-                                 S->d_scratch, S->stride, S->sw, S->rb, qhead, topq, status, abort_flag, e->sms * bb,
-                                 st, std::sqrt(S->min_am_prob)));
+        PF_TRY(launch(std::sqrt(S->min_am_prob)));
         PF_TRY(cudaEventRecord(e->ev2, st));
         for (int q = 0; q < S->npairs; ++q)
             PF_TRY(cudaMemcpyAsync(H + S->lay[q].bmacc, Dv + S->lay[q].bmacc,

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "lcg_device.cuh"
+
 namespace lcg {
 
 // NOT_READY pattern of a D entry that a group has yet to write (a NaN that no
@@ -42,6 +44,21 @@ struct PFPair {
     // reads them instead of recomputing the group.
     T *rect;
     int rect_states;
+    // Pairs swept lane per group (FP32, pf_lane_kernels.cu): the work items and
+    // the entries by quad as in PairDev; dw is then ordered by column block and
+    // row, rect holds the items' kept storage (a line of 32 per band cell)
+    const LaneItem *litems;
+    const int4 *cre;
+    const int4 *blkrows;
+    const int *quad_start;
+};
+
+// Scratch of the lane-per-group launches, in floats: per block, in it per warp,
+// in that for M (0: kept) and, backward, for M_bar; then the vectors per row
+struct PFLaneScratch {
+    void *base = nullptr;
+    long long block = 0, warp = 0, slot = 0, back_slot = 0;
+    int blocks = 0;
 };
 
 // queue: (pair, group) work items in dependency-respecting order, the top
@@ -65,5 +82,13 @@ cudaError_t pf_fwd_occupancy(int rb, int *blocks_per_sm);
 template <typename T>
 cudaError_t pf_back_occupancy(int rb, int *blocks_per_sm);
 int pf_warps_per_block();
+
+cudaError_t pf_lane_occupancy(int rb, int *blocks_per_sm);
+cudaError_t pf_launch_lane_fwd(const void *pairs, int npairs, const int2 *queue, int nitems, const PFLaneScratch &s, int rb,
+                               unsigned int *qhead, unsigned int *topq, int *status, int *abort_flag, cudaStream_t st);
+// theta as for pf_launch_back
+cudaError_t pf_launch_lane_back(const void *pairs, int npairs, const int2 *queue, int nitems, const PFLaneScratch &s,
+                                int rb, unsigned int *qhead, unsigned int *topq, int *status, int *abort_flag,
+                                cudaStream_t st, double theta);
 
 }  // namespace lcg
