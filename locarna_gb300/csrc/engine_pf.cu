@@ -45,7 +45,7 @@ size_t up16(size_t x) { return (x + 15) / 16 * 16; }
 
 struct PFLayout {
     int n, m, na, npos, bandcells;  // npos: D entries (arc matches with a band cell as right ends)
-    size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, w, D, Dbar, cnt, bmacc, res, topM, topE, topF, rect;
+    size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, gpow, w, D, Dbar, cnt, bmacc, res, topM, topE, topF, rect;
     size_t litems, cre, blkrows, quad_start;  // lane per group
     double log_c_total;  // (n+m) log c
 };
@@ -221,6 +221,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         L.bm = take(up, sizeof(T) * (p.n + 1) * (p.m + 1));
         L.gA = take(up, sizeof(T) * (p.n + 1));
         L.gB = take(up, sizeof(T) * (p.m + 1));
+        L.gpow = take(up, sizeof(T) * 33);
         L.w = take(up, sizeof(T) * std::max(L.npos, 1));
         L.D = take(up, sizeof(T) * std::max(L.npos, 1));
     }
@@ -356,7 +357,18 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         const double ow = std::exp(((double)t.indel_opening + dl[1]) / temp);
         double logc = 0.0;
         if (sizeof(T) == 4) logc = seq_log_pf(t, bm, gA, gB, ow) / (double)(n + m);
-        const double c = std::exp(logc), c2 = c * c;
+        double c = std::exp(logc);
+        // the estimate moved so that the first gap weight over it is a float: the
+        // others mostly equal it, and a rounded weight's error adds up over the
+        // gaps of an alignment (80 against 439 nt: 360 of them)
+        if (sizeof(T) == 4) {
+            const double g = gB[1] / (double)(float)(gB[1] / c);
+            if (std::isfinite(g) && g > 0.0) {
+                c = g;
+                logc = std::log(c);
+            }
+        }
+        const double c2 = c * c;
         L.log_c_total = logc * (n + m);
         std::memcpy(H + L0.rowinfo, p.rowinfo.data(), 16ull * (n + 2));
         if (!p.crow.empty()) std::memcpy(H + L0.crow, p.crow.data(), 4ull * p.crow.size());
@@ -412,6 +424,9 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         d.gu = hgB[1];
         for (int j = 2; j <= m && d.gu > T(0); ++j)
             if (hgB[j] != hgB[1]) d.gu = T(0);
+        T *hgp = (T *)(H + L0.gpow);
+        for (int k = 0; k <= 32; ++k) hgp[k] = (T)std::pow((double)d.gu, k);
+        d.gpow = (const T *)(Dv + L0.gpow);
         d.inv_s = (T)(1.0 / pf_scale);
         d.arcf = (T)(pf_scale / (c2 * c2));
         d.w = (const T *)(Dv + L0.w);

@@ -23,6 +23,7 @@ struct PFPair {
     const T *gA, *gB;      // scaled gap weights
     T o;                   // gap-opening weight
     T gu;                  // the value of every gB[j], j >= 1, if they are all the same, else 0
+    const T *gpow;         // 33: its powers 0 to 32, each rounded once
     T inv_s;               // 1 / pf_scale
     T arcf;                // pf_scale / c^4
     // per D position (the arc match's position in crow):

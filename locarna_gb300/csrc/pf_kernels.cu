@@ -54,8 +54,8 @@ __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int b
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
     const bool uni = P.gu > T(0);
-    const PFPow<T> W = pf_pow(P.gu);
-    const T guo = P.gu * o, wl = pf_power(W, lane + 1);
+    const PFPow<T> W = pf_pow(P);
+    const T guo = P.gu * o, wl = P.gpow[lane + 1];
 #define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
     // E and the arc-term sums start at zero; the cell sweep puts zero back
     // into every arc-term column it reads, so no row needs a clearing pass
@@ -348,8 +348,8 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
     const bool uni = P.gu > T(0);
-    const PFPow<T> W = pf_pow(P.gu);
-    const T guo = P.gu * o, wr = pf_power(W, 32 - lane);
+    const PFPow<T> W = pf_pow(P);
+    const T guo = P.gu * o, wr = P.gpow[32 - lane];
     T *const Eb = R.E;
     T *const Xb = R.Ar;
     // diagonal adjoint contributions X_bar(i,j) bm(i,j) to M_bar(i-1,j-1):

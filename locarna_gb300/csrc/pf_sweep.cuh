@@ -44,31 +44,23 @@ __device__ __forceinline__ T pf_wait(const T *p, int *status, volatile int *abor
 }
 
 // The gap chains' factors of a pair whose columns all have the same gap weight
-// g (single sequences): g^1, 2, 4, 8, 16 for the warp scans and g^(lane+1),
-// g^(32-lane) for their carries. FP64 arithmetic is what bounds the FP64
+// g (single sequences): g^1, 2, 4, 8, 16 for the warp scans (the carries take
+// gpow[lane + 1] and gpow[32 - lane]). FP64 arithmetic is what bounds the FP64
 // passes (an SM issues two FP64 operations a clock), and the scan with constant
-// factors takes 5 multiply-adds a cell instead of 10.
+// factors takes 5 multiply-adds a cell instead of 10. The powers come rounded
+// once from the host: squared up here, g^16 was up to 15 roundings off, which the
+// sweeps of lanes and of rows did not share (80 against 439 nt in FP32: am_prob
+// 2.2e-6 off in norm).
 template <typename T>
 struct PFPow {
     T p[5];
 };
 template <typename T>
-__device__ __forceinline__ PFPow<T> pf_pow(T g) {
+__device__ __forceinline__ PFPow<T> pf_pow(const PFPair<T> &P) {
     PFPow<T> w;
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        w.p[k] = g;
-        g *= g;
-    }
+    for (int k = 0; k < 5; ++k) w.p[k] = P.gpow[1 << k];
     return w;
-}
-template <typename T>
-__device__ __forceinline__ T pf_power(const PFPow<T> &w, int n) {  // g^n, 1 <= n <= 32
-    T x = T(1);
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-        if (n >> k & 1) x *= w.p[k];
-    return n == 32 ? w.p[4] * w.p[4] : x;
 }
 
 extern __shared__ unsigned char pf_smem_raw[];
@@ -116,24 +108,34 @@ __device__ __forceinline__ T ld_cg(const T *p) { return __ldcg(p); }
 // (the top level now after the groups, 1.2 ms); the truncated pass over ten pairs
 // of 80-240 nt, which is little else, 2.1 -> 0.9. A row costs 6 to 8 us still:
 // some 20 FP64 operations a column at 2 a clock per SM, L2 latency of M_bar and
-// of the entries, and the fence before the counters. Scans with constant
-// factors, entries loaded a row ahead and longer naps of the waiting warps
-// changed nothing.
+// of the entries, and the fence before the counters. Entries
+// loaded a row ahead and longer naps of the waiting warps changed nothing.
 
 // The recurrence x -> a x + b over the block's threads, in thread order, from
 // the value c before the first one (the same in all threads): c becomes the
 // value after the last thread, the result is the value before this thread and
-// *own the one after it. sm: 2 PF_WARPS values, not the ones of the last call.
+// *own the one after it. W: the powers of a where all threads have the same a
+// (then pa = a^(lane + 1)), else nullptr. sm: 2 PF_WARPS values, not the ones of
+// the last call.
 template <typename T>
-__device__ __forceinline__ T pf_block_scan(T a, T b, T &c, T *own, T *sm) {
+__device__ __forceinline__ T pf_block_scan(T a, T b, const PFPow<T> *W, T pa, T &c, T *own, T *sm) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (W) {
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const T a1 = __shfl_up_sync(0xffffffffu, a, off);
-        const T b1 = __shfl_up_sync(0xffffffffu, b, off);
-        if (lane >= off) {
-            b = a * b1 + b;
-            a = a * a1;
+        for (int k = 0; k < 5; ++k) {
+            const T b1 = __shfl_up_sync(0xffffffffu, b, 1 << k);
+            if (lane >= 1 << k) b += W->p[k] * b1;
+        }
+        a = pa;
+    } else {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const T a1 = __shfl_up_sync(0xffffffffu, a, off);
+            const T b1 = __shfl_up_sync(0xffffffffu, b, off);
+            if (lane >= off) {
+                b = a * b1 + b;
+                a = a * a1;
+            }
         }
     }
     if (lane == 31) {
@@ -162,6 +164,9 @@ __device__ __noinline__ void pf_top_sweep(const PFPair<T> &P, T *__restrict__ Eg
     const int n = P.n, m = P.m, pitch = m + 1;
     const T o = P.o, arcf = P.arcf;
     T *const Mg = P.topM;
+    const bool uni = P.gu > T(0);
+    const PFPow<T> W = pf_pow(P);
+    const T pa = P.gpow[(tid & 31) + 1];
 #define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
     for (int c = tid; c < R.rb; c += NT) R.E[c] = R.Ar[c] = T(0);
     auto put = [&](size_t at, T M, T E, T F) {
@@ -179,7 +184,7 @@ __device__ __noinline__ void pf_top_sweep(const PFPair<T> &P, T *__restrict__ Eg
         for (int base = 1; base < L0; base += NT, bf ^= 1) {
             const int j = base + tid;
             T v;
-            pf_block_scan<T>(j < L0 ? P.gB[j] : T(1), T(0), c, &v, sm[bf]);
+            pf_block_scan<T>(j < L0 ? P.gB[j] : T(1), T(0), uni ? &W : nullptr, pa, c, &v, sm[bf]);
             if (j < L0) {
                 R.Mp[RG(j)] = R.Np[RG(j)] = v;
                 put(j, v, T(0), T(0));
@@ -231,10 +236,10 @@ __device__ __noinline__ void pf_top_sweep(const PFPair<T> &P, T *__restrict__ Eg
                     X += R.Ar[RG(j)] * arcf;
                     R.Ar[RG(j)] = T(0);
                 }
-                a = j < m ? P.gB[j + 1] : T(0);
+                a = uni ? P.gu : j < m ? P.gB[j + 1] : T(0);
                 b = a * o * (X + Ei);
             }
-            const T F = pf_block_scan<T>(a, b, Fc, &own, sm[bf]);
+            const T F = pf_block_scan<T>(a, b, uni ? &W : nullptr, pa, Fc, &own, sm[bf]);
             if (act) {
                 const T N = X + F, M = N + Ei;
                 R.E[RG(j)] = Ei;
@@ -279,6 +284,9 @@ __device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict
     const T o = P.o, arcf = P.arcf;
     T *const Eb = R.E, *const Xb = R.Ar;
     T *Dn = R.Mp, *Dc = R.Mc;  // diagonal contributions, as in pf_group_back
+    const bool uni = P.gu > T(0);
+    const PFPow<T> W = pf_pow(P);
+    const T pa = P.gpow[lane + 1];
 #define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
     for (int i = warp; i <= n; i += PF_WARPS) {
         const int hi = max(P.rowinfo[i].y, i < n ? P.rowinfo[i + 1].y : 0);
@@ -320,13 +328,13 @@ __device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict
                 Mbar = ld_cg(Mb + c) + Dc[RG(j)];
                 Dc[RG(j)] = T(0);
                 Ebn = Eb[RG(j)];
-                gn = j < hi ? P.gB[j + 1] : T(0);
+                gn = uni ? P.gu : j < hi ? P.gB[j + 1] : T(0);
                 bmj = P.bm[c];
                 Md = Mg[c - pitch - 1];
             }
             const T MN = Mbar + Ebn * gAno;
             // F_bar(j) = gB(j+1) F_bar(j+1) + (M_bar + N_bar)(j)
-            const T Fbr = pf_block_scan<T>(act ? gn : T(1), MN, Fbc, &own, sm[bf]);
+            const T Fbr = pf_block_scan<T>(act ? gn : T(1), MN, uni ? &W : nullptr, pa, Fbc, &own, sm[bf]);
             const T Fb = own;
             if (act) {
                 const T Qbar = Fbr * gn * o;
