@@ -701,6 +701,16 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
     return LCG_OK;
 }
 
+// Whether the device makes the index structures of a chunk: from 2,000 arc
+// matches on its two launches (10 us) cost less than the host's 30 ns per arc
+// match (one 60 x 60 pair: 500 arc matches, 15 us on the host).
+bool index_on_device(const lcg_pair_tables *pairs, int npairs) {
+    if (const char *v = std::getenv("LCG_DEVICE_INDEX")) return v[0] != '0';
+    long long am = 0;
+    for (int q = 0; q < npairs; ++q) am += std::max(pairs[q].num_arcmatches, 0);
+    return am >= 2000;
+}
+
 }  // namespace lcg_host
 
 namespace {
@@ -832,16 +842,6 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
     if (opts->no_lonely_pairs) cells /= 50;  // few arc matches have a stacked partner
     const double warp = cells / 80 + longest / 6, l32 = cells / 130 + 0.6 * longest, l64 = cells / 170 + 1.4 * longest;
     return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
-}
-
-// Whether the device makes the index structures of a chunk: from 2,000 arc
-// matches on its two launches (10 us) cost less than the host's 30 ns per arc
-// match (one 60 x 60 pair: 500 arc matches, 15 us on the host).
-bool index_on_device(const lcg_pair_tables *pairs, int npairs) {
-    if (const char *v = std::getenv("LCG_DEVICE_INDEX")) return v[0] != '0';
-    long long am = 0;
-    for (int q = 0; q < npairs; ++q) am += std::max(pairs[q].num_arcmatches, 0);
-    return am >= 2000;
 }
 
 // pairs per chunk: one chunk for small batches, else up to 8 chunks of at
@@ -1775,7 +1775,7 @@ static lcg_status align_impl(lcg_engine e, const lcg_pair_tables *pairs, int32_t
         next.clear();
         next.resize(nq);
         const int lanes = lane_width(e, pairs + q0, nq, opts);
-        const bool dev = index_on_device(pairs + q0, nq);
+        const bool dev = lcg_host::index_on_device(pairs + q0, nq);
         lcg_host::parallel_for(nq, [&](int q) { prep_pair(pairs[q0 + q], *opts, next[q], lanes, dev); });
         t_prep += ms_between(a, clk::now());
         for (int q = 0; q < nq && rc == LCG_OK; ++q)
@@ -1977,7 +1977,7 @@ lcg_status lcg_align_kbest(lcg_engine e, const lcg_pair_tables *pairs, int32_t n
     c.kbest = true;
     c.prep.resize(npairs);
     const int lanes = lane_width(e, pairs, npairs, opts);
-    const bool dev = index_on_device(pairs, npairs);
+    const bool dev = lcg_host::index_on_device(pairs, npairs);
     lcg_host::parallel_for(npairs, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q], lanes, dev); });
     for (int q = 0; q < npairs; ++q)
         if (c.prep[q].code != LCG_OK) return fail(c.prep[q].code, "pair " + std::to_string(q) + ": " + c.prep[q].err);

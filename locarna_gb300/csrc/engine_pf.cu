@@ -19,6 +19,7 @@
 #include "../../include/locarna_gb300.h"
 #include "engine_prep.hh"
 #include "engine_state.hh"
+#include "index_device.cuh"
 #include "lcg_device.cuh"
 #include "pf_device.cuh"
 
@@ -47,6 +48,9 @@ struct PFLayout {
     int n, m, na, npos, bandcells;  // npos: D entries (arc matches with a band cell as right ends)
     size_t rowinfo, crow, rowarc, groups, dw, bm, gA, gB, gpow, w, D, Dbar, cnt, bmacc, res, topM, topE, topF, rect;
     size_t litems, cre, blkrows, quad_start;  // lane per group
+    size_t am_score, am_dsw, am_pos, D0, am_prob;
+    // index structures made on the device (index_kernels.cu)
+    size_t min_col, max_col, cre_start, arcs4, lefts, row_start, row_arcs, am_lr, cursor, gcursor;
     double log_c_total;  // (n+m) log c
 };
 
@@ -60,7 +64,7 @@ struct PFState {
     char *d_scratch = nullptr;
     size_t scratch_cap = 0;
     std::vector<PFLayout> lay;
-    size_t off_pairs = 0, off_queue = 0, off_queue_back = 0, off_ctrl = 0, out_begin = 0, out_end = 0, total = 0;
+    size_t off_pairs = 0, off_queue = 0, off_queue_back = 0, off_ctrl = 0, off_am = 0, out_begin = 0, out_end = 0, total = 0;
     size_t nitems = 0;
     int sw = 0, rb = 0;
     long long stride = 0;
@@ -72,7 +76,8 @@ struct PFState {
     bool lanes = false;  // the batch is swept lane per group (pf_lane_kernels.cu)
     PFLaneScratch lane_scratch;
     std::vector<double> log_z;
-    std::vector<std::vector<int>> am_pos;  // per pair: D position of each arc match
+    std::vector<double> zs;  // per pair: Z in the scaled frame
+    int max_entries = 0;  // most arc matches or band cells of a pair
 };
 
 PFState *state_of(lcg_engine e) {
@@ -157,7 +162,8 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     lcg_align_opts ao{0, 0, 0, 0};
     std::vector<lcg_host::Prep> prep(npairs);
     bool lanes = sizeof(T) == 4 && pf_lanes(pairs, npairs, o);
-    lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], lanes ? 32 : 0); });
+    const bool dev = lcg_host::index_on_device(pairs, npairs);
+    lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], lanes ? 32 : 0, dev); });
     if (lanes) {
         // all pairs or none: a pair whose band is too wide keeps the batch off it
         bool all = true;
@@ -165,7 +171,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         if (!all) {
             lanes = false;
             prep.assign(npairs, lcg_host::Prep());
-            lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q]); });
+            lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], 0, dev); });
         }
     }
     S->lanes = lanes;
@@ -178,7 +184,6 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     }
     // layout
     S->lay.assign(npairs, PFLayout{});
-    S->am_pos.assign(npairs, std::vector<int>());
     size_t up = 0;
     auto take = [](size_t &cur, size_t bytes) {
         size_t r = cur;
@@ -199,6 +204,11 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     S->off_queue = take(up, sizeof(int2) * nitems);
     S->off_queue_back = take(up, sizeof(int2) * nitems);
     S->off_ctrl = take(up, 64);
+    S->off_am = take(up, sizeof(PFArcMatches) * npairs);
+    const size_t off_index = take(up, (sizeof(PairDev) + sizeof(IndexPair)) * npairs);
+    int index_n = 0, index_lefts = -1;  // -1: every pair's index is the host's
+    S->max_entries = 1;
+    std::vector<char> dsw(npairs);
     for (int q = 0; q < npairs; ++q) {
         const auto &p = prep[q];
         PFLayout &L = S->lay[q];
@@ -208,13 +218,32 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         L.npos = p.num_pos;
         L.bandcells = p.bandcells;
         L.rowinfo = take(up, 16ull * (p.n + 2));
-        L.crow = take(up, 4ull * std::max<size_t>(p.crow.size(), 4));
+        S->max_entries = std::max(S->max_entries, std::max(L.na, L.bandcells));
+        L.am_score = take(up, 4ull * std::max(L.na, 1));
+        dsw[q] = o->param_delta[2] != 0.0 && specs && specs[q].am_dscore_dsw;
+        if (dsw[q]) L.am_dsw = take(up, 8ull * std::max(L.na, 1));
+        if (p.device_index) {
+            index_n = std::max(index_n, p.n);
+            index_lefts = std::max(index_lefts, (int)p.lefts.size());
+            L.min_col = take(up, 4ull * (p.n + 2));
+            L.max_col = take(up, 4ull * (p.n + 2));
+            L.cre_start = take(up, 4ull * std::max<size_t>(p.cre_start.size(), 1));
+            L.arcs4 = take(up, 16ull * std::max<size_t>(p.arcs4.size(), 1));
+            L.lefts = take(up, 16ull * std::max<size_t>(p.lefts.size(), 1));
+            L.row_start = take(up, 4ull * p.row_start.size());
+            L.row_arcs = take(up, 4ull * std::max<size_t>(p.row_arcs.size(), 1));
+            L.am_lr = take(up, 4ull * std::max<size_t>(p.am_lr.size(), 1));
+        } else {
+            L.crow = take(up, 4ull * std::max<size_t>(p.crow.size(), 4));
+            L.dw = take(up, sizeof(int4) * std::max<size_t>(p.dw.size(), 1));
+            if (lanes) L.cre = take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
+            L.am_pos = take(up, 4ull * std::max<size_t>(p.am_pos.size(), 1));
+            L.D0 = take(up, 4ull * std::max(L.npos, 1));
+        }
         L.rowarc = take(up, 4ull * p.rowarc.size());
         L.groups = take(up, sizeof(GroupItem) * p.groups.size());
-        L.dw = take(up, sizeof(int4) * std::max<size_t>(p.dw.size(), 1));
         if (lanes) {
             L.litems = take(up, sizeof(LaneItem) * std::max<size_t>(p.litems.size(), 1));
-            L.cre = take(up, 4ull * std::max<size_t>(p.cre.size(), 4));
             L.blkrows = take(up, sizeof(int4) * p.blkrows.size());
             L.quad_start = take(up, 4ull * p.quad_start.size());
         }
@@ -222,20 +251,36 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         L.gA = take(up, sizeof(T) * (p.n + 1));
         L.gB = take(up, sizeof(T) * (p.m + 1));
         L.gpow = take(up, sizeof(T) * 33);
-        L.w = take(up, sizeof(T) * std::max(L.npos, 1));
-        L.D = take(up, sizeof(T) * std::max(L.npos, 1));
     }
-    // zero-initialised device section, then the output section
-    const size_t zero_begin = up;
-    for (int q = 0; q < npairs; ++q) S->lay[q].cnt = take(up, 4ull * std::max(S->lay[q].npos, 1));
-    const size_t out_begin = up;
+    // the output section, zero at first like the counters and D_bar behind it;
+    // then what only the device holds
+    const size_t zero_begin = up, out_begin = up;
     for (int q = 0; q < npairs; ++q) {
         PFLayout &L = S->lay[q];
         L.res = take(up, 8ull * 4);
-        L.Dbar = take(up, sizeof(double) * std::max(L.npos, 1));
         L.bmacc = take(up, sizeof(double) * std::max(L.bandcells, 1));
+        L.am_prob = take(up, sizeof(double) * std::max(L.na, 1));
     }
     const size_t out_end = up;
+    for (int q = 0; q < npairs; ++q) {
+        PFLayout &L = S->lay[q];
+        L.cnt = take(up, 4ull * std::max(L.npos, 1));
+        L.Dbar = take(up, sizeof(double) * std::max(L.npos, 1));
+    }
+    const size_t zero_end = up;
+    for (int q = 0; q < npairs; ++q) {
+        PFLayout &L = S->lay[q];
+        L.w = take(up, sizeof(T) * std::max(L.npos, 1));
+        L.D = take(up, sizeof(T) * std::max(L.npos, 1));
+        if (!prep[q].device_index) continue;
+        L.crow = take(up, 8ull * std::max(L.npos, 2));
+        L.cre = take(up, 16ull * std::max(L.npos, 1));
+        L.dw = take(up, sizeof(int4) * std::max(prep[q].num_dw, 1));
+        L.am_pos = take(up, 4ull * std::max(L.na, 1));
+        L.D0 = take(up, 4ull * std::max(L.npos, 1));
+        L.cursor = take(up, 4ull * std::max(L.bandcells, 1));
+        L.gcursor = take(up, 4ull * prep[q].groups.size());
+    }
     for (int q = 0; q < npairs; ++q) S->lay[q].topM = take(up, sizeof(T) * (S->lay[q].n + 1) * (S->lay[q].m + 1));
     // Kept group rectangles: the forward writes every group's M (and, for
     // the gap gradients, E and F) to a rectangle of its own and the backward
@@ -371,13 +416,61 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         const double c2 = c * c;
         L.log_c_total = logc * (n + m);
         std::memcpy(H + L0.rowinfo, p.rowinfo.data(), 16ull * (n + 2));
-        if (!p.crow.empty()) std::memcpy(H + L0.crow, p.crow.data(), 4ull * p.crow.size());
+        auto put = [&](size_t at, const void *src, size_t bytes) {
+            if (bytes) std::memcpy(H + at, src, bytes);
+            return Dv + at;
+        };
+        PairDev &X = ((PairDev *)(H + off_index))[q];
+        IndexPair &ix = ((IndexPair *)(H + off_index + sizeof(PairDev) * npairs))[q];
+        std::memset(&ix, 0, sizeof ix);
+        if (p.device_index) {
+            std::memset(&X, 0, sizeof X);
+            X.n = n;
+            X.m = m;
+            X.flags = p.flags;
+            X.min_col = (const int *)put(L0.min_col, p.min_col.data(), 4ull * (n + 2));
+            X.max_col = (const int *)put(L0.max_col, p.max_col.data(), 4ull * (n + 2));
+            X.rowinfo = (const int4 *)(Dv + L0.rowinfo);
+            X.cre_start = (const int *)put(L0.cre_start, p.cre_start.data(), 4ull * p.cre_start.size());
+            X.cre = (const int4 *)(Dv + L0.cre);
+            X.crow = (const int2 *)(Dv + L0.crow);
+            X.rowarc = (const int2 *)(Dv + L0.rowarc);
+            X.D = (int *)(Dv + L0.D0);
+            X.am_score = (const int *)(Dv + L0.am_score);
+            X.groups = (const GroupItem *)(Dv + L0.groups);
+            X.dw = (const int4 *)(Dv + L0.dw);
+            X.lane_groups = p.lane_groups;
+            ix.arcs = (const int4 *)put(L0.arcs4, p.arcs4.data(), 16ull * p.arcs4.size());
+            ix.lefts = (const int4 *)put(L0.lefts, p.lefts.data(), 16ull * p.lefts.size());
+            ix.nlefts = (int)p.lefts.size();
+            ix.row_start = (const int *)put(L0.row_start, p.row_start.data(), 4ull * p.row_start.size());
+            ix.row_arcs = (const int *)put(L0.row_arcs, p.row_arcs.data(), 4ull * p.row_arcs.size());
+            ix.am_lr = (const int *)put(L0.am_lr, p.am_lr.data(), 4ull * p.am_lr.size());
+            ix.am_pos = (int *)(Dv + L0.am_pos);
+            ix.cursor = (int *)(Dv + L0.cursor);
+            ix.gcursor = (int *)(Dv + L0.gcursor);
+        } else {
+            put(L0.crow, p.crow.data(), 4ull * p.crow.size());
+            put(L0.dw, p.dw.data(), sizeof(int4) * p.dw.size());
+            if (lanes) put(L0.cre, p.cre.data(), 4ull * p.cre.size());
+            put(L0.am_pos, p.am_pos.data(), 4ull * p.am_pos.size());
+            put(L0.D0, p.Dinit.data(), 4ull * p.Dinit.size());
+        }
+        put(L0.am_score, t.am_score, 4ull * L.na);
+        if (dsw[q]) put(L0.am_dsw, sp->am_dscore_dsw, 8ull * L.na);
+        PFArcMatches &am = ((PFArcMatches *)(H + S->off_am))[q];
+        am.na = L.na;
+        am.score = (const int *)(Dv + L0.am_score);
+        am.dsw = dsw[q] ? (const double *)(Dv + L0.am_dsw) : nullptr;
+        am.pos = (const int *)(Dv + L0.am_pos);
+        am.D0 = (const int *)(Dv + L0.D0);
+        am.prob = (double *)(Dv + L0.am_prob);
+        am.bandcells = L.bandcells;
+        am.zs = 0.0;
         std::memcpy(H + L0.groups, p.groups.data(), sizeof(GroupItem) * p.groups.size());
-        if (!p.dw.empty()) std::memcpy(H + L0.dw, p.dw.data(), sizeof(int4) * p.dw.size());
         std::memcpy(H + L0.rowarc, p.rowarc.data(), 4ull * p.rowarc.size());
         if (lanes) {
             if (!p.litems.empty()) std::memcpy(H + L0.litems, p.litems.data(), sizeof(LaneItem) * p.litems.size());
-            if (!p.cre.empty()) std::memcpy(H + L0.cre, p.cre.data(), 4ull * p.cre.size());
             std::memcpy(H + L0.blkrows, p.blkrows.data(), sizeof(int4) * p.blkrows.size());
             std::memcpy(H + L0.quad_start, p.quad_start.data(), 4ull * p.quad_start.size());
         }
@@ -387,26 +480,6 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         for (int i = 0; i <= n; ++i) hgA[i] = (T)(gA[i] / c);
         T *hgB = (T *)(H + L0.gB);
         for (int j = 0; j <= m; ++j) hgB[j] = (T)(gB[j] / c);
-        T *hw = (T *)(H + L0.w);
-        T *hD = (T *)(H + L0.D);
-        for (int k = 0; k < L.na; ++k) {
-            const int pos = p.am_pos[k];
-            if (pos < 0) continue;  // never a term: its right ends are not a band cell
-            const double dsw = (sp && sp->am_dscore_dsw) ? dl[2] * sp->am_dscore_dsw[k] : 0.0;
-            hw[pos] = (T)std::exp(((double)t.am_score[k] + dsw) / temp);
-            if (p.Dinit[pos] == NOT_READY) {
-                if (sizeof(T) == 8) {
-                    long long bits = PF_NOT_READY_F64;
-                    std::memcpy(&hD[pos], &bits, 8);
-                } else {
-                    int bits = PF_NOT_READY_F32;
-                    std::memcpy(&hD[pos], &bits, 4);
-                }
-            } else {
-                hD[pos] = T(0);
-            }
-        }
-        S->am_pos[q] = p.am_pos;
         PFPair<T> &d = hp[q];
         std::memset(&d, 0, sizeof d);
         d.n = n;
@@ -496,12 +569,18 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     S->lane_scratch.base = S->d_scratch;
     cudaStream_t st = e->stream;
     PF_TRY(cudaMemcpyAsync(Dv, H, zero_begin, cudaMemcpyHostToDevice, st));
-    PF_TRY(cudaMemsetAsync(Dv + zero_begin, 0, out_end - zero_begin, st));
+    PF_TRY(cudaMemsetAsync(Dv + zero_begin, 0, zero_end - zero_begin, st));
     unsigned int *qhead = (unsigned int *)(Dv + S->off_ctrl);
     int *status = (int *)(Dv + S->off_ctrl + 4);
     int *abort_flag = (int *)(Dv + S->off_ctrl + 8);
     unsigned int *topq = (unsigned int *)(Dv + S->off_ctrl + 12);
     PF_TRY(cudaEventRecord(e->ev0, st));
+    if (index_lefts >= 0)
+        PF_TRY(launch_index((const PairDev *)(Dv + off_index),
+                            (const IndexPair *)(Dv + off_index + sizeof(PairDev) * npairs), npairs, index_n,
+                            index_lefts, st));
+    PF_TRY(pf_launch_entries<T>(Dv + S->off_pairs, (const PFArcMatches *)(Dv + S->off_am), npairs, S->max_entries,
+                                o->param_delta[2], temp, st));
     if (lanes)
         PF_TRY(pf_launch_lane_fwd(Dv + S->off_pairs, npairs, (const int2 *)(Dv + S->off_queue), (int)nitems,
                                   S->lane_scratch, rb, qhead, topq, status, abort_flag, st));
@@ -519,7 +598,9 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     S->fwd_ms = ms;
     if (((int *)(H + S->off_ctrl))[1] & ST_TIMEOUT) return pf_fail(LCG_ERR_TIMEOUT, "a device wait timed out (PF forward)");
     S->log_z.resize(npairs);
+    S->zs.resize(npairs);
     for (int q = 0; q < npairs; ++q) {
+        S->zs[q] = std::exp(((double *)(H + S->lay[q].res))[0]);
         log_z[q] = ((double *)(H + S->lay[q].res))[0] + S->lay[q].log_c_total;
         S->log_z[q] = log_z[q];
     }
@@ -561,14 +642,14 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
                                  S->rb, qhead, topq, status, abort_flag, e->sms * bb, st, theta, S->gap_gradients);
     };
     PF_TRY(launch(0.0));
+    // probabilities where the sums are
+    for (int q = 0; q < S->npairs; ++q) ((PFArcMatches *)(H + S->off_am))[q].zs = S->zs[q];
+    PF_TRY(cudaMemcpyAsync(Dv + S->off_am, H + S->off_am, sizeof(PFArcMatches) * S->npairs, cudaMemcpyHostToDevice, st));
+    const PFArcMatches *const am = (const PFArcMatches *)(Dv + S->off_am);
+    PF_TRY(pf_launch_probs<T>(Dv + S->off_pairs, am, S->npairs, S->max_entries, st));
     PF_TRY(cudaEventRecord(e->ev2, st));
     PF_TRY(cudaMemcpyAsync(H + S->off_ctrl, Dv + S->off_ctrl, 64, cudaMemcpyDeviceToHost, st));
     PF_TRY(cudaMemcpyAsync(H + S->out_begin, Dv + S->out_begin, S->out_end - S->out_begin, cudaMemcpyDeviceToHost, st));
-    // D values (for the arc-match probabilities)
-    for (int q = 0; q < S->npairs; ++q)
-        if (S->lay[q].npos > 0)
-            PF_TRY(cudaMemcpyAsync(H + S->lay[q].D, Dv + S->lay[q].D, sizeof(T) * S->lay[q].npos,
-                                   cudaMemcpyDeviceToHost, st));
     PF_TRY(cudaStreamSynchronize(st));
     float ms = 0;
     cudaEventElapsedTime(&ms, e->ev1, e->ev2);
@@ -579,10 +660,9 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
         const PFLayout &L = S->lay[q];
         lcg_pf_result &r = results[q];
         const double *res = (const double *)(H + L.res);
-        const double Zs = std::exp(res[0]);  // Z in the scaled frame
-        const T *D = (const T *)(H + L.D);
-        const double *Db = (const double *)(H + L.Dbar);
-        const double *acc = (const double *)(H + L.bmacc);
+        const double Zs = S->zs[q];
+        const double *am_prob = (const double *)(H + L.am_prob);
+        const double *bm_prob = (const double *)(H + L.bmacc);  // by band cell
         const int4 *rowinfo = (const int4 *)(H + L.rowinfo);
         const lcg_pf_grad_spec *g = grads ? &grads[q] : nullptr;
         r.log_z = S->log_z[q];
@@ -597,12 +677,9 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
         const bool sw_grad = g && g->am_dscore_dsw;
         if (r.am_prob || sw_grad) {
             double dsw = 0.0;
-            const std::vector<int> &pos = S->am_pos[q];
-            for (int k = 0; k < L.na; ++k) {
-                const double p = pos[k] >= 0 ? (double)D[pos[k]] * Db[pos[k]] / Zs : 0.0;
-                if (r.am_prob) r.am_prob[k] = p;
-                if (sw_grad) dsw += p * g->am_dscore_dsw[k];
-            }
+            if (r.am_prob && L.na) std::memcpy(r.am_prob, am_prob, sizeof(double) * L.na);
+            if (sw_grad)
+                for (int k = 0; k < L.na; ++k) dsw += am_prob[k] * g->am_dscore_dsw[k];
             r.dlogz_dstruct_weight = dsw * invT;
         }
         const bool bm_grad = g && g->code_a && g->code_b;
@@ -613,7 +690,7 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
             for (int i = 1; i <= n; ++i) {
                 const int lo = std::max(1, rowinfo[i].x), hi = std::min(m, rowinfo[i].y);
                 for (int j = lo; j <= hi; ++j) {
-                    const double p = (double)acc[rowinfo[i].w + j - rowinfo[i].x] / Zs;
+                    const double p = bm_prob[rowinfo[i].w + j - rowinfo[i].x];
                     if (r.bm_prob) r.bm_prob[(size_t)i * (m + 1) + j] = p;
                     if (bm_grad && g->code_a[i] >= 0 && g->code_a[i] < 4 && g->code_b[j] >= 0 && g->code_b[j] < 4)
                         cnt[4 * g->code_a[i] + g->code_b[j]] += p;
@@ -635,6 +712,7 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
             PF_TRY(cudaMemsetAsync(Dv + S->lay[q].bmacc, 0, sizeof(double) * std::max(S->lay[q].bandcells, 1), st));
         PF_TRY(cudaMemsetAsync(Dv + S->off_ctrl, 0, 64, st));
         PF_TRY(launch(std::sqrt(S->min_am_prob)));
+        PF_TRY(pf_launch_probs<T>(Dv + S->off_pairs, am, S->npairs, S->max_entries, st));
         PF_TRY(cudaEventRecord(e->ev2, st));
         for (int q = 0; q < S->npairs; ++q)
             PF_TRY(cudaMemcpyAsync(H + S->lay[q].bmacc, Dv + S->lay[q].bmacc,
@@ -646,14 +724,13 @@ lcg_status pf_backward_t(lcg_engine e, PFState *S, const lcg_pf_grad_spec *grads
             lcg_pf_result &r = results[q];
             if (!r.bm_prob) continue;
             const PFLayout &L = S->lay[q];
-            const double Zs = std::exp(((const double *)(H + L.res))[0]);
-            const double *acc = (const double *)(H + L.bmacc);
+            const double *bm_prob = (const double *)(H + L.bmacc);
             const int4 *rowinfo = (const int4 *)(H + L.rowinfo);
             const int n = L.n, m = L.m;
             for (int i = 1; i <= n; ++i) {
                 const int lo = std::max(1, rowinfo[i].x), hi = std::min(m, rowinfo[i].y);
                 for (int j = lo; j <= hi; ++j)
-                    r.bm_prob[(size_t)i * (m + 1) + j] = acc[rowinfo[i].w + j - rowinfo[i].x] / Zs;
+                    r.bm_prob[(size_t)i * (m + 1) + j] = bm_prob[rowinfo[i].w + j - rowinfo[i].x];
             }
         }
     }

@@ -82,6 +82,9 @@ struct Prep {
 lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes = 0,
                      bool device_index = false);
 
+// whether prep_pair should leave that to the device, for these pairs
+bool index_on_device(const lcg_pair_tables *pairs, int npairs);
+
 void set_error(const std::string &msg);
 
 // the two stages of lcg_prepare_pairs (host_prep.cpp): inputs, bands and

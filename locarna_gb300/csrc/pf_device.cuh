@@ -54,6 +54,17 @@ struct PFPair {
     const int *quad_start;
 };
 
+// A pair's arc matches, in the caller's order, and its results
+struct PFArcMatches {
+    int na, bandcells;
+    const int *score;   // per arc match
+    const double *dsw;  // its derivative by the structure weight (nullptr: no offset of that)
+    const int *pos;     // its D index, -1: never a term
+    const int *D0;      // per D index: NOT_READY if a group writes it
+    double *prob;
+    double zs;          // Z in the scaled frame
+};
+
 // Scratch of the lane-per-group launches, in floats: per block, in it per warp,
 // in that for M (0: kept) and, backward, for M_bar; then the vectors per row
 struct PFLaneScratch {
@@ -76,6 +87,14 @@ template <typename T>
 cudaError_t pf_launch_back(const void *pairs, int npairs, const int2 *queue, int nitems, void *scratch,
                            long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq, int *status,
                            int *abort_flag, int blocks, cudaStream_t st, double theta = 0.0, bool grads = true);
+// w and D at the start of the forward pass; max_entries: most arc matches or band
+// cells of a pair, dsw: offset of the structure weight
+template <typename T>
+cudaError_t pf_launch_entries(const void *pairs, const PFArcMatches *am, int npairs, int max_entries, double dsw,
+                              double temperature, cudaStream_t st);
+// PFArcMatches::prob, and bmacc over Z, after a backward pass
+template <typename T>
+cudaError_t pf_launch_probs(const void *pairs, const PFArcMatches *am, int npairs, int max_entries, cudaStream_t st);
 // rb: ring size of the shared-memory rows (a power of two above the span of
 // any two consecutive band rows)
 template <typename T>

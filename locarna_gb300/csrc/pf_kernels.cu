@@ -682,7 +682,66 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
     }
 }
 
+// ---------------------------------------------------------------- arc matches
+
+constexpr int PF_ENTRY_BLOCKS = 32;  // blocks of 256 per pair at most
+
+// Boltzmann weights exp(score / temperature) (scoring.hh:857-860), scores
+// shifted by the continuous offset of the structure weight, to the D entries,
+// and the entries' state before the forward pass. With the index structures
+// made on the device (index_kernels.cu) the host touches an arc match once, to
+// count, and with the probabilities divided out here it only copies them: the host's
+// part of a forward and backward over a 200-nt pair 1.6 -> 0.8 ms, over 21 pairs of
+// 80-500 nt 20 -> 9 ms.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    pf_entries_kernel(const PFPair<T> *__restrict__ pairs, const PFArcMatches *__restrict__ ams, double dsw,
+                      double temperature) {
+    const PFPair<T> &P = pairs[blockIdx.x];
+    const PFArcMatches am = ams[blockIdx.x];
+    for (int k = blockIdx.y * 256 + threadIdx.x; k < am.na; k += gridDim.y * 256) {
+        const int pos = am.pos[k];
+        if (pos < 0) continue;  // never a term: its right ends are not a band cell
+        const double s = (double)am.score[k] + (am.dsw ? dsw * am.dsw[k] : 0.0);
+        const_cast<T *>(P.w)[pos] = (T)exp(s / temperature);
+        if (am.D0[pos] != NOT_READY) P.D[pos] = T(0);
+        else if constexpr (sizeof(T) == 8) P.D[pos] = __longlong_as_double(PF_NOT_READY_F64);
+        else P.D[pos] = __int_as_float(PF_NOT_READY_F32);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+    pf_probs_kernel(const PFPair<T> *__restrict__ pairs, const PFArcMatches *__restrict__ ams) {
+    const PFPair<T> &P = pairs[blockIdx.x];
+    const PFArcMatches am = ams[blockIdx.x];
+    const int k0 = blockIdx.y * 256 + threadIdx.x, step = gridDim.y * 256;
+    for (int k = k0; k < am.na; k += step) {
+        const int pos = am.pos[k];
+        am.prob[k] = pos >= 0 ? (double)P.D[pos] * P.Dbar[pos] / am.zs : 0.0;
+    }
+    for (int k = k0; k < am.bandcells; k += step) P.bmacc[k] /= am.zs;
+}
+
 // ---------------------------------------------------------------- launchers
+
+static dim3 pf_entry_grid(int npairs, int max_entries) {
+    return dim3(npairs, std::max(1, std::min(PF_ENTRY_BLOCKS, (max_entries + 255) / 256)));
+}
+
+template <typename T>
+cudaError_t pf_launch_entries(const void *pairs, const PFArcMatches *am, int npairs, int max_entries, double dsw,
+                              double temperature, cudaStream_t st) {
+    pf_entries_kernel<T><<<pf_entry_grid(npairs, max_entries), 256, 0, st>>>((const PFPair<T> *)pairs, am, dsw,
+                                                                            temperature);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t pf_launch_probs(const void *pairs, const PFArcMatches *am, int npairs, int max_entries, cudaStream_t st) {
+    pf_probs_kernel<T><<<pf_entry_grid(npairs, max_entries), 256, 0, st>>>((const PFPair<T> *)pairs, am);
+    return cudaGetLastError();
+}
 
 template <typename T>
 static size_t pf_smem(int rb) {
@@ -776,6 +835,12 @@ cudaError_t pf_back_occupancy(int rb, int *blocks_per_sm) {
 
 int pf_warps_per_block() { return PF_WARPS; }
 
+template cudaError_t pf_launch_entries<double>(const void *, const PFArcMatches *, int, int, double, double,
+                                               cudaStream_t);
+template cudaError_t pf_launch_entries<float>(const void *, const PFArcMatches *, int, int, double, double,
+                                              cudaStream_t);
+template cudaError_t pf_launch_probs<double>(const void *, const PFArcMatches *, int, int, cudaStream_t);
+template cudaError_t pf_launch_probs<float>(const void *, const PFArcMatches *, int, int, cudaStream_t);
 template cudaError_t pf_launch_fwd<double>(const void *, int, const int2 *, int, void *, long long, int, int,
                                            unsigned int *, unsigned int *, int *, int *, int, cudaStream_t, int, bool);
 template cudaError_t pf_launch_fwd<float>(const void *, int, const int2 *, int, void *, long long, int, int,
