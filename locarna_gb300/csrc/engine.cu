@@ -1283,7 +1283,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     // ---- scratch
     const bool sl = opts->struct_local != 0;
     const int rb = lcg_host::ring_size(span);
-    bool fast = true, lfast = true, sl_fast = true;
+    bool fast = true, lfast = true, sl_fast = true, ahead = false;
     for (auto &p : prep) {
         bool &f = (p.flags & PF_LANES) ? lfast : fast;
         f = f && (p.flags & PF_SCLS) && !(p.flags & (PF_ANCHORS | PF_NOLP | PF_STACK));
@@ -1300,7 +1300,14 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     if (!of[0].empty()) {
         int blocks_per_sm = 0;
         if (sl) CUDA_TRY(sl_prepare(sw, rb, sl_fast, keep, &blocks_per_sm));
-        else CUDA_TRY(fill_occupancy(rb, e->counting, fast, &blocks_per_sm));
+        else {
+            // Few items: half the warps an SM, twice the registers, loads ahead.
+            // Fill times with and without: 220 groups (60 nt) 60 and 64 us, 2,900
+            // (150 nt) 249 and 270, 3,900 (6 pairs of 70-110 nt) 160 and 169; 5,900
+            // (200 nt) 547 and 517, 6,700 (6 pairs of 90-130 nt) 238 and 223.
+            ahead = !e->counting && (long long)nitems[0] <= 32ll * e->sms;
+            CUDA_TRY(fill_occupancy(rb, e->counting, fast, ahead, &blocks_per_sm));
+        }
         if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
         if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
         blocks = e->sms * blocks_per_sm;
@@ -1358,7 +1365,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     if (use_graph) {
         key = {(long long)(uintptr_t)Dv, (long long)(uintptr_t)H, (long long)(uintptr_t)scratch, (long long)down_begin,
                (long long)down_end, (long long)off_ctrl, (long long)off_pairs, (long long)off_queue, (long long)nitems[0],
-               blocks, sw, rb, stride, fast, e->counting, sl, sl_fast, keep, opts->do_trace, npairs,
+               blocks, sw, rb, stride, fast, ahead, e->counting, sl, sl_fast, keep, opts->do_trace, npairs,
                (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lfast, lgroups,
                (long long)off_index, index_n, index_lefts};
         if (s.graph->exec && s.graph->key == key) {
@@ -1415,7 +1422,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             ++c.launches;
         } else if (!of[0].empty()) {
             CUDA_TRY(launch_fill(d_pairs, (const int2 *)(Dv + off_queue), (int)nitems[0], scratch, stride, sw, rb,
-                                 fast, qhead, status, abort_flag, blocks, st, counters));
+                                 fast, ahead, qhead, status, abort_flag, blocks, st, counters));
             ++c.launches;
         }
         CUDA_TRY(record(s.ev1));

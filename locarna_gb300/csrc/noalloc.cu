@@ -157,7 +157,7 @@ extern "C" lcg_status lcg_align_score_static(const lcg_pair_tables *pair, const 
     int blocks_per_sm = 0;
     const int rb = lcg_host::ring_size(p.span);
     const bool fast = (p.flags & PF_SCLS) && !(p.flags & (PF_ANCHORS | PF_NOLP | PF_STACK));
-    STATIC_TRY(fill_occupancy(rb, false, fast, &blocks_per_sm));
+    STATIC_TRY(fill_occupancy(rb, false, fast, false, &blocks_per_sm));
     int sms = 0;
     STATIC_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const size_t room = LCG_STATIC_SCRATCH_BYTES - fixed;
@@ -266,7 +266,7 @@ extern "C" lcg_status lcg_align_score_static(const lcg_pair_tables *pair, const 
     STATIC_TRY(h2d(o_D, p.Dinit.data(), 4ull * p.num_pos));
 
     STATIC_TRY_DRAIN(launch_fill((const PairDev *)(base + o_pair), (const int2 *)(base + o_queue),
-                                 (int)p.groups.size(), scratch, stride, sw, rb, fast,
+                                 (int)p.groups.size(), scratch, stride, sw, rb, fast, false,
                                  (unsigned int *)(base + o_ctrl), (int *)(base + o_ctrl + 4),
                                  (int *)(base + o_ctrl + 8), (int)blocks, s, nullptr),
                      s);

@@ -26,6 +26,10 @@ constexpr int FILL_WARPS = LCG_FILL_WARPS;  // warps per block of the fill kerne
 // shared ints per warp of the row sweep for ring size rb (see run_group)
 __host__ __device__ inline int smem_warp_ints(int rb) { return 5 * rb + 256; }
 constexpr int FILL_MIN_BLOCKS = LCG_FILL_MIN_BLOCKS;  // resident blocks per SM the register budget targets
+#ifndef LCG_FILL_AHEAD_BLOCKS
+#define LCG_FILL_AHEAD_BLOCKS 2
+#endif
+constexpr int FILL_AHEAD_BLOCKS = LCG_FILL_AHEAD_BLOCKS;  // the same of the fill kernel for few items
 constexpr int TRACE_WARPS = 4;  // warps per block of the trace kernel
 // polls of a bounded device wait (~ seconds), then ST_TIMEOUT; a test build
 // shortens it (LCG_SPIN_LIMIT)
@@ -96,8 +100,11 @@ __device__ __noinline__ int inner_term(const PairDev &P, const int4 *e, int *sta
 // penalized alignment (ModifiedScoringView, aligner_impl.hh:190-275) with
 // every position penalised by lam: sigma - 2 lam, gap costs - lam, arc-match
 // terms D(a,b) - lam (|a| + |b|) (the host bounds lam (n+m) below 2^27).
+// AHEAD: a row's first 64 entries are read a row and a half ahead of it and
+// their D and M values half a row (the corners lie four rows above at least); for
+// launches with registers to spare (sankoff_fill_kernel).
 template <int NCH, bool ANCH, bool SCLS, bool TOP, bool WAIT, bool DWRITE, bool COUNT, bool MOD = false,
-          bool INNER = true>
+          bool INNER = true, bool AHEAD = false>
 __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, int *__restrict__ Mg,
                             int pitch, int sbase, int ringn,
                             const int4 *__restrict__ dw, int ndw, bool globalA, bool globalB,
@@ -194,13 +201,56 @@ __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, in
     int4 rnxt = rowinfo[min(al + 1, P.n + 1)];
     int2 anxt = rowarc[min(al + 1, P.n + 1)];
     int cnxt = SCLS ? P.rcls[min(al + 1, P.n + 1)] : 0;
+    int2 anx2 = make_int2(0, 0);
+    int2 enx[2];            // AHEAD: the next row's first entries
+    int dvx[2], mvx[2];     // and their values, where they are terms of it
+    auto entries = [&](int2 a) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int e = a.x + 32 * u + lane;
+            enx[u] = e < a.y ? crow[e] : make_int2(0xffff, 0);
+        }
+    };
+    auto is_term = [&](int2 en, int lo, int hi) {
+        const int ca = en.x & 0xffff;
+        return ca >= al && ca != 0xffff && en.x >> 16 >= bl && en.y >= lo && en.y <= hi;
+    };
+    auto values = [&](int2 a, int4 r) {
+        const int lo = max(bl + 1, r.x), hi = min(br - 1, r.y);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const bool ok = is_term(enx[u], lo, hi);
+            const int ca = enx[u].x & 0xffff, cbl = enx[u].x >> 16, e = a.x + 32 * u + lane;
+            dvx[u] = ok ? (WAIT ? ld_volatile(Dp + e) : Dp[e]) : 0;
+            mvx[u] = ok ? Mg[(ca - al) * pitch + (cbl - bl)] : 0;
+        }
+    };
+    if (AHEAD) {
+        anx2 = rowarc[min(al + 2, P.n + 1)];
+        entries(anxt);
+        values(anxt, rnxt);
+    }
 
     for (int i = al + 1; i < ar; ++i) {
         const int4 rcur = rnxt;
         const int2 acur = anxt;
         const int rcl16 = cnxt * 16;  // SCLS: row class of row i
         rnxt = rowinfo[min(i + 1, P.n + 1)];
-        anxt = rowarc[min(i + 1, P.n + 1)];
+        int2 en0[2];
+        int dv0[2], mv0[2];
+        if (AHEAD) {
+            anxt = anx2;
+            anx2 = rowarc[min(i + 2, P.n + 1)];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                en0[u] = enx[u];
+                dv0[u] = dvx[u];
+                mv0[u] = mvx[u];
+            }
+            entries(anxt);
+        } else {
+            anxt = rowarc[min(i + 1, P.n + 1)];
+        }
         if (SCLS) cnxt = P.rcls[min(i + 1, P.n + 1)];
         const int minc = rcur.x;
         const int gAi = rcur.z - (MOD ? lam : 0);
@@ -227,7 +277,7 @@ __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, in
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int e = e0 + 32 * u + lane;
-                en[u] = e < acur.y ? crow[e] : make_int2(0xffff, 0);
+                en[u] = AHEAD && e0 == acur.x ? en0[u] : e < acur.y ? crow[e] : make_int2(0xffff, 0);
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -248,8 +298,13 @@ __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, in
                     n_terms += ok[u];
                 }
                 const int e = e0 + 32 * u + lane;
-                dv[u] = ok[u] ? (WAIT ? ld_volatile(Dp + e) : Dp[e]) : 0;
-                mv[u] = ok[u] ? Mg[(ca - al) * pitch + (cbl - bl)] : 0;
+                if (AHEAD && e0 == acur.x) {
+                    dv[u] = dv0[u];
+                    mv[u] = mv0[u];
+                } else {
+                    dv[u] = ok[u] ? (WAIT ? ld_volatile(Dp + e) : Dp[e]) : 0;
+                    mv[u] = ok[u] ? Mg[(ca - al) * pitch + (cbl - bl)] : 0;
+                }
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -262,6 +317,7 @@ __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, in
             }
             if (ball[0] != 0xffffffffu || ball[1] != 0xffffffffu) break;
         }
+        if (AHEAD) values(anxt, rnxt);
         __syncwarp();
         int B;  // M(i, lo-1)
         if (minc <= bl) {
@@ -443,7 +499,7 @@ __device__ void run_group_c(const PairDev &P, int al, int ar, int bl, int br, in
 // FAST: every pair of the launch has a sigma class table, no anchors, no
 // lonely-pair or stacking terms (INNER = false: the D writes are the plain
 // fill_D_entries, so this hot instantiation carries no inner-term code).
-template <bool TOP, bool WAIT, bool DWRITE, bool COUNT = false, bool FAST = false, bool MOD = false>
+template <bool TOP, bool WAIT, bool DWRITE, bool COUNT = false, bool FAST = false, bool MOD = false, bool AHEAD = false>
 __device__ __forceinline__ void run_group(const PairDev &P, int cpl, int al, int ar, int bl, int br,
                                           int *__restrict__ Mg, int pitch, int sbase, int ringn,
                                           const int4 *__restrict__ dw, int ndw,
@@ -451,23 +507,23 @@ __device__ __forceinline__ void run_group(const PairDev &P, int cpl, int al, int
                                           volatile int *abort_flag, TopOut *tout,
                                           unsigned long long *counters = nullptr, int lam = 0) {
     if (FAST)
-        run_group_c<4, false, true, TOP, WAIT, DWRITE, COUNT, MOD, false>(P, al, ar, bl, br, Mg, pitch, sbase, ringn,
+        run_group_c<4, false, true, TOP, WAIT, DWRITE, COUNT, MOD, false, AHEAD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn,
                                                                           dw, ndw, globalA, globalB, local_top, status,
                                                                           abort_flag, tout, counters, lam);
     else if ((P.flags & PF_ANCHORS) && (P.flags & PF_SCLS))
-        run_group_c<4, true, true, TOP, WAIT, DWRITE, COUNT, MOD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
+        run_group_c<4, true, true, TOP, WAIT, DWRITE, COUNT, MOD, true, AHEAD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
                                                              globalA, globalB, local_top, status, abort_flag,
                                                              tout, counters, lam);
     else if (P.flags & PF_ANCHORS)
-        run_group_c<4, true, false, TOP, WAIT, DWRITE, COUNT, MOD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
+        run_group_c<4, true, false, TOP, WAIT, DWRITE, COUNT, MOD, true, AHEAD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
                                                               globalA, globalB, local_top, status, abort_flag,
                                                               tout, counters, lam);
     else if (P.flags & PF_SCLS)
-        run_group_c<4, false, true, TOP, WAIT, DWRITE, COUNT, MOD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
+        run_group_c<4, false, true, TOP, WAIT, DWRITE, COUNT, MOD, true, AHEAD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
                                                               globalA, globalB, local_top, status, abort_flag,
                                                               tout, counters, lam);
     else
-        run_group_c<4, false, false, TOP, WAIT, DWRITE, COUNT, MOD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
+        run_group_c<4, false, false, TOP, WAIT, DWRITE, COUNT, MOD, true, AHEAD>(P, al, ar, bl, br, Mg, pitch, sbase, ringn, dw, ndw,
                                                                globalA, globalB, local_top, status, abort_flag,
                                                                tout, counters, lam);
 }
@@ -490,7 +546,7 @@ static __device__ __forceinline__ void warp_argmax(int &v, int &k1, int &k2) {
 
 // top level + final argmax: align_top_level_free_endgaps (aligner.cc:736-819)
 // and align_top_level_locally (aligner.cc:823-880)
-template <bool COUNT, bool FAST = false, bool MOD = false>
+template <bool COUNT, bool FAST = false, bool MOD = false, bool AHEAD = false>
 __device__ __forceinline__ void run_top(const PairDev &P, int cpl, int sbase, int ringn,
                                      int *status, volatile int *abort_flag,
                                      unsigned long long *counters, int lam = 0,
@@ -507,7 +563,7 @@ __device__ __forceinline__ void run_top(const PairDev &P, int cpl, int sbase, in
     const int fe = P.free_endgaps;
     TopOut to;
     if (local) {
-        run_group<true, !MOD, false, COUNT, FAST, MOD>(P, cpl, sA - 1, n + 1, sB - 1, m + 1, Mg, m1, sbase, ringn,
+        run_group<true, !MOD, false, COUNT, FAST, MOD, AHEAD>(P, cpl, sA - 1, n + 1, sB - 1, m + 1, Mg, m1, sbase, ringn,
                                                       nullptr, 0, false, false, true, status, abort_flag,
                                                       &to, counters, lam);
         int v = to.best, i = to.bi, j = to.bj;
@@ -529,7 +585,7 @@ __device__ __forceinline__ void run_top(const PairDev &P, int cpl, int sbase, in
         }
         return;
     }
-    run_group<true, !MOD, false, COUNT, FAST, MOD>(P, cpl, sA - 1, n + 1, sB - 1, m + 1, Mg, m1, sbase, ringn,
+    run_group<true, !MOD, false, COUNT, FAST, MOD, AHEAD>(P, cpl, sA - 1, n + 1, sB - 1, m + 1, Mg, m1, sbase, ringn,
                                                   nullptr, 0, !(fe & 4), !(fe & 1), false, status, abort_flag,
                                                   &to, counters, lam);
     __syncwarp();

@@ -35,8 +35,14 @@
 
 namespace lcg {
 
-template <bool COUNT, bool FAST>
-__global__ void __launch_bounds__(FILL_WARPS * 32, FILL_MIN_BLOCKS)
+// A row is a chain of latencies (its entries, their values, the maxima, the scan),
+// which 32 warps an SM hide from one another at 64 registers. A launch of fewer
+// groups than that has nothing to hide them with: AHEAD takes 16 warps an SM and up
+// to 128 registers, reads entries and values ahead and spills nothing (one 60-nt
+// pair 64 -> 60 us, one 150-nt pair 270 -> 249 us). At 64 registers the same
+// loads spill and cost more than they hide (one 400-nt pair 3.3 -> 3.9 ms).
+template <bool COUNT, bool FAST, bool AHEAD>
+__global__ void __launch_bounds__(FILL_WARPS * 32, AHEAD ? FILL_AHEAD_BLOCKS : FILL_MIN_BLOCKS)
     sankoff_fill_kernel(const PairDev *__restrict__ pairs, const int2 *__restrict__ queue,
                         int nitems, int *scratch,
                         long long scratch_stride, int sw, int rb, unsigned int *qhead, int *status,
@@ -56,11 +62,11 @@ __global__ void __launch_bounds__(FILL_WARPS * 32, FILL_MIN_BLOCKS)
         const GroupItem it = P.groups[qi.y];
         const int4 *__restrict__ dw = P.dw;
         if (it.top) {
-            run_top<COUNT, FAST>(P, it.cpl, sbase, rb, status, abort_flag, counters);
+            run_top<COUNT, FAST, false, AHEAD>(P, it.cpl, sbase, rb, status, abort_flag, counters);
         } else {
             // the group's own kept rectangle, or the warp's scratch slot
             const bool kept = P.rect && it.rect_off >= 0;
-            run_group<false, true, true, COUNT, FAST>(P, it.cpl, it.al, it.ar, it.bl, it.br,
+            run_group<false, true, true, COUNT, FAST, false, AHEAD>(P, it.cpl, it.al, it.ar, it.bl, it.br,
                                                 kept ? P.rect + it.rect_off : Mg, kept ? it.br - it.bl : sw,
                                                 sbase, rb, dw + it.dw_start, it.dw_count, true, true, false,
                                                 status, abort_flag, nullptr, counters);
@@ -156,28 +162,21 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
 
 // ---------------------------------------------------------------- launchers
 
-template <bool COUNT, bool FAST>
-static const void *fill_fn() {
-    return (const void *)sankoff_fill_kernel<COUNT, FAST>;
+using FillKernel = void (*)(const PairDev *, const int2 *, int, int *, long long, int, int, unsigned int *, int *,
+                            int *, unsigned long long *);
+static FillKernel fill_kernel(bool counting, bool fast, bool ahead) {
+    if (counting) return fast ? sankoff_fill_kernel<true, true, false> : sankoff_fill_kernel<true, false, false>;
+    if (ahead) return fast ? sankoff_fill_kernel<false, true, true> : sankoff_fill_kernel<false, false, true>;
+    return fast ? sankoff_fill_kernel<false, true, false> : sankoff_fill_kernel<false, false, false>;
 }
 
 cudaError_t launch_fill(const PairDev *pairs, const int2 *queue, int nitems,
-                        int *scratch, long long scratch_stride, int sw, int rb, bool fast, unsigned int *qhead,
-                        int *status, int *abort_flag, int blocks, cudaStream_t st,
+                        int *scratch, long long scratch_stride, int sw, int rb, bool fast, bool ahead,
+                        unsigned int *qhead, int *status, int *abort_flag, int blocks, cudaStream_t st,
                         unsigned long long *counters) {
     size_t smem = (size_t)FILL_WARPS * smem_warp_ints(rb) * sizeof(int);
-    if (counters && fast)
-        sankoff_fill_kernel<true, true><<<blocks, FILL_WARPS * 32, smem, st>>>(
-            pairs, queue, nitems, scratch, scratch_stride, sw, rb, qhead, status, abort_flag, counters);
-    else if (counters)
-        sankoff_fill_kernel<true, false><<<blocks, FILL_WARPS * 32, smem, st>>>(
-            pairs, queue, nitems, scratch, scratch_stride, sw, rb, qhead, status, abort_flag, counters);
-    else if (fast)
-        sankoff_fill_kernel<false, true><<<blocks, FILL_WARPS * 32, smem, st>>>(
-            pairs, queue, nitems, scratch, scratch_stride, sw, rb, qhead, status, abort_flag, counters);
-    else
-        sankoff_fill_kernel<false, false><<<blocks, FILL_WARPS * 32, smem, st>>>(
-            pairs, queue, nitems, scratch, scratch_stride, sw, rb, qhead, status, abort_flag, counters);
+    fill_kernel(counters != nullptr, fast, ahead)<<<blocks, FILL_WARPS * 32, smem, st>>>(
+        pairs, queue, nitems, scratch, scratch_stride, sw, rb, qhead, status, abort_flag, counters);
     return cudaGetLastError();
 }
 
@@ -245,7 +244,7 @@ cudaError_t launch_gather_res(const PairDev *pairs, const int *items, int nitems
 int fill_warps_per_block() { return FILL_WARPS; }
 int trace_warps_per_block() { return TRACE_WARPS; }
 
-cudaError_t fill_occupancy(int rb, bool counting, bool fast, int *blocks_per_sm) {
+cudaError_t fill_occupancy(int rb, bool counting, bool fast, bool ahead, int *blocks_per_sm) {
     size_t smem = (size_t)FILL_WARPS * smem_warp_ints(rb) * sizeof(int);
     int dev = 0, optin = 0;
     cudaError_t ge = cudaGetDevice(&dev);
@@ -255,8 +254,7 @@ cudaError_t fill_occupancy(int rb, bool counting, bool fast, int *blocks_per_sm)
         *blocks_per_sm = 0;
         return cudaSuccess;
     }
-    const void *k = counting ? (fast ? fill_fn<true, true>() : fill_fn<true, false>())
-                             : (fast ? fill_fn<false, true>() : fill_fn<false, false>());
+    const void *k = (const void *)fill_kernel(counting, fast, ahead);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

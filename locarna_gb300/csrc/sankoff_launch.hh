@@ -9,10 +9,11 @@
 
 namespace lcg {
 // fast: every pair has a sigma class table and no anchor constraints
+// ahead (fill_ahead, not when counting): the kernel for few items
 // queue: (pair, group) work items in dependency-respecting order
 cudaError_t launch_fill(const PairDev *pairs, const int2 *queue, int nitems, int *scratch,
-                        long long scratch_stride, int sw, int rb, bool fast, unsigned int *qhead, int *status,
-                        int *abort_flag, int blocks, cudaStream_t st, unsigned long long *counters);
+                        long long scratch_stride, int sw, int rb, bool fast, bool ahead, unsigned int *qhead,
+                        int *status, int *abort_flag, int blocks, cudaStream_t st, unsigned long long *counters);
 // the lane-per-group fill (pairs with PF_LANES); queue: (pair, lane item)
 // work items, item nlitems = the top level; per warp `slot` ints of matrix
 // storage (0 with kept rectangles) and `qslot` ints of gap states in scratch
@@ -30,7 +31,7 @@ cudaError_t launch_top(const PairDev *pairs, const int *items, int nitems, const
                        int *status, cudaStream_t st);
 // out[5 q + k] = result word k (score, max_i, max_j, min_i, min_j) of pair items[q]
 cudaError_t launch_gather_res(const PairDev *pairs, const int *items, int nitems, int *out, cudaStream_t st);
-cudaError_t fill_occupancy(int rb, bool counting, bool fast, int *blocks_per_sm);
+cudaError_t fill_occupancy(int rb, bool counting, bool fast, bool ahead, int *blocks_per_sm);
 cudaError_t trace_prepare(int rb);
 int fill_warps_per_block();
 int trace_warps_per_block();
