@@ -54,12 +54,27 @@ __device__ __forceinline__ int maxplus_scan(int a, int b, int x0, int lane) {
     return max(addc(x0, a), b);
 }
 
-// One left-end group with exclusions. Mg holds NS state matrices, state s at
-// Mg + s*mstride (NS = 4 in the fill: the states arc terms read; 8 in the
-// traceback recomputation).
+// The states of a matrix cell lie together (NS ints: four in a warp's slot of the
+// fill, which are those that arc terms read; eight where the traceback walks), so
+// that a term is one 16-byte load: with a matrix per state its four words came from
+// four sectors of L2 and DRAM (fill of a 400 x 400 pair 8.3 -> 7.8 ms, traceback 0.75 ->
+// 0.64). What bounds the fill is the latency of a row's entries and their terms
+// with 16 warps an SM (116 registers, 14 KB of rows a warp; issue slots a quarter
+// used, DRAM 1.4 of 6.8 TB/s): entries read a row, or 32, ahead 9.6 -> 8.3 ms; 64 at
+// a time gave nothing more.
+template <int NS>
+__device__ __forceinline__ void sl_put(int *Mg, long long cell, int m0, int m1, int m2, int m3, int m4, int m5, int m6,
+                                       int m7) {
+    int4 *const p = (int4 *)(Mg + cell * NS);
+    p[0] = make_int4(m0, m1, m2, m3);
+    if (NS == 8) p[1] = make_int4(m4, m5, m6, m7);
+}
+
+// One left-end group with exclusions. Mg holds NS states per cell, rows of
+// `pitch` cells.
 template <bool WAIT, bool DWRITE, int NS>
 __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, int *__restrict__ Mg,
-                             long long mstride, int pitch, int *sm, int sw,
+                             int pitch, int *sm, int sw,
                              const int4 *__restrict__ dw, int ndw, int *status,
                              volatile int *abort_flag) {
     const int lane = threadIdx.x & 31;
@@ -102,9 +117,7 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
                 const int c = j - bl;
                 prev[0][c] = vg; prev[1][c] = vg; prev[4][c] = vg;
                 prev[2][c] = vx; prev[3][c] = vx; prev[5][c] = vx;
-                int vals[8] = {vg, vg, vx, vx, vg, v0, vx, v0};
-#pragma unroll
-                for (int s2 = 0; s2 < NS; ++s2) Mg[s2 * mstride + c] = vals[s2];
+                sl_put<NS>(Mg, c, vg, vg, vx, vx, vg, v0, vx, v0);
             }
             carry += __shfl_sync(0xffffffffu, s, 31);
             blocked_carry = blocked_carry || bm != 0;
@@ -112,8 +125,7 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
         if (lane == 0) {
 #pragma unroll
             for (int k = 0; k < 6; ++k) prev[k][0] = 0;
-#pragma unroll
-            for (int s2 = 0; s2 < NS; ++s2) Mg[s2 * mstride] = 0;
+            sl_put<NS>(Mg, 0, 0, 0, 0, 0, 0, 0, 0, 0);
         }
         if (al + 1 < ar) {
             int L1 = min(br, P.max_col[al + 1] + 1);
@@ -145,10 +157,8 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
             Bs[0] = bg; Bs[2] = bg; Bs[5] = bg;
             Bs[1] = bx; Bs[3] = bx; Bs[7] = bx;
             Bs[4] = b0; Bs[6] = b0;
-            if (lane == 0) {
-#pragma unroll
-                for (int s2 = 0; s2 < NS; ++s2) Mg[s2 * mstride + (long long)(i - al) * pitch] = Bs[s2];
-            }
+            if (lane == 0)
+                sl_put<NS>(Mg, (long long)(i - al) * pitch, Bs[0], Bs[1], Bs[2], Bs[3], Bs[4], Bs[5], Bs[6], Bs[7]);
         } else {
 #pragma unroll
             for (int s2 = 0; s2 < 8; ++s2) Bs[s2] = NEG;
@@ -190,8 +200,11 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
                         if (blq <= bl) continue;
                         const int dv = WAIT ? wait_D(P.D, ent.x, status, abort_flag) : P.D[ent.x];
                         const long long o = (long long)(alq - 1 - al) * pitch + (blq - 1 - bl);
-#pragma unroll
-                        for (int s2 = 0; s2 < 4; ++s2) arcv[s2] = max(arcv[s2], Mg[s2 * mstride + o] + dv);
+                        const int4 mv = *(const int4 *)(Mg + o * NS);
+                        arcv[0] = max(arcv[0], mv.x + dv);
+                        arcv[1] = max(arcv[1], mv.y + dv);
+                        arcv[2] = max(arcv[2], mv.z + dv);
+                        arcv[3] = max(arcv[3], mv.w + dv);
                     }
                 }
             }
@@ -260,9 +273,7 @@ __device__ void run_group_sl(const PairDev &P, int al, int ar, int bl, int br, i
                 cur[3][c] = M3;
                 cur[4][c] = M4;
                 cur[5][c] = M6;
-                const int vals[8] = {M0, M1, M2, M3, M4, M5, M6, M7};
-#pragma unroll
-                for (int s2 = 0; s2 < NS; ++s2) Mg[s2 * mstride + roff + j] = vals[s2];
+                sl_put<NS>(Mg, roff + j, M0, M1, M2, M3, M4, M5, M6, M7);
             }
         }
         __syncwarp();
@@ -332,10 +343,8 @@ __device__ __forceinline__ int fscan_prefix(int x, int pa, int gdel, int &Pc, in
 }
 
 // One left-end group with exclusions, fast path: pairs without anchor
-// constraints and with a sigma class table (PF_SCLS). Writes NS state
-// matrices to Mg (state s at Mg + s*mstride; NS = 4 in the fill: the states
-// arc terms read; 8 in the traceback recomputation) and, with DWRITE, the
-// group's D entries.
+// constraints and with a sigma class table (PF_SCLS). Writes NS states per
+// cell to Mg (rows of `pitch` cells) and, with DWRITE, the group's D entries.
 // The states, their order and values are those of run_group_sl; what
 // differs is how they are computed:
 //  * shared-memory rows are indexed by ring position (column j at j mod
@@ -355,7 +364,7 @@ __device__ __forceinline__ int fscan_prefix(int x, int pa, int gdel, int &Pc, in
 // 11-14 arc-term maxima of 0-3; then the class table.
 template <bool WAIT, bool DWRITE, int NS>
 __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, int *__restrict__ Mg,
-                              long long mstride, int pitch, int sbase, int ringn,
+                              int pitch, int sbase, int ringn,
                               const int4 *__restrict__ dw, int ndw, int *status, volatile int *abort_flag) {
     const int lane = threadIdx.x & 31;
     const int go = P.go, X = P.excl;
@@ -396,24 +405,13 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
         ROW(2)[rj] = X;
         ROW(3)[rj] = X;
         ROW(5)[rj] = X;
-        const int c = j - bl;
-        Mg[c] = vg;
-        Mg[mstride + c] = vg;
-        Mg[2 * mstride + c] = X;
-        Mg[3 * mstride + c] = X;
-        if (NS == 8) {
-            Mg[4 * mstride + c] = vg;
-            Mg[5 * mstride + c] = 0;
-            Mg[6 * mstride + c] = X;
-            Mg[7 * mstride + c] = 0;
-        }
+        sl_put<NS>(Mg, j - bl, vg, vg, X, X, vg, 0, X, 0);
     }
     if (lane == 0) {
         const int r0 = RG(bl);
 #pragma unroll
         for (int k = 0; k < 6; ++k) ROW(k)[r0] = 0;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) Mg[s * mstride] = 0;
+        sl_put<NS>(Mg, 0, 0, 0, 0, 0, 0, 0, 0, 0);
     }
     // cells above the band of row al+1
     if (al + 1 < ar) {
@@ -433,12 +431,17 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
     int4 rnxt = rowinfo[min(al + 1, P.n + 1)];
     int2 anxt = rowarc[min(al + 1, P.n + 1)];
     int cnxt = P.rcls[min(al + 1, P.n + 1)];
+    // a row's first 32 entries are loaded a row ahead, the further ones 32 ahead
+    int2 anx2 = rowarc[min(al + 2, P.n + 1)];
+    auto entry = [&](int e, int end) { return e < end ? crow[e] : make_int2(0xffff, 0); };
+    int2 enx = entry(anxt.x + lane, anxt.y);
     for (int i = al + 1; i < ar; ++i) {
         const int4 rcur = rnxt;
         const int2 acur = anxt;
         const int rcl16 = cnxt * 16;
         rnxt = rowinfo[min(i + 1, P.n + 1)];
-        anxt = rowarc[min(i + 1, P.n + 1)];
+        anxt = anx2;
+        anx2 = rowarc[min(i + 2, P.n + 1)];
         cnxt = P.rcls[min(i + 1, P.n + 1)];
         const int minc = rcur.x;
         const int gAi = rcur.z;
@@ -449,7 +452,8 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
         bool rowarcs = false;
         for (int e0 = acur.x; e0 < acur.y; e0 += 32) {
             const int e = e0 + lane;
-            const int2 en = e < acur.y ? crow[e] : make_int2(0xffff, 0);
+            const int2 en = enx;
+            enx = entry(e + 32, acur.y);
             const int ca = en.x & 0xffff, cbl = en.x >> 16;  // inner corner (a.l-1, b.l-1)
             const bool okA = ca >= al && ca != 0xffff;       // a.l > al
             const unsigned ball = __ballot_sync(0xffffffffu, okA);
@@ -458,9 +462,8 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
             if (okA && cbl >= bl && en.y >= lo && en.y <= hi) {
                 int dv = WAIT ? ld_volatile(Dp + e) : Dp[e];
                 const long long o = (long long)(ca - al) * pitch + (cbl - bl);
-                int mv[4];
-#pragma unroll
-                for (int s = 0; s < 4; ++s) mv[s] = Mg[s * mstride + o];
+                const int4 m = *(const int4 *)(Mg + o * NS);
+                const int mv[4] = {m.x, m.y, m.z, m.w};
                 if (WAIT && dv == NOT_READY) dv = wait_D(Dp, e, status, abort_flag);
                 const int rr = RG(en.y);
 #pragma unroll
@@ -468,6 +471,7 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
             }
             if (ball != 0xffffffffu) break;
         }
+        enx = entry(anxt.x + lane, anxt.y);
         __syncwarp();
 
         // ---- column bl (aligner.cc:264-368 by state) and the row's start
@@ -477,19 +481,7 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
             B0 = colg;
             B1 = X;
             B4 = 0;
-            if (lane == 0) {
-                const long long r = (long long)(i - al) * pitch;
-                Mg[r] = B0;
-                Mg[mstride + r] = B1;
-                Mg[2 * mstride + r] = B0;
-                Mg[3 * mstride + r] = B1;
-                if (NS == 8) {
-                    Mg[4 * mstride + r] = B4;
-                    Mg[5 * mstride + r] = B0;
-                    Mg[6 * mstride + r] = B4;
-                    Mg[7 * mstride + r] = B1;
-                }
-            }
+            if (lane == 0) sl_put<NS>(Mg, (long long)(i - al) * pitch, B0, B1, B0, B1, B4, B0, B4, B1);
         }
         // lane 0: the diagonal carries (row i-1 at column lo-1), then column
         // lo-1 of row i
@@ -597,16 +589,7 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
                 ROW(3)[rj] = M3;
                 ROW(4)[rj] = M4;
                 ROW(5)[rj] = M6;
-                Mg[roff + j] = M0;
-                Mg[mstride + roff + j] = M1;
-                Mg[2 * mstride + roff + j] = M2;
-                Mg[3 * mstride + roff + j] = M3;
-                if (NS == 8) {
-                    Mg[4 * mstride + roff + j] = M4;
-                    Mg[5 * mstride + roff + j] = M5;
-                    Mg[6 * mstride + roff + j] = M6;
-                    Mg[7 * mstride + roff + j] = M7;
-                }
+                sl_put<NS>(Mg, roff + j, M0, M1, M2, M3, M4, M5, M6, M7);
             }
         }
         __syncwarp();
@@ -649,9 +632,9 @@ __device__ void run_group_slf(const PairDev &P, int al, int ar, int bl, int br, 
 }
 
 // KEEP: the chunk keeps its group rectangles (PairDev::rect); a group with
-// a kept rectangle writes all eight states there, interleaved by row (row
-// i-al of state s at rect + 8 rect_off + (i-al) 8w + s w, w = br - bl), so
-// that the traceback walks it instead of recomputing it.
+// a kept rectangle writes all eight states there (cell (i-al) w + j - bl, w =
+// br - bl, at rect + 8 rect_off), so that the traceback walks it instead of
+// recomputing it.
 template <bool FAST, bool KEEP>
 __global__ void __launch_bounds__(SL_FILL_WARPS * 32)
     sankoff_sl_fill_kernel(const PairDev *__restrict__ pairs, const int2 *__restrict__ queue,
@@ -681,16 +664,16 @@ __global__ void __launch_bounds__(SL_FILL_WARPS * 32)
             const int w = it.br - it.bl;
             int *Mk = P.rect + 8ll * it.rect_off;
             if (FAST)
-                run_group_slf<true, true, 8>(P, it.al, it.ar, it.bl, it.br, Mk, w, 8 * w, (int)(sm - smem), rb,
+                run_group_slf<true, true, 8>(P, it.al, it.ar, it.bl, it.br, Mk, w, (int)(sm - smem), rb,
                                              dw + it.dw_start, it.dw_count, status, abort_flag);
             else
-                run_group_sl<true, true, 8>(P, it.al, it.ar, it.bl, it.br, Mk, w, 8 * w, sm, sw,
+                run_group_sl<true, true, 8>(P, it.al, it.ar, it.bl, it.br, Mk, w, sm, sw,
                                             dw + it.dw_start, it.dw_count, status, abort_flag);
         } else if (FAST) {
-            run_group_slf<true, true, 4>(P, it.al, it.ar, it.bl, it.br, Mg, scratch_stride, sw, (int)(sm - smem), rb,
+            run_group_slf<true, true, 4>(P, it.al, it.ar, it.bl, it.br, Mg, sw, (int)(sm - smem), rb,
                                 dw + it.dw_start, it.dw_count, status, abort_flag);
         } else {
-            run_group_sl<true, true, 4>(P, it.al, it.ar, it.bl, it.br, Mg, scratch_stride, sw, sm, sw,
+            run_group_sl<true, true, 4>(P, it.al, it.ar, it.bl, it.br, Mg, sw, sm, sw,
                                         dw + it.dw_start, it.dw_count, status, abort_flag);
         }
         __syncwarp();
@@ -700,16 +683,17 @@ __global__ void __launch_bounds__(SL_FILL_WARPS * 32)
 // ---------------------------------------------------------------- traceback
 
 // trace_in_arcmatch (aligner.cc:1233-1343) as a loop over (state, i, j), by a
-// whole warp; M of state s is Mg + s*mstride (the top level has only state
-// NO_NO).
-static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, long long mstride, int pitch,
+// whole warp; ns states per cell (1: the top level, which has only state NO_NO),
+// rows of `pitch` cells.
+static __device__ __noinline__ void walk_sl(Walker &w, const int *Mg, int ns, int pitch,
                                             int al, int bl, int state, int i, int j, bool tl,
                                             int *status, int lam = 0) {
     const PairDev &P = w.P;
     const bool local = P.flags & PF_SEQU_LOCAL;
     const int fe = P.free_endgaps;
     const int X = P.excl, lane = threadIdx.x & 31;
-#define MS(s, x, y) Mg[(long long)(s) * mstride + (long long)((x) - al) * pitch + ((y) - bl)]
+    const int smask = ns == 1 ? 0 : 7;
+#define MS(s, x, y) Mg[((long long)((x) - al) * pitch + ((y) - bl)) * ns + ((s) & smask)]
     // cells above (left of) (i, j) in `state` that hold the same value, up to 32
     auto run_up = [&](int Mij) {
         const unsigned no = __ballot_sync(0xffffffffu, !(i - lane > al && MS(state, i - lane - 1, j) == Mij));
@@ -809,7 +793,7 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
     __syncwarp();
     {
         const int sA = sel.rst ? sel.rst[pair].x : 1, sB = sel.rst ? sel.rst[pair].y : 1;
-        walk_sl(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), 0, P.m + 1, sA - 1, sB - 1, S_NO_NO,
+        walk_sl(w, P.topM + (size_t)(sA - 1) * (P.m + 1) + (sB - 1), 1, P.m + 1, sA - 1, sB - 1, S_NO_NO,
                 P.res[R_MAXI], P.res[R_MAXJ], true, status, lam);
         if (lane == 0) P.segs[0] = make_int4(-1, 0, w.ntok, 0);
         nseg = 1;
@@ -842,17 +826,15 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         // from the fill, else recomputed into the pair's scratch slot
         const int2 kr = P.am_rect ? P.am_rect[k] : make_int2(-1, 0);
         const int *Mw = Mg;
-        long long ms = scratch_stride;
         int pw = sw;
         if (kr.x >= 0) {
             Mw = P.rect + 8ll * kr.x;
-            ms = kr.y;
-            pw = 8 * kr.y;
+            pw = kr.y;
         } else if (FAST) {
-            run_group_slf<false, false, 8>(P, ends.x, ends.y, ends.z, ends.w, Mg, scratch_stride, sw,
+            run_group_slf<false, false, 8>(P, ends.x, ends.y, ends.z, ends.w, Mg, sw,
                                            (int)(sm - smem), rb, nullptr, 0, status, (volatile int *)&dummy_abort);
         } else {
-            run_group_sl<false, false, 8>(P, ends.x, ends.y, ends.z, ends.w, Mg, scratch_stride, sw, sm, sw,
+            run_group_sl<false, false, 8>(P, ends.x, ends.y, ends.z, ends.w, Mg, sw, sm, sw,
                                           nullptr, 0, status, (volatile int *)&dummy_abort);
         }
         __syncwarp();
@@ -866,8 +848,8 @@ __global__ void __launch_bounds__(TRACE_WARPS * 32)
         const int dv = nolp ? kpos : P.D[kpos], sc = nolp ? 0 : P.am_score[k];
         const int start = w.ntok;
         for (int s2 = 0; s2 < 4; ++s2) {
-            if (dv == Mw[s2 * ms + o] + sc) {
-                walk_sl(w, Mw, ms, pw, ends.x, ends.z, s2, ar - 1, br - 1, false, status);
+            if (dv == Mw[8 * o + s2] + sc) {
+                walk_sl(w, Mw, 8, pw, ends.x, ends.z, s2, ar - 1, br - 1, false, status);
                 break;
             }
         }
