@@ -402,18 +402,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         const double ow = std::exp(((double)t.indel_opening + dl[1]) / temp);
         double logc = 0.0;
         if (sizeof(T) == 4) logc = seq_log_pf(t, bm, gA, gB, ow) / (double)(n + m);
-        double c = std::exp(logc);
-        // the estimate moved so that the first gap weight over it is a float: the
-        // others mostly equal it, and a rounded weight's error adds up over the
-        // gaps of an alignment (80 against 439 nt: 360 of them)
-        if (sizeof(T) == 4) {
-            const double g = gB[1] / (double)(float)(gB[1] / c);
-            if (std::isfinite(g) && g > 0.0) {
-                c = g;
-                logc = std::log(c);
-            }
-        }
-        const double c2 = c * c;
+        const double c = std::exp(logc), c2 = c * c;
         L.log_c_total = logc * (n + m);
         std::memcpy(H + L0.rowinfo, p.rowinfo.data(), 16ull * (n + 2));
         auto put = [&](size_t at, const void *src, size_t bytes) {
