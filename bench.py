@@ -601,7 +601,7 @@ def run_ours(args):
         eng.run_pp_call(pcall)  # results are on the host when it returns
         wall_s += time.perf_counter() - s0
         phases = [a + b for a, b in zip(phases, eng.last_phases())]
-        e2e_launches += eng.last_stats()[1] + 1  # + the envelope launch
+        e2e_launches += eng.last_stats()[1] + 2  # + the envelope's two launches
     barrier_sync(world)
     res = Engine.decode_pp_call(pcall)
     graph_captures, graph_replays = eng.last_graphs()

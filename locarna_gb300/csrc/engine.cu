@@ -830,6 +830,9 @@ struct Chunk {
 int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg_align_opts *opts) {
     if (e->counting || opts->struct_local) return 0;
     if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) == 64 ? 64 : std::atoi(v) == 32 ? 32 : 0;
+    // without lonely pairs few arc matches are left, and lanes idle (276 pairs of
+    // 60-400 nt: 4.6 ms with one warp per group, 14.7 with 32 groups)
+    if (opts->no_lonely_pairs) return 0;
     double cells = 0, longest = 0;
     for (int q = 0; q < npairs; ++q) {
         const lcg_pair_tables &t = pairs[q];
@@ -839,7 +842,6 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
         cells += 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
         longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
     }
-    if (opts->no_lonely_pairs) cells /= 50;  // few arc matches have a stacked partner
     const double warp = cells / 80 + longest / 6, l32 = cells / 130 + 0.6 * longest, l64 = cells / 170 + 1.4 * longest;
     return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
 }
