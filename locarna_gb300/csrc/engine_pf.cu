@@ -483,7 +483,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         d.gA = (const T *)(Dv + L0.gA);
         d.gB = (const T *)(Dv + L0.gB);
         d.o = (T)ow;
-        d.gu = hgB[1];
+        d.gu = sizeof(T) == 8 || !o->gap_gradients ? hgB[1] : T(0);
         for (int j = 2; j <= m && d.gu > T(0); ++j)
             if (hgB[j] != hgB[1]) d.gu = T(0);
         T *hgp = (T *)(H + L0.gpow);

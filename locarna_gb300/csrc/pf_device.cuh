@@ -22,7 +22,7 @@ struct PFPair {
     const T *bm;           // (n+1)(m+1) scaled base-match weights
     const T *gA, *gB;      // scaled gap weights
     T o;                   // gap-opening weight
-    T gu;                  // the value of every gB[j], j >= 1, if they are all the same, else 0
+    T gu;                  // the value of every gB[j], j >= 1, if they are all the same, else 0; 0 in FP32 with gap gradients
     const T *gpow;         // 33: its powers 0 to 32, each rounded once
     T inv_s;               // 1 / pf_scale
     T arcf;                // pf_scale / c^4

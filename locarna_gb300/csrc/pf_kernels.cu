@@ -46,14 +46,14 @@ namespace lcg {
 // descending) are read 32 at a time until the first a.l <= al, and each term
 // M(a.l-1,b.l-1) D(am) s is summed into its column with a shared-memory
 // atomicAdd. COUNTU counts the uses of every D entry (for the backward pass).
-template <typename T, bool WAIT, bool DWRITE, bool COUNTU, bool SAVE, bool SAVEEF = true>
+template <typename T, bool WAIT, bool DWRITE, bool COUNTU, bool SAVE, bool SAVEEF, bool UNI>
 __device__ void pf_group_sweep(const PFPair<T> &P, int al, int ar, int bl, int br, T *__restrict__ Mg,
                                T *__restrict__ Eg, T *__restrict__ Fg, int pitch, PFRows<T> R,
                                const int4 *__restrict__ dw, int ndw, int *status, volatile int *abort_flag) {
     const int lane = threadIdx.x & 31;
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
-    const bool uni = P.gu > T(0);
+    const bool uni = UNI && P.gu > T(0);
     const PFPow<T> W = pf_pow(P);
     const T guo = P.gu * o, wl = P.gpow[lane + 1];
 #define RG(j) ((j) - R.rb * (int)__umulhi((unsigned)(j), R.magic))
@@ -305,11 +305,11 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
             const int w = it.br - it.bl;
             const size_t sz = (size_t)(it.ar - it.al) * w;
             T *Mk = P.rect + (size_t)KEEP * it.rect_off;
-            pf_group_sweep<T, true, true, true, true, KEEP == 3>(P, it.al, it.ar, it.bl, it.br, Mk, Mk + sz,
+            pf_group_sweep<T, true, true, true, true, KEEP == 3, pf_factors<T>(EF)>(P, it.al, it.ar, it.bl, it.br, Mk, Mk + sz,
                                                                  Mk + 2 * sz, w, R, P.dw + it.dw_start, it.dw_count,
                                                                  status, abort_flag);
         } else {
-            pf_group_sweep<T, true, true, true, false>(P, it.al, it.ar, it.bl, it.br, Mg, nullptr, nullptr, pitch, R,
+            pf_group_sweep<T, true, true, true, false, false, pf_factors<T>(EF)>(P, it.al, it.ar, it.bl, it.br, Mg, nullptr, nullptr, pitch, R,
                                                        P.dw + it.dw_start, it.dw_count, status, abort_flag);
         }
         __syncwarp();
@@ -347,7 +347,7 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
     const int lane = threadIdx.x & 31;
     const int m1 = P.m + 1;
     const T o = P.o, arcf = P.arcf;
-    const bool uni = P.gu > T(0);
+    const bool uni = pf_factors<T>(GRADS) && P.gu > T(0);
     const PFPow<T> W = pf_pow(P);
     const T guo = P.gu * o, wr = P.gpow[32 - lane];
     T *const Eb = R.E;
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(PF_WARPS * 32, pf_min_blocks<T>())
             Ew = Mw + sz;
             Fw = Ew + sz;
         } else {
-            pf_group_sweep<T, false, false, false, true, GRADS>(P, al, ar, bl, br, Mg, Eg, Fg, pitch, R, nullptr,
+            pf_group_sweep<T, false, false, false, true, GRADS, pf_factors<T>(GRADS)>(P, al, ar, bl, br, Mg, Eg, Fg, pitch, R, nullptr,
                                                                 0, status, abort_flag);
         }
         __syncwarp();

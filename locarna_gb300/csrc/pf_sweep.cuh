@@ -55,6 +55,14 @@ template <typename T>
 struct PFPow {
     T p[5];
 };
+// With gap gradients the FP32 sweeps keep the scan of pairs (a, b), and gu is then 0
+// in all of them, so that all round a run of gaps alike: at 64 registers the factors
+// cost that backward pass more than they save (28 pairs of 160-200 nt: 26.5 ms
+// against 25.7; without gap gradients a 200-nt pair 2.43 ms against 2.64).
+template <typename T>
+__host__ __device__ constexpr bool pf_factors(bool grads) {
+    return sizeof(T) == 8 || !grads;
+}
 template <typename T>
 __device__ __forceinline__ PFPow<T> pf_pow(const PFPair<T> &P) {
     PFPow<T> w;
