@@ -240,8 +240,9 @@ lcg_status lcg_engine_set_graphs(lcg_engine eng, int32_t on);
  * recomputes.
  * LocARNA-P (lcg_pf_forward / lcg_pf_backward) keeps the groups' M (and E, F
  * for the gap gradients) from the forward for the backward pass under the
- * same budget, by default in FP64 only (4 GiB; in FP32 the backward's
- * recomputation is faster than reading the kept values back). */
+ * same budget, by default in FP64 (4 GiB) and for FP32 batches swept lane per
+ * group (16 GiB); in other FP32 calls the backward's recomputation is faster
+ * than reading the kept values back. */
 lcg_status lcg_engine_set_rect_budget(lcg_engine eng, int64_t bytes);
 /* Graph captures and replays of the last lcg_align_pairs call. */
 lcg_status lcg_engine_last_graphs(lcg_engine eng, int64_t *captures, int64_t *replays);
