@@ -331,7 +331,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         S->d_arena = nullptr;
         S->cap = 0;
         // with room to grow, else without, else without the kept rectangles
-        for (size_t bytes : {total + total / 4, total, bare}) {
+        for (size_t bytes : {total + std::min<size_t>(total / 4, (size_t)1 << 30), total, bare}) {
             if (cudaMalloc(&S->d_arena, bytes) == cudaSuccess) {
                 S->cap = bytes;
                 break;
