@@ -818,31 +818,45 @@ struct Chunk {
 // (sankoff_fill_kernel). An estimate of the three fill times from the pairs'
 // sizes; the constants are fits to measured fills on a GB300. Matrix cells:
 // 2 (n + m) per arc match within 30 % over 60-500 nt. One warp per group fills
-// 80 cells/ns, lane per group 130 (32 groups) or 170 (64). A lane item is
-// serial: the longest one of a pair takes 2.2 us per quad and 50 ns per arc
-// match, and a launch ends with six tenths of that (64 groups: 1.4 times), where
-// the row sweep of one group takes a sixth. So single pairs and small batches go
-// to one warp per group (one 400 x 400 pair: 3.1 ms against 9.6 ms), batches to
-// lanes (fill of 28 profile pairs of 80-300 columns: 5.0 -> 4.7 ms with 32
-// groups, 5.9 with 64; 45 stacking pairs of 100-300 nt: 8.6 -> 6.7, 7.4 with 64;
-// 66 pairs of 60-300 nt: 8.9 -> 7.4 with either; 276 pairs of 60-400 nt in two
-// chunks: 126 -> 82, 64 with 64).
+// 80 cells/ns (dense scores 58, stacking 70) and ends with an eighth of the
+// longest pair's time in lanes, L = 2.2 us per quad and 50 ns per arc match. A
+// lane item is serial: a launch takes 1.38 L (64 groups: 2 L) and 1 ns per 250
+// (530) cells, or, when there is enough to do, 1 ns per 120 (150) cells. So
+// single pairs and small batches go to one warp per group (one 400 x 400 pair:
+// 3.1 ms against 9.6; 15 pairs of 200-300 nt: 6.0 against 7.3), batches to lanes
+// (28 profile pairs of 80-300 columns: 5.6 against 4.9 with 32 groups; 28 pairs of
+// 200-300 nt 10.1 -> 8.8, 45 stacking pairs of 100-300 nt 9.0 -> 6.7; 276 pairs of
+// 60-400 nt in two chunks: 130 -> 84, 70 with 64).
 int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg_align_opts *opts) {
     if (e->counting || opts->struct_local) return 0;
     if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) == 64 ? 64 : std::atoi(v) == 32 ? 32 : 0;
     // without lonely pairs few arc matches are left, and lanes idle (276 pairs of
     // 60-400 nt: 4.6 ms with one warp per group, 14.7 with 32 groups)
     if (opts->no_lonely_pairs) return 0;
-    double cells = 0, longest = 0;
+    double cells = 0, warp = 0, longest = 0;
     for (int q = 0; q < npairs; ++q) {
         const lcg_pair_tables &t = pairs[q];
-        if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || !t.min_col || !t.max_col) continue;
+        if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || t.len_b < 1 || !t.sigma || !t.min_col || !t.max_col)
+            continue;
         double band = 0;
         for (int i = 0; i <= t.len_a; ++i) band += t.max_col[i] - t.min_col[i] + 1;
-        cells += 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
+        // dense scores: more than 16 values in a row (single sequences: 4)
+        const int *const row = t.sigma + (size_t)((t.len_a + 1) / 2) * (t.len_b + 1);
+        int value[16], nv = 0;
+        for (int j = 1; j <= t.len_b && nv <= 16; ++j) {
+            const int x = row[j];
+            if (std::find(value, value + nv, x) != value + nv) continue;
+            if (nv < 16) value[nv] = x;
+            ++nv;
+        }
+        const double c = 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
+        cells += c;
+        warp += c / (nv > 16 ? 58 : t.am_stack_score ? 70 : 80);
         longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
     }
-    const double warp = cells / 80 + longest / 6, l32 = cells / 130 + 0.6 * longest, l64 = cells / 170 + 1.4 * longest;
+    warp += longest / 8;
+    const double l32 = std::max(cells / 250 + 1.38 * longest, cells / 120);
+    const double l64 = std::max(cells / 530 + 2 * longest, cells / 150);
     return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
 }
 
