@@ -117,7 +117,8 @@ __device__ __forceinline__ T ld_cg(const T *p) { return __ldcg(p); }
 // of 80-240 nt, which is little else, 2.1 -> 0.9. A row costs 6 to 8 us still:
 // some 20 FP64 operations a column at 2 a clock per SM, L2 latency of M_bar and
 // of the entries, and the fence before the counters. Entries
-// loaded a row ahead and longer naps of the waiting warps changed nothing.
+// loaded a row ahead, two columns a thread and longer naps of the waiting warps
+// changed nothing.
 
 // The recurrence x -> a x + b over the block's threads, in thread order, from
 // the value c before the first one (the same in all threads): c becomes the
