@@ -416,7 +416,9 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
             std::memset(&X, 0, sizeof X);
             X.n = n;
             X.m = m;
-            X.flags = p.flags;
+            // the recursions know no stacking: stacking tables are ignored,
+            // and the index has no inner arc matches
+            X.flags = p.flags & ~PF_STACK;
             X.min_col = (const int *)put(L0.min_col, p.min_col.data(), 4ull * (n + 2));
             X.max_col = (const int *)put(L0.max_col, p.max_col.data(), 4ull * (n + 2));
             X.rowinfo = (const int4 *)(Dv + L0.rowinfo);

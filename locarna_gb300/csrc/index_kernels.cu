@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(INDEX_WARPS * 32)
     const int4 left = X.lefts[w];  // (first and past its last arc, first and past its last group)
     int4 *const dw = (int4 *)P.dw;
     int2 *const dwn = (int2 *)P.dwn;
-    const bool lanes = P.flags & PF_LANES, stack = P.flags & PF_STACK;
+    const bool lanes = P.flags & PF_LANES, stack = (P.flags & PF_STACK) && X.inner_a;
     for (int g = left.z + lane; g < left.w; g += 32) X.gcursor[g] = P.groups[g].dw_start;
     __syncwarp();
     for (int s = left.x; s < left.y; ++s) {
