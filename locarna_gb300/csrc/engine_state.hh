@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdlib>
 #include <vector>
 
 #include "../../include/locarna_gb300.h"
@@ -96,10 +97,30 @@ struct lcg_engine_s {
     size_t env_dev_cap = 0;
     char *env_host = nullptr;
     size_t env_host_cap = 0;
+    // most bytes a wave of envelopes takes: a wave that could not be allocated
+    // halves it for the engine's later calls
+    size_t env_wave_bytes = (size_t)16 << 30;
     // bytes the last lcg_prepare_pairs call copied host->device / device->host
     long long prep_h2d = 0, prep_d2h = 0;
 };
 
 namespace lcg_host {
+// cudaMalloc that leaves *p null and the runtime's last error clear on failure.
+// A test build (LCG_TEST_ALLOC) refuses what is larger than $LCG_TEST_ALLOC_BYTES.
+template <typename T>
+cudaError_t device_alloc(T **p, size_t bytes) {
+    cudaError_t e = cudaSuccess;
+#ifdef LCG_TEST_ALLOC
+    if (const char *v = std::getenv("LCG_TEST_ALLOC_BYTES"))
+        if (bytes > (size_t)std::atoll(v)) e = cudaErrorMemoryAllocation;
+#endif
+    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+    }
+    return e;
+}
+
 void pf_release(lcg_engine_s *e);
 }

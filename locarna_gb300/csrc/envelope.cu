@@ -428,9 +428,9 @@ struct Pending {
     cudaEvent_t done = nullptr;
 };
 
-// One wave (pairs [q0, q1) whose rows fit the device budget) staged,
-// enqueued and, with wait, finished; without wait the wave's outputs are
-// described in *pend.
+// One wave (pairs [q0, q1), wave_end) staged, enqueued and, with wait, finished;
+// without wait the wave's outputs are described in *pend. LCG_ERR_NOMEM: nothing
+// is enqueued.
 static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1, const PairIn *in, PairOut *out,
                                bool wait, Pending *pend, std::string &err);
 
@@ -457,18 +457,21 @@ static EnvConst make_const(const Params &Pm) {
     return C;
 }
 
-static size_t wave_end(const PairIn *in, int q0, int npairs) {
-    // waves of pairs whose forward rows fit a device budget
-    const size_t budget = (size_t)16 << 30;
-    size_t fz_bytes = 0;
-    int q1 = q0;
-    for (; q1 < npairs; ++q1) {
-        const size_t n1 = (size_t)in[q1].n + 1, m1 = (size_t)in[q1].m + 1;
-        const size_t f = 8 * 7 * n1 * m1 + 8 * n1;
-        if (q1 > q0 && fz_bytes + f > budget) break;
-        fz_bytes += f;
-    }
-    return (size_t)q1;
+// device bytes of a pair beside its staged inputs: forward and reverse rows (three
+// states each) and match weights, 56 bytes a cell, and the rows' exponents
+static size_t pair_bytes(const PairIn &p) {
+    const size_t n1 = (size_t)p.n + 1, m1 = (size_t)p.m + 1;
+    return 8 * 7 * n1 * m1 + 8 * n1;
+}
+
+// the wave that starts with pair q0: at least that pair, and as many as the
+// engine's budget takes
+static int wave_end(lcg_engine eng, const PairIn *in, int q0, int npairs, size_t *bytes = nullptr) {
+    size_t sum = pair_bytes(in[q0]);
+    int q1 = q0 + 1;
+    for (; q1 < npairs && sum + pair_bytes(in[q1]) <= eng->env_wave_bytes; ++q1) sum += pair_bytes(in[q1]);
+    if (bytes) *bytes = sum;
+    return q1;
 }
 
 lcg_status compute(lcg_engine eng, const Params &Pm, int npairs, const PairIn *in, PairOut *out, std::string &err) {
@@ -480,9 +483,15 @@ lcg_status compute(lcg_engine eng, const Params &Pm, int npairs, const PairIn *i
     }
     const EnvConst C = make_const(Pm);
     for (int q0 = 0; q0 < npairs;) {
-        const int q1 = (int)wave_end(in, q0, npairs);
-        lcg_status rc = enqueue_wave(eng, C, q0, q1, in, out, true, nullptr, err);
-        if (rc != LCG_OK) return rc;
+        size_t bytes;
+        const int q1 = wave_end(eng, in, q0, npairs, &bytes);
+        const lcg_status rc = enqueue_wave(eng, C, q0, q1, in, out, true, nullptr, err);
+        if (rc == LCG_ERR_NOMEM && q1 - q0 > 1) {
+            eng->env_wave_bytes = bytes / 2;  // in smaller waves
+            continue;
+        }
+        if (rc == LCG_ERR_NOMEM) out[q0].flag = 2;  // a pair too large for the memory left: the host's
+        else if (rc != LCG_OK) return rc;
         q0 = q1;
     }
     return LCG_OK;
@@ -498,13 +507,16 @@ lcg_status compute_begin(lcg_engine eng, const Params &Pm, int npairs, const Pai
         return LCG_ERR_CUDA;
     }
     // more than one wave: computed now (the pinned staging holds one wave)
-    if ((int)wave_end(in, 0, npairs) < npairs) return compute(eng, Pm, npairs, in, out, err);
+    size_t bytes;
+    if (wave_end(eng, in, 0, npairs, &bytes) < npairs) return compute(eng, Pm, npairs, in, out, err);
     auto *p = new Pending;
     lcg_status rc = enqueue_wave(eng, make_const(Pm), 0, npairs, in, out, false, p, err);
     if (rc != LCG_OK) {
         if (p->done) cudaEventDestroy(p->done);
         delete p;
-        return rc;
+        if (rc != LCG_ERR_NOMEM) return rc;
+        eng->env_wave_bytes = bytes / 2;
+        return compute(eng, Pm, npairs, in, out, err);
     }
     *pending = p;
     return LCG_OK;
@@ -558,27 +570,28 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
     const size_t out_end = hs;
     size_t ds = hs;  // device-only section after the mirrored staging
     dev_off.resize(nq);
-    for (int k = 0; k < nq; ++k) {
-        const size_t n1 = (size_t)in[q0 + k].n + 1, m1 = (size_t)in[q0 + k].m + 1;
-        dev_off[k] = take(ds, 8 * 7 * n1 * m1 + 8 * n1);
-    }
+    for (int k = 0; k < nq; ++k) dev_off[k] = take(ds, pair_bytes(in[q0 + k]));
     // the buffers are reused only after the previous computation ended
     // (compute waits; a pending one is ended before the next begins)
     if (ds > eng->env_dev_cap) {
         if (eng->env_dev) cudaFree(eng->env_dev);
         eng->env_dev = nullptr;
         eng->env_dev_cap = 0;
-        if (cudaMalloc(&eng->env_dev, ds + ds / 4) != cudaSuccess) {
+        // with room to grow, else without; else the caller takes a smaller wave
+        for (size_t cap : {ds + std::min<size_t>(ds / 4, (size_t)1 << 30), ds})
+            if (!eng->env_dev_cap && lcg_host::device_alloc(&eng->env_dev, cap) == cudaSuccess) eng->env_dev_cap = cap;
+        if (!eng->env_dev_cap) {
             err = "envelope device allocation failed";
             return LCG_ERR_NOMEM;
         }
-        eng->env_dev_cap = ds + ds / 4;
     }
     if (out_end > eng->env_host_cap) {
         if (eng->env_host) cudaFreeHost(eng->env_host);
         eng->env_host = nullptr;
         eng->env_host_cap = 0;
         if (cudaMallocHost(&eng->env_host, out_end + out_end / 4) != cudaSuccess) {
+            cudaGetLastError();
+            eng->env_host = nullptr;
             err = "envelope pinned allocation failed";
             return LCG_ERR_NOMEM;
         }

@@ -39,13 +39,14 @@ struct PairIn {
 // restrict_by_trace_probabilities before clamping, n+1 each) and a flag:
 // 0 = exact, 1 = a probability within the rounding margin of the threshold
 // could move a bound, 2 = values outside the safe range of the reference's
-// float type. Flagged pairs are recomputed on the host.
+// float type, or a pair that the device has no memory for. Flagged pairs are
+// recomputed on the host.
 struct PairOut {
     int32_t *newmin, *newmax;
     int flag;
 };
 
-// Compute the envelopes of npairs pairs on the engine's device (one warp per
+// Compute the envelopes of npairs pairs on the engine's device (one block per
 // pair). Returns LCG_OK or an error with err set.
 lcg_status compute(lcg_engine eng, const Params &P, int npairs, const PairIn *in, PairOut *out, std::string &err);
 
