@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -56,6 +57,7 @@ struct EnvConst {
     double sw, itemp, go, ge, gopen1, min_prob, mu;
     double score[16];
     int local, fe, rfe, exp_limit;
+    int range;  // rows are scaled back once their largest value leaves 2^-range .. 2^range
 };
 
 // value = v * 2^e, v kept in [1, 2) (or 0)
@@ -150,7 +152,6 @@ struct EnvShare {
     int hmax[4];
 };
 
-constexpr int ENV_RANGE = 128;
 
 // One direction of the partition function (PFGotoh::pf_gotoh, edge_probs.icc:
 // 76-162) by 128 threads: rows in order, 128 columns at a time. The gap chain
@@ -158,9 +159,9 @@ constexpr int ENV_RANGE = 128;
 // warp (constant factors where its 32 columns are all in the band), the warps'
 // totals combined through shared memory. Rows are kept in HBM for the edge
 // probabilities and, where they fit, two of them in shared memory. A row that
-// has left 2^-ENV_RANGE .. 2^ENV_RANGE is scaled back to 1 .. 2 by a power of
-// two (exact); zexp holds the exponents. Returns the flag (2: values that the
-// reference's float type would not hold); local alignment: *zloc, the sum of zM.
+// has left 2^-range .. 2^range is scaled back to 1 .. 2 by a power of two
+// (exact); zexp holds the exponents. Returns the flag (2: values that the
+// reference's float type or the scaled FP64 rows would not hold); local alignment: *zloc, the sum of zM.
 template <bool REV>
 __device__ int env_pass(const EnvDev &P, const EnvConst &C, double *rows, EnvShare &sh, XAcc *zloc) {
     const int tid = threadIdx.x & (ENV_SIDE - 1), lane = tid & 31, sub = tid >> 5;
@@ -299,8 +300,8 @@ __device__ int env_pass(const EnvDev &P, const EnvConst &C, double *rows, EnvSha
             mx = fmax(fmax(sh.top[0], sh.top[1]), fmax(sh.top[2], sh.top[3]));
             d = mx > 0.0 ? ilogb(mx) : 0;
         }
-        if (e + d + 2 > C.exp_limit) flag = 2;
-        if (d > ENV_RANGE || d < -ENV_RANGE) {
+        if (e + d + 2 > C.exp_limit || d > 1023) flag = 2;
+        if (d > C.range || d < -C.range) {
             for (int k = tid; k < 3 * m1; k += ENV_SIDE) {
                 const double v = ldexp(cur[k], -d);
                 cur[k] = v;
@@ -434,7 +435,7 @@ struct Pending {
 static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1, const PairIn *in, PairOut *out,
                                bool wait, Pending *pend, std::string &err);
 
-static EnvConst make_const(const Params &Pm) {
+static EnvConst make_const(const Params &Pm, int npairs, const PairIn *in) {
     EnvConst C;
     C.sw = Pm.sw;
     C.itemp = 1.0 / Pm.temp;
@@ -453,7 +454,16 @@ static EnvConst make_const(const Params &Pm) {
     if (Pm.fe & LCG_FREE_RIGHT_2) rfe |= LCG_FREE_LEFT_2;
     C.rfe = rfe;
     C.exp_limit = Pm.exp_limit;
-
+    // A row may stay within 2^-128 .. 2^128 unscaled where a row's step (a match
+    // weight, and a gap of any length) changes it by far less than the rest of
+    // FP64's range; else every row is scaled to 1 .. 2, and the step has all of it.
+    int max_m = 0;
+    double score = 0.0;
+    for (int q = 0; q < npairs; ++q) max_m = std::max(max_m, in[q].m);
+    for (double s : Pm.score) score = std::max(score, std::fabs(s));
+    const double step = (2.0 * std::fabs(Pm.sw) + score) * std::fabs(C.itemp) / std::log(2.0) +
+                        std::fabs(std::log2(Pm.g_open)) + max_m * std::max(0.0, std::log2(Pm.g_ext));
+    C.range = step < 256.0 ? 128 : 0;
     return C;
 }
 
@@ -481,7 +491,7 @@ lcg_status compute(lcg_engine eng, const Params &Pm, int npairs, const PairIn *i
         err = std::string("cudaSetDevice: ") + cudaGetErrorString(ce);
         return LCG_ERR_CUDA;
     }
-    const EnvConst C = make_const(Pm);
+    const EnvConst C = make_const(Pm, npairs, in);
     for (int q0 = 0; q0 < npairs;) {
         size_t bytes;
         const int q1 = wave_end(eng, in, q0, npairs, &bytes);
@@ -510,7 +520,7 @@ lcg_status compute_begin(lcg_engine eng, const Params &Pm, int npairs, const Pai
     size_t bytes;
     if (wave_end(eng, in, 0, npairs, &bytes) < npairs) return compute(eng, Pm, npairs, in, out, err);
     auto *p = new Pending;
-    lcg_status rc = enqueue_wave(eng, make_const(Pm), 0, npairs, in, out, false, p, err);
+    lcg_status rc = enqueue_wave(eng, make_const(Pm, npairs, in), 0, npairs, in, out, false, p, err);
     if (rc != LCG_OK) {
         if (p->done) cudaEventDestroy(p->done);
         delete p;
