@@ -35,6 +35,7 @@
 #include "../../include/locarna_gb300.h"
 #include "engine_state.hh"
 #include "envelope.hh"
+#include "smem_limit.hh"
 
 namespace {
 
@@ -668,7 +669,7 @@ static lcg_status enqueue_wave(lcg_engine eng, const EnvConst &C, int q0, int q1
     }
     env_weights_kernel<<<dim3(nq, (max_n + 7) / 8), 256, 0, st>>>((const EnvDev *)(D + o_pairs), C);
     const size_t smem = std::min<size_t>(ENV_ROW_SMEM, 4 * 3 * sizeof(double) * (size_t)(max_m + 1));
-    if ((ce = cudaFuncSetAttribute(envelope_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+    if ((ce = lcg::allow_smem((const void *)envelope_kernel, smem)) != cudaSuccess)
         return fail_cuda(ce, "envelope launch");
     envelope_kernel<<<nq, ENV_THREADS, smem, st>>>((const EnvDev *)(D + o_pairs), C, smem);
     if ((ce = cudaGetLastError()) != cudaSuccess) return fail_cuda(ce, "envelope launch");

@@ -35,6 +35,7 @@
 #include "lcg_device.cuh"
 #include "pf_device.cuh"
 #include "pf_sweep.cuh"
+#include "smem_limit.hh"
 
 namespace lcg {
 
@@ -757,7 +758,7 @@ cudaError_t pf_launch_fwd(const void *pairs, int npairs, const int2 *queue, int 
              : keep_states == 1 ? pf_fwd_kernel<T, 1, false>
              : top_ef           ? pf_fwd_kernel<T, 0, true>
                                 : pf_fwd_kernel<T, 0, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)k, smem);
     if (e != cudaSuccess) return e;
     k<<<blocks, PF_WARPS * 32, smem, st>>>((const PFPair<T> *)pairs, npairs, queue, nitems, (T *)scratch, stride,
                                            pitch, rb, qhead, topq, status, abort_flag);
@@ -786,7 +787,7 @@ static cudaError_t pf_cap_blocks(K kernel, const char *var, size_t smem, int *bl
 template <typename T>
 cudaError_t pf_fwd_occupancy(int rb, int *blocks_per_sm) {
     const size_t smem = pf_smem<T>(rb);
-    cudaError_t e = cudaFuncSetAttribute(pf_fwd_kernel<T, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)pf_fwd_kernel<T, 0, true>, smem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pf_fwd_kernel<T, 0, true>, PF_WARPS * 32, smem);
     if (e != cudaSuccess) return e;
@@ -798,8 +799,7 @@ static cudaError_t pf_launch_back_k(const void *pairs, int npairs, const int2 *q
                                     long long stride, int pitch, int rb, unsigned int *qhead, unsigned int *topq,
                                     int *status, int *abort_flag, int blocks, cudaStream_t st, double theta) {
     const size_t smem = pf_smem<T>(rb);
-    cudaError_t e = cudaFuncSetAttribute(pf_back_kernel<T, TRUNC, GRADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = allow_smem((const void *)pf_back_kernel<T, TRUNC, GRADS>, smem);
     if (e != cudaSuccess) return e;
     pf_back_kernel<T, TRUNC, GRADS><<<blocks, PF_WARPS * 32, smem, st>>>(
         (const PFPair<T> *)pairs, npairs, queue, nitems, (T *)scratch, stride, pitch, rb, qhead, topq, status,
@@ -824,8 +824,7 @@ cudaError_t pf_launch_back(const void *pairs, int npairs, const int2 *queue, int
 template <typename T>
 cudaError_t pf_back_occupancy(int rb, int *blocks_per_sm) {
     const size_t smem = pf_smem<T>(rb);
-    cudaError_t e = cudaFuncSetAttribute(pf_back_kernel<T, false, true>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)pf_back_kernel<T, false, true>, smem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pf_back_kernel<T, false, true>, PF_WARPS * 32,
                                                       smem);

@@ -44,6 +44,7 @@
 
 #include "lane_sweep.cuh"
 #include "pf_sweep.cuh"
+#include "smem_limit.hh"
 
 namespace lcg {
 
@@ -914,7 +915,7 @@ static size_t pfl_smem(bool back, int rb) {
 }
 
 static cudaError_t pfl_occupancy(const void *fn, size_t smem, int *blocks_per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(fn, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, LANE_WARPS * 32, smem);
 }

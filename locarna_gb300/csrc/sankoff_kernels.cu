@@ -32,6 +32,7 @@
 #include <stdint.h>
 
 #include "sankoff_group.cuh"
+#include "smem_limit.hh"
 
 namespace lcg {
 
@@ -225,11 +226,8 @@ cudaError_t launch_top(const PairDev *pairs, const int *items, int nitems, const
                        int *status, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
     size_t smem = (size_t)TRACE_WARPS * smem_warp_ints(rb) * sizeof(int);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(sankoff_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem((const void *)sankoff_top_kernel, smem);
+    if (e != cudaSuccess) return e;
     int blocks = (nitems + TRACE_WARPS - 1) / TRACE_WARPS;
     sankoff_top_kernel<<<blocks, TRACE_WARPS * 32, smem, st>>>(pairs, items, nitems, lam, rst, rb, status);
     return cudaGetLastError();
@@ -255,19 +253,13 @@ cudaError_t fill_occupancy(int rb, bool counting, bool fast, bool ahead, int *bl
         return cudaSuccess;
     }
     const void *k = (const void *)fill_kernel(counting, fast, ahead);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(k, smem);
+    if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, k, FILL_WARPS * 32, smem);
 }
 
 cudaError_t trace_prepare(int rb) {
-    size_t smem = (size_t)TRACE_WARPS * smem_warp_ints(rb) * sizeof(int);
-    if (smem > 48 * 1024)
-        return cudaFuncSetAttribute(sankoff_trace_kernel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return cudaSuccess;
+    return allow_smem((const void *)sankoff_trace_kernel, (size_t)TRACE_WARPS * smem_warp_ints(rb) * sizeof(int));
 }
 
 }  // namespace lcg

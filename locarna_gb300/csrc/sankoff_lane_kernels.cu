@@ -57,6 +57,7 @@
 
 #include "lane_sweep.cuh"
 #include "sankoff_launch.hh"
+#include "smem_limit.hh"
 
 namespace lcg {
 
@@ -472,7 +473,7 @@ cudaError_t lane_occupancy(int groups, int rb, bool fast, int *blocks_per_sm) {
     if (e != cudaSuccess) return e;
     *blocks_per_sm = 0;
     if (smem > (size_t)optin) return cudaSuccess;
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(fn, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, fn, LANE_WARPS * 32, smem);
 }

@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "sankoff_group.cuh"
+#include "smem_limit.hh"
 
 namespace lcg {
 
@@ -889,12 +890,12 @@ cudaError_t sl_prepare(int sw, int rb, bool fast, bool keep, int *blocks_per_sm)
                          : (const void *)sankoff_sl_fill_kernel<false, false>;
     const void *kk = fast ? (const void *)sankoff_sl_fill_kernel<true, true>
                           : (const void *)sankoff_sl_fill_kernel<false, true>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = allow_smem(kk, smem);
     if (e != cudaSuccess) return e;
     const void *kt = fast ? (const void *)sankoff_sl_trace_kernel<true> : (const void *)sankoff_sl_trace_kernel<false>;
-    e = cudaFuncSetAttribute(kt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_t);
+    e = allow_smem(kt, smem_t);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, keep ? kk : k, SL_FILL_WARPS * 32, smem);
 }
