@@ -238,6 +238,13 @@ lcg_status lcg_engine_set_graphs(lcg_engine eng, int32_t on);
  * 64 groups) and 32 GiB for structure-local chunks (a 400 x 400 nt pair takes
  * ~25 GB). Where the device has not that much memory left, the chunk
  * recomputes.
+ * A batch filled lane per group whose storage is not kept takes its warps'
+ * slots from scratch: up to 24 GiB by default; with bytes >= 0 up to `bytes` or
+ * what the slots of one warp per group take (some GiB for sequences of
+ * hundreds of nt), whichever is more, and where few warps fit in that, the
+ * batch is filled by one warp per group. Every in-flight chunk (two at most)
+ * has its own, held until the engine is destroyed. LocARNA-P's FP32 batches
+ * likewise.
  * LocARNA-P (lcg_pf_forward / lcg_pf_backward) keeps the groups' M (and E, F
  * for the gap gradients) from the forward for the backward pass under the
  * same budget, by default in FP64 (4 GiB) and for FP32 batches swept lane per

@@ -10,6 +10,7 @@
 #include <atomic>
 #include <cstdio>
 #include <chrono>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -753,7 +754,7 @@ struct Assembler {
     }
 };
 
-// at most this much scratch for the slots of a lane-per-group launch
+// scratch for the slots of a lane-per-group launch, unless the caller sets a budget
 constexpr long long LANE_SCRATCH_BYTES = 24ll << 30;
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -814,6 +815,20 @@ struct Chunk {
     bool no_keep = false;  // the kept rectangles did not fit the device's memory
 };
 
+// Whether a lane-per-group launch whose slots leave it `blocks` of the `want` blocks
+// that it has items and room on the SMs for is better left to one warp per group. With
+// 608 blocks wanted, 24 RNAs of 60-400 nt take 79 ms (all blocks), 99 (257), 127 (171)
+// and 144 (141; one warp per group 144), 10 of 500-600 nt 241 (366), 298 (274) and 411
+// (183; 322), 6 of 1000-1100 nt 1617 (323) and 1761 (215; 1665).
+bool few_blocks(long long blocks, long long want) { return blocks < 1 || 5 * blocks < 2 * want; }
+
+// Bytes of slots that a lane-per-group launch may have: a bounded amount, or the
+// caller's budget (lcg_engine_set_rect_budget), but at least what those of the fill
+// with one warp per group take (other).
+long long lane_slot_bytes(lcg_engine e, long long other) {
+    return std::max(e->rect_budget < 0 ? LANE_SCRATCH_BYTES : e->rect_budget, other);
+}
+
 // Groups per item of the lane-per-group fill for a chunk, 0: one warp per group
 // (sankoff_fill_kernel). An estimate of the three fill times from the pairs'
 // sizes; the constants are fits to measured fills on a GB300. Matrix cells:
@@ -833,7 +848,7 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
     // without lonely pairs few arc matches are left, and lanes idle (276 pairs of
     // 60-400 nt: 4.6 ms with one warp per group, 14.7 with 32 groups)
     if (opts->no_lonely_pairs) return 0;
-    double cells = 0, warp = 0, longest = 0;
+    double cells = 0, warp = 0, longest = 0, max_band = 0, max_area = 0;
     for (int q = 0; q < npairs; ++q) {
         const lcg_pair_tables &t = pairs[q];
         if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || t.len_b < 1 || !t.sigma || !t.min_col || !t.max_col)
@@ -853,10 +868,22 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
         cells += c;
         warp += c / (nv > 16 ? 58 : t.am_stack_score ? 70 : 80);
         longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
+        max_band = std::max(max_band, band);
+        max_area = std::max(max_area, (t.len_a + 1.0) * (t.len_b + 2.0));
     }
+    // The share of the wanted blocks that the slots have room for (a line of `width`
+    // ints per band cell and warp), unless the items' storage is kept (about twice
+    // their groups' cells): a fill with fewer blocks is slower by as much. (chunk_launch
+    // has the exact sizes, after a preparation that it would have to repeat.)
+    const double keep = e->rect_budget < 0 ? (double)RECT_BUDGET_LANES : (double)e->rect_budget;
+    const double room = (double)lane_slot_bytes(e, (long long)(4.0 * e->sms * 32 * max_area));
+    auto share = [&](int width) {
+        const double want = 4.0 * e->sms * 4.0 * width * lane_warps_per_block() * max_band;
+        return 8 * cells <= keep ? 1.0 : std::min(1.0, room / std::max(want, 1.0));
+    };
     warp += longest / 8;
-    const double l32 = std::max(cells / 250 + 1.38 * longest, cells / 120);
-    const double l64 = std::max(cells / 530 + 2 * longest, cells / 150);
+    const double l32 = std::max(cells / 250 + 1.38 * longest, cells / 120 / share(32));
+    const double l64 = std::max(cells / 530 + 2 * longest, cells / 150 / share(64));
     return warp <= std::min(l32, l64) ? 0 : l32 <= l64 ? 32 : 64;
 }
 
@@ -943,6 +970,20 @@ lcg_status mod_top_levels(const lcg_align_opts *opts, Chunk &c, const PairDev *d
     c.ratio.assign(lambda.begin(), lambda.end());
     sel->flags = TRACE_KEEP_MIN;
     return LCG_OK;
+}
+
+lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all, const lcg_align_opts *opts,
+                        Chunk &c, double *pack_ms);
+
+// chunk_launch with the chunk prepared again for one warp per group
+lcg_status without_lanes(lcg_engine e, const Slot &s, const lcg_pair_tables *all, const lcg_align_opts *opts,
+                         Chunk &c, double *pack_ms) {
+    const lcg_pair_tables *const pairs = all + c.q0;
+    const bool dev = lcg_host::index_on_device(pairs, c.nq);
+    c.prep.assign(c.nq, Prep());
+    lcg_host::parallel_for(c.nq, [&](int q) { prep_pair(pairs[q], *opts, c.prep[q], 0, dev); });
+    c.no_keep = false;
+    return chunk_launch(e, s, all, opts, c, pack_ms);
 }
 
 // Lay out, pack and enqueue one prepared chunk on its buffer set: one
@@ -1344,11 +1385,16 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         CUDA_TRY(lane_occupancy(lgroups, rb, lfast, &blocks_per_sm));
         if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
         if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
-        // no more blocks than items, and at most LANE_SCRATCH_BYTES of slots
+        // no more blocks than items, and a bounded amount of slots: a caller's
+        // budget holds for them too, but for what the other fill would take
+        int bps = 0;
+        CUDA_TRY(fill_occupancy(rb, false, lfast, false, &bps));
+        const long long limit = lane_slot_bytes(e, 4ll * e->sms * bps * fill_warps_per_block() * stride);
         const long long block_ints = lane_warps_per_block() * (lslot + lqslot);
-        long long b = std::min<long long>((long long)e->sms * blocks_per_sm,
-                                          ((long long)nitems[1] + lane_warps_per_block() - 1) / lane_warps_per_block());
-        lblocks = (int)std::max<long long>(1, std::min<long long>(b, LANE_SCRATCH_BYTES / 4 / block_ints));
+        const long long want = std::min<long long>((long long)e->sms * blocks_per_sm,
+                                                   ((long long)nitems[1] + lane_warps_per_block() - 1) / lane_warps_per_block());
+        lblocks = (int)std::min<long long>(want, limit / 4 / block_ints);
+        if (few_blocks(lblocks, want)) return without_lanes(e, s, all, opts, c, pack_ms);
         lane_ints = (size_t)lblocks * (size_t)block_ints;
     }
     size_t trace_slots = (size_t)npairs * (sl ? 8 : 1);

@@ -39,7 +39,7 @@ lcg_status pf_fail(lcg_status c, const std::string &m) {
         if (_e != cudaSuccess) return pf_fail(LCG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
     } while (0)
 
-// at most this much scratch for the slots of a lane-per-group launch
+// scratch for the slots of a lane-per-group launch, unless the caller sets a budget
 constexpr long long PF_LANE_SCRATCH_BYTES = 24ll << 30;
 
 size_t up16(size_t x) { return (x + 15) / 16 * 16; }
@@ -129,6 +129,13 @@ double seq_log_pf(const lcg_pair_tables &t, const std::vector<double> &bm, const
     return logscale + std::log(std::max(Mp[m], 1e-300));
 }
 
+// Bytes of slots that a lane-per-group launch may have: a bounded amount, or the
+// caller's budget (lcg_engine_set_rect_budget), but at least what those of one warp
+// per group take (other).
+long long pf_lane_slot_bytes(lcg_engine e, long long other) {
+    return std::max(e->rect_budget < 0 ? PF_LANE_SCRATCH_BYTES : e->rect_budget, other);
+}
+
 // Whether an FP32 batch is swept lane per group (pf_lane_kernels.cu). An
 // estimate of both times from the pairs' sizes, with lane_width's measures (cells
 // and the longest item's time, engine.cu); the constants are fits to forward and
@@ -156,12 +163,12 @@ bool pf_lanes(const lcg_pair_tables *pairs, int npairs, const lcg_pf_opts *o) {
 
 template <typename T>
 lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, int npairs, const lcg_pf_opts *o,
-                        const lcg_pf_grad_spec *specs, double *log_z) {
+                        const lcg_pf_grad_spec *specs, double *log_z, bool allow_lanes = true) {
     const double temp = o->temperature > 0 ? o->temperature : 300.0;
     const double pf_scale = o->pf_scale > 0 ? o->pf_scale : 1.0;
     lcg_align_opts ao{0, 0, 0, 0};
     std::vector<lcg_host::Prep> prep(npairs);
-    bool lanes = sizeof(T) == 4 && pf_lanes(pairs, npairs, o);
+    bool lanes = allow_lanes && sizeof(T) == 4 && pf_lanes(pairs, npairs, o);
     const bool dev = lcg_host::index_on_device(pairs, npairs);
     lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], lanes ? 32 : 0, dev); });
     if (lanes) {
@@ -532,8 +539,15 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         s.warp = s.slot + s.back_slot + rows;
         s.block = (std::max(pf_warps_per_block() * s.warp, top) + 31) / 32 * 32;
         // no more blocks than items, and a bounded amount of scratch
-        const long long want = std::max<long long>(npairs, (long long)(nitems + pf_warps_per_block() - 1) / pf_warps_per_block());
-        s.blocks = (int)std::max(1ll, std::min({(long long)e->sms * bf, want, PF_LANE_SCRATCH_BYTES / 4 / s.block}));
+        const long long want =
+            std::min((long long)e->sms * bf,
+                     std::max<long long>(npairs, (long long)(nitems + pf_warps_per_block() - 1) / pf_warps_per_block()));
+        PF_TRY(pf_back_occupancy<T>(rb, &bb));
+        const long long limit = pf_lane_slot_bytes(e, 4ll * e->sms * bb * pf_warps_per_block() * stride * sizeof(T));
+        s.blocks = (int)std::min(want, limit / 4 / s.block);
+        // with few blocks one warp per group takes no longer (6 pairs of 700-800 nt, 608
+        // wanted: 1070 ms with 563, 1480 with 314, one warp per group 1495)
+        if (2 * s.blocks < want) return pf_forward_t<T>(e, S, pairs, npairs, o, specs, log_z, false);
         need = (size_t)s.blocks * (size_t)s.block * sizeof(T);
     } else {
         PF_TRY(pf_fwd_occupancy<T>(rb, &bf));

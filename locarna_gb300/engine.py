@@ -275,7 +275,8 @@ class Engine:
         """lcg_engine_set_rect_budget: bytes of kept group rectangles per
         chunk (0: the traceback always recomputes; negative: the defaults,
         4 GiB for plain chunks, 16 GiB for lane-per-group batches and 32 GiB
-        for structure-local chunks)."""
+        for structure-local chunks). It bounds the scratch of lane-per-group
+        batches as well (by default 24 GiB per chunk in flight)."""
         _check(self.lib, self.lib.lcg_engine_set_rect_budget(self.h, int(nbytes)))
 
     def set_autotune(self, on):
