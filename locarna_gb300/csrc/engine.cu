@@ -769,6 +769,7 @@ struct Slot {
     size_t *stage_cap;
     int **d_scratch;
     size_t *scratch_cap;
+    lcg_denied *denied;
     cudaEvent_t ev0, ev1, ev2;
     lcg_graph_cache *graph;
 };
@@ -776,10 +777,10 @@ struct Slot {
 Slot slot_of(lcg_engine e, int k) {
     if (k == 0)
         return Slot{e->stream, &e->d_arena, &e->arena_cap, &e->h_stage, &e->stage_cap,
-                    &e->d_scratch, &e->scratch_cap, e->ev0, e->ev1, e->ev2, &e->graph};
+                    &e->d_scratch, &e->scratch_cap, &e->denied, e->ev0, e->ev1, e->ev2, &e->graph};
     lcg_buffer_set &b = e->alt;
     return Slot{b.stream, &b.d_arena, &b.arena_cap, &b.h_stage, &b.stage_cap,
-                &b.d_scratch, &b.scratch_cap, b.ev0, b.ev1, b.ev2, &b.graph};
+                &b.d_scratch, &b.scratch_cap, &b.denied, b.ev0, b.ev1, b.ev2, &b.graph};
 }
 
 // byte offsets of one pair's tables in the arena
@@ -1024,7 +1025,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             if ((ln ? p.lane_lines : p.rect_cells) < 0 || (p.flags & PF_NOLP)) keep = false;
             bytes += ln ? 4.0 * p.lane_groups * (double)p.lane_lines : (double)rect_bytes_per_cell * (double)p.rect_cells;
         }
-        keep = keep && bytes <= (double)budget;
+        keep = keep && bytes <= (double)budget && bytes < (double)s.denied->arena;
     }
     c.off.assign(npairs, PairOff{});
     std::vector<PairOff> &off = c.off;
@@ -1151,19 +1152,21 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     // the set's graph addresses its arena, staging and scratch: it goes
     // before any of them is freed
     if (total > *s.arena_cap) {
-        s.graph->release();
-        if (*s.d_arena) cudaFree(*s.d_arena);
-        *s.d_arena = nullptr;
-        *s.arena_cap = 0;
-        const size_t cap = total + std::min<size_t>(total / 4, (size_t)1 << 30);
-        if (cudaMalloc(s.d_arena, cap) != cudaSuccess) {
-            cudaGetLastError();
+        if (!keep || total < s.denied->arena) {
+            s.graph->release();
+            if (*s.d_arena) cudaFree(*s.d_arena);
             *s.d_arena = nullptr;
+            *s.arena_cap = 0;
+            // with room to grow, else without
+            for (size_t cap : {total + std::min<size_t>(total / 4, (size_t)1 << 30), total})
+                if (!*s.arena_cap && lcg_host::device_alloc(s.d_arena, cap) == cudaSuccess) *s.arena_cap = cap;
+        }
+        if (total > *s.arena_cap) {
             if (!keep) return fail(LCG_ERR_NOMEM, "device arena allocation failed");
+            s.denied->arena = std::min(s.denied->arena, total);
             c.no_keep = true;  // without the kept rectangles
             return chunk_launch(e, s, all, opts, c, pack_ms);
         }
-        *s.arena_cap = cap;
     }
     if (down_end > *s.stage_cap) {
         s.graph->release();
@@ -1354,7 +1357,8 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     int blocks = 0, lblocks = 0;
     size_t group_ints = 0, lane_ints = 0;  // scratch of the fill launches
     int lgroups = 0;
-    long long lslot = 0, lqslot = 0;
+    long long lslot = 0, lqslot = 0, lwant = 0;
+    size_t other_ints = 0;  // what the fill with one warp per group would take for the lane pairs
     if (!sl) CUDA_TRY(trace_prepare(rb));
     if (!of[0].empty()) {
         int blocks_per_sm = 0;
@@ -1389,30 +1393,37 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         // budget holds for them too, but for what the other fill would take
         int bps = 0;
         CUDA_TRY(fill_occupancy(rb, false, lfast, false, &bps));
-        const long long limit = lane_slot_bytes(e, 4ll * e->sms * bps * fill_warps_per_block() * stride);
+        other_ints = (size_t)e->sms * bps * fill_warps_per_block() * (size_t)stride;
+        const long long limit = lane_slot_bytes(e, 4ll * (long long)other_ints);
         const long long block_ints = lane_warps_per_block() * (lslot + lqslot);
-        const long long want = std::min<long long>((long long)e->sms * blocks_per_sm,
-                                                   ((long long)nitems[1] + lane_warps_per_block() - 1) / lane_warps_per_block());
-        lblocks = (int)std::min<long long>(want, limit / 4 / block_ints);
-        if (few_blocks(lblocks, want)) return without_lanes(e, s, all, opts, c, pack_ms);
+        lwant = std::min<long long>((long long)e->sms * blocks_per_sm,
+                                    ((long long)nitems[1] + lane_warps_per_block() - 1) / lane_warps_per_block());
+        lblocks = (int)std::min<long long>(lwant, limit / 4 / block_ints);
+        if (few_blocks(lblocks, lwant)) return without_lanes(e, s, all, opts, c, pack_ms);
         lane_ints = (size_t)lblocks * (size_t)block_ints;
     }
     size_t trace_slots = (size_t)npairs * (sl ? 8 : 1);
     auto scratch_need = [&]() { return std::max({group_ints, lane_ints, trace_slots * (size_t)stride}); };
-    if (scratch_need() > *s.scratch_cap) {
+    // With little memory left a lane launch takes fewer blocks, or, where those are
+    // few and there is room for the other fill's scratch, one warp per group.
+    auto grow_scratch = [&](size_t ints) {
         s.graph->release();
         if (*s.d_scratch) cudaFree(*s.d_scratch);
-        *s.d_scratch = nullptr;
         *s.scratch_cap = 0;
-        // with little memory left, a lane launch takes fewer warps
-        while (cudaMalloc(s.d_scratch, scratch_need() * sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            *s.d_scratch = nullptr;
-            if (lblocks <= 1) return fail(LCG_ERR_NOMEM, "device scratch allocation failed");
-            lblocks /= 2;
-            lane_ints /= 2;
-        }
-        *s.scratch_cap = scratch_need();
+        if (lcg_host::device_alloc(s.d_scratch, ints * sizeof(int)) == cudaSuccess) *s.scratch_cap = ints;
+        else s.denied->scratch = std::min(s.denied->scratch, ints * sizeof(int));
+        return *s.scratch_cap > 0;
+    };
+    while (scratch_need() > *s.scratch_cap) {
+        if (lblocks <= 1 || 4 * scratch_need() < s.denied->scratch)
+            if (grow_scratch(scratch_need())) break;
+        if (lblocks <= 1) return fail(LCG_ERR_NOMEM, "device scratch allocation failed");
+        lane_ints = lane_ints / lblocks * (lblocks / 2);
+        lblocks /= 2;
+        if (!few_blocks(lblocks, lwant)) continue;
+        const size_t other = std::max(other_ints, trace_slots * (size_t)stride);
+        if (other <= *s.scratch_cap || (4 * other < s.denied->scratch && grow_scratch(other)))
+            return without_lanes(e, s, all, opts, c, pack_ms);
     }
     int *scratch = *s.d_scratch;
 
@@ -1935,6 +1946,8 @@ lcg_status lcg_align_pp_pairs(lcg_engine e, const char *const *pp_a, const char 
 lcg_status lcg_engine_set_rect_budget(lcg_engine e, int64_t bytes) {
     if (!e) return fail(LCG_ERR_ARG, "null engine");
     e->rect_budget = bytes < 0 ? -1 : bytes;
+    e->denied = e->alt.denied = lcg_denied();
+    lcg_host::pf_forget_denied(e);
     return LCG_OK;
 }
 

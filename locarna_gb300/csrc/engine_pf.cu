@@ -63,6 +63,7 @@ struct PFState {
     size_t hcap = 0;
     char *d_scratch = nullptr;
     size_t scratch_cap = 0;
+    lcg_denied denied;
     std::vector<PFLayout> lay;
     size_t off_pairs = 0, off_queue = 0, off_queue_back = 0, off_ctrl = 0, off_am = 0, out_begin = 0, out_end = 0, total = 0;
     size_t nitems = 0;
@@ -333,21 +334,20 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         }
     }
     size_t total = up;
+    if (keep && total > S->cap && total >= S->denied.arena) {
+        keep = false;
+        total = bare;
+    }
     if (total > S->cap) {
         if (S->d_arena) cudaFree(S->d_arena);
         S->d_arena = nullptr;
         S->cap = 0;
         // with room to grow, else without, else without the kept rectangles
-        for (size_t bytes : {total + std::min<size_t>(total / 4, (size_t)1 << 30), total, bare}) {
-            if (cudaMalloc(&S->d_arena, bytes) == cudaSuccess) {
-                S->cap = bytes;
-                break;
-            }
-            cudaGetLastError();
-            S->d_arena = nullptr;
-        }
-        if (!S->d_arena) return pf_fail(LCG_ERR_NOMEM, "PF device arena allocation failed");
+        for (size_t bytes : {total + std::min<size_t>(total / 4, (size_t)1 << 30), total, bare})
+            if (!S->cap && lcg_host::device_alloc(&S->d_arena, bytes) == cudaSuccess) S->cap = bytes;
+        if (!S->cap) return pf_fail(LCG_ERR_NOMEM, "PF device arena allocation failed");
         if (S->cap < total) {
+            S->denied.arena = std::min(S->denied.arena, total);
             keep = false;
             total = bare;
         }
@@ -523,7 +523,8 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     int bf = 0, bb = 0;
     const int rb = lcg_host::ring_size(span);
     const long long stride = (long long)rows_max * sw;
-    size_t need;
+    size_t need, other = 0;  // other: what one warp per group would take for a lane batch
+    long long want = 0;
     if (lanes) {
         PF_TRY(pf_lane_occupancy(rb, &bf));
         if (bf < 1) return pf_fail(LCG_ERR_UNSUPPORTED, "PF kernels do not fit on an SM");
@@ -539,11 +540,11 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         s.warp = s.slot + s.back_slot + rows;
         s.block = (std::max(pf_warps_per_block() * s.warp, top) + 31) / 32 * 32;
         // no more blocks than items, and a bounded amount of scratch
-        const long long want =
-            std::min((long long)e->sms * bf,
-                     std::max<long long>(npairs, (long long)(nitems + pf_warps_per_block() - 1) / pf_warps_per_block()));
+        want = std::min((long long)e->sms * bf,
+                        std::max<long long>(npairs, (long long)(nitems + pf_warps_per_block() - 1) / pf_warps_per_block()));
         PF_TRY(pf_back_occupancy<T>(rb, &bb));
-        const long long limit = pf_lane_slot_bytes(e, 4ll * e->sms * bb * pf_warps_per_block() * stride * sizeof(T));
+        other = (size_t)e->sms * bb * pf_warps_per_block() * 4 * (size_t)stride * sizeof(T);
+        const long long limit = pf_lane_slot_bytes(e, (long long)other);
         s.blocks = (int)std::min(want, limit / 4 / s.block);
         // with few blocks one warp per group takes no longer (6 pairs of 700-800 nt, 608
         // wanted: 1070 ms with 563, 1480 with 314, one warp per group 1495)
@@ -557,19 +558,26 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
         const size_t back_slots = (size_t)e->sms * bb * pf_warps_per_block() * 4;
         need = std::max(fwd_slots, back_slots) * (size_t)stride * sizeof(T);
     }
-    if (need > S->scratch_cap) {
+    // with little memory left a lane launch takes fewer blocks, or, where those are few
+    // and there is room for the scratch of the other, one warp per group
+    auto grow_scratch = [&](size_t bytes) {
         if (S->d_scratch) cudaFree(S->d_scratch);
-        S->d_scratch = nullptr;
         S->scratch_cap = 0;
-        // with little memory left, a lane launch takes fewer blocks
-        while (cudaMalloc(&S->d_scratch, need) != cudaSuccess) {
-            cudaGetLastError();
-            S->d_scratch = nullptr;
-            if (!lanes || S->lane_scratch.blocks <= 1) return pf_fail(LCG_ERR_NOMEM, "PF scratch allocation failed");
-            S->lane_scratch.blocks /= 2;
-            need = (size_t)S->lane_scratch.blocks * (size_t)S->lane_scratch.block * sizeof(T);
-        }
-        S->scratch_cap = need;
+        if (lcg_host::device_alloc(&S->d_scratch, bytes) == cudaSuccess) S->scratch_cap = bytes;
+        else S->denied.scratch = std::min(S->denied.scratch, bytes);
+        return S->scratch_cap > 0;
+    };
+    int fixed = 1;  // (no lanes: nothing to make smaller)
+    int &blocks = lanes ? S->lane_scratch.blocks : fixed;
+    while (need > S->scratch_cap) {
+        if (blocks <= 1 || need < S->denied.scratch)
+            if (grow_scratch(need)) break;
+        if (blocks <= 1) return pf_fail(LCG_ERR_NOMEM, "PF scratch allocation failed");
+        blocks /= 2;
+        need = (size_t)blocks * (size_t)S->lane_scratch.block * sizeof(T);
+        if (2 * blocks >= want) continue;
+        if (other <= S->scratch_cap || (other < S->denied.scratch && grow_scratch(other)))
+            return pf_forward_t<T>(e, S, pairs, npairs, o, specs, log_z, false);
     }
     S->lane_scratch.base = S->d_scratch;
     cudaStream_t st = e->stream;
@@ -753,6 +761,10 @@ void pf_release(lcg_engine_s *e) {
     if (S->d_scratch) cudaFree(S->d_scratch);
     delete S;
     e->pf = nullptr;
+}
+
+void pf_forget_denied(lcg_engine e) {
+    if (e->pf) ((PFState *)e->pf)->denied = lcg_denied();
 }
 }  // namespace lcg_host
 

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <cstddef>
+#include <cstdint>
+#include <cstdio>
 #include <cstdlib>
 #include <vector>
 
@@ -26,6 +28,14 @@ struct lcg_graph_cache {
     }
 };
 
+// The smallest sizes (bytes) of a buffer set's arena and scratch that the device
+// had no memory for: where a call has a smaller form (nothing kept, fewer blocks),
+// it takes that at once from then on, until the caller sets the budget again
+// (lcg_engine_set_rect_budget).
+struct lcg_denied {
+    size_t arena = SIZE_MAX, scratch = SIZE_MAX;
+};
+
 // Device arena, pinned staging, fill scratch, stream and events of one
 // in-flight chunk of an lcg_align_pairs call. The engine's own fields are
 // the first set; `alt` is the second one of the double-buffered pipeline.
@@ -38,6 +48,7 @@ struct lcg_buffer_set {
     size_t stage_cap = 0;
     int *d_scratch = nullptr;
     size_t scratch_cap = 0;  // ints
+    lcg_denied denied;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     lcg_graph_cache graph;
 };
@@ -61,6 +72,7 @@ struct lcg_engine_s {
     size_t stage_cap = 0;
     int *d_scratch = nullptr;
     size_t scratch_cap = 0;  // ints
+    lcg_denied denied;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     double last_ms = 0, last_fill_ms = 0, last_trace_ms = 0;
     long long last_launches = 0;
@@ -106,13 +118,17 @@ struct lcg_engine_s {
 
 namespace lcg_host {
 // cudaMalloc that leaves *p null and the runtime's last error clear on failure.
-// A test build (LCG_TEST_ALLOC) refuses what is larger than $LCG_TEST_ALLOC_BYTES.
+// A test build (LCG_TEST_ALLOC) refuses what is larger than $LCG_TEST_ALLOC_BYTES and
+// says so on stderr.
 template <typename T>
 cudaError_t device_alloc(T **p, size_t bytes) {
     cudaError_t e = cudaSuccess;
 #ifdef LCG_TEST_ALLOC
     if (const char *v = std::getenv("LCG_TEST_ALLOC_BYTES"))
-        if (bytes > (size_t)std::atoll(v)) e = cudaErrorMemoryAllocation;
+        if (bytes > (size_t)std::atoll(v)) {
+            e = cudaErrorMemoryAllocation;
+            std::fprintf(stderr, "refused %zu\n", bytes);
+        }
 #endif
     if (e == cudaSuccess) e = cudaMalloc(p, bytes);
     if (e != cudaSuccess) {
@@ -123,4 +139,5 @@ cudaError_t device_alloc(T **p, size_t bytes) {
 }
 
 void pf_release(lcg_engine_s *e);
+void pf_forget_denied(lcg_engine_s *e);  // lcg_denied of the partition-function state
 }

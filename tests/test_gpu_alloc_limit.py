@@ -47,6 +47,7 @@ def child():
         r = subprocess.run([sys.executable, "-c", head + textwrap.dedent(code)], capture_output=True, text=True,
                            timeout=300)
         assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
+        return r.stderr  # one line "refused <bytes>" per refused allocation
     return run
 
 
@@ -68,3 +69,54 @@ def test_envelopes_in_smaller_waves(child):
                 assert t.envelope_ok == r.envelope_ok
         print("ok")
     """)
+
+
+# ten pairs with whole bands: the items' storage (1.8 GB) and the slots of all warps
+# (6.0 GB) are refused at every limit; one warp per group takes 0.5 GB of scratch, so
+# the batch goes there at 900 MB and to a few blocks of lanes below. The second call
+# makes no attempt that has failed before, setting the budget forgets them.
+@pytest.mark.gpu
+@pytest.mark.parametrize("lanes", [32, 64])
+@pytest.mark.parametrize("megabytes", [900, 300, 150])
+def test_lane_fill_with_less_memory(child, lanes, megabytes):
+    err = child(f"""
+        os.environ["LCG_LANES"] = "{lanes}"
+        tabs, _ = prepare_pairs(Engine(0), pairs, min_trace_probability=0.0)
+        ref = [(r.score, r.edges) for r in Engine(0).align_pairs(tabs)]
+        eng = Engine(0)
+        limit({megabytes} << 20)
+        for k in range(2):
+            assert [(r.score, r.edges) for r in eng.align_pairs(tabs)] == ref
+            print("call", k, file=sys.stderr, flush=True)
+        eng.set_rect_budget(-1)
+        assert [(r.score, r.edges) for r in eng.align_pairs(tabs)] == ref
+        print("ok")
+    """)
+    first, second, third = err.split("call")
+    assert "refused" in first and "refused" not in second and "refused" in third, err
+
+
+# (one warp per group takes 2.2 GB here: 3000 MB goes there)
+@pytest.mark.gpu
+@pytest.mark.parametrize("megabytes", [3000, 900, 300, 150])
+def test_pf_lanes_with_less_memory(child, megabytes):
+    err = child(f"""
+        os.environ["LCG_LANES"] = "32"
+        kw = dict(precision=32, min_am_prob=0.0, gap_gradients=False)
+        tabs, _ = prepare_pairs(Engine(0), pairs, min_trace_probability=0.0, pf_precision=0)
+        ref = Engine(0)
+        lz = ref.pf_forward(tabs, **kw)
+        probs = ref.pf_backward()
+        eng = Engine(0)
+        limit({megabytes} << 20)
+        for k in range(2):
+            got = eng.pf_forward(tabs, **kw)
+            assert np.max(np.abs(np.array(got) - np.array(lz)) / np.maximum(1.0, np.abs(lz))) <= 1e-5
+            for r, p in zip(eng.pf_backward(), probs):
+                assert np.max(np.abs(r["am_prob"] - p["am_prob"]), initial=0.0) <= 1e-5
+                assert np.max(np.abs(r["bm_prob"] - p["bm_prob"])) <= 1e-5
+            print("call", k, file=sys.stderr, flush=True)
+        print("ok")
+    """)
+    first, second, _ = err.split("call")
+    assert "refused" in first and "refused" not in second, err
