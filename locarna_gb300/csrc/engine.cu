@@ -165,10 +165,16 @@ static bool scan_arc_matches(const lcg_pair_tables &t, Prep &p, std::vector<int>
     return true;
 }
 
-// Limits of the lane-per-group fill: the shared-memory rows of its top-level
-// items (span), and 80 MB of matrix storage per warp
-constexpr int LANE_MAX_SPAN = 640;
-constexpr int LANE_MAX_BANDCELLS = 600000;
+bool lane_pair(const lcg_pair_tables &t, long long *band) {
+    if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || t.len_b < 1 || !t.min_col || !t.max_col) return false;
+    long long cells = 0, span = 2;
+    for (int i = 0; i <= t.len_a; ++i) {
+        cells += (long long)t.max_col[i] - t.min_col[i] + 1;
+        if (i < t.len_a) span = std::max(span, (long long)t.max_col[i + 1] - t.min_col[i] + 3);
+    }
+    if (band) *band = cells;
+    return span <= LANE_MAX_SPAN && cells <= LANE_MAX_BANDCELLS;
+}
 
 lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes,
                      bool device_index) {
@@ -361,8 +367,7 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
             }
         }
     }
-    if (o.struct_local || anchors || t.indel_opening > 0 || p.span > LANE_MAX_SPAN || p.bandcells > LANE_MAX_BANDCELLS)
-        lanes = 0;
+    if (o.struct_local || !lane_pair(t)) lanes = 0;
     p.lane_groups = lanes;
     int entries = 0;
     if (lanes) {
@@ -852,10 +857,8 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
     double cells = 0, warp = 0, longest = 0, max_band = 0, max_area = 0;
     for (int q = 0; q < npairs; ++q) {
         const lcg_pair_tables &t = pairs[q];
-        if (t.match_lo || t.indel_opening > 0 || t.len_a < 1 || t.len_b < 1 || !t.sigma || !t.min_col || !t.max_col)
-            continue;
-        double band = 0;
-        for (int i = 0; i <= t.len_a; ++i) band += t.max_col[i] - t.min_col[i] + 1;
+        long long band;
+        if (!t.sigma || !lcg_host::lane_pair(t, &band)) continue;  // (one warp per group in any case)
         // dense scores: more than 16 values in a row (single sequences: 4)
         const int *const row = t.sigma + (size_t)((t.len_a + 1) / 2) * (t.len_b + 1);
         int value[16], nv = 0;
@@ -868,8 +871,8 @@ int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg
         const double c = 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
         cells += c;
         warp += c / (nv > 16 ? 58 : t.am_stack_score ? 70 : 80);
-        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
-        max_band = std::max(max_band, band);
+        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + (double)band) / 32 + 50.0 * t.num_arcmatches);
+        max_band = std::max(max_band, (double)band);
         max_area = std::max(max_area, (t.len_a + 1.0) * (t.len_b + 2.0));
     }
     // The share of the wanted blocks that the slots have room for (a line of `width`

@@ -149,16 +149,15 @@ long long pf_lane_slot_bytes(lcg_engine e, long long other) {
 // 65 and 21 of 80-500 nt 72 instead of 152.
 bool pf_lanes(const lcg_pair_tables *pairs, int npairs, const lcg_pf_opts *o) {
     if (o->gap_gradients) return false;  // the adjoint of the gap weights reads E and F
-    if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) >= 32;
     double cells = 0, longest = 0;
     for (int q = 0; q < npairs; ++q) {
         const lcg_pair_tables &t = pairs[q];
-        if (t.len_a < 1 || !t.min_col || !t.max_col) return false;
-        double band = 0;
-        for (int i = 0; i <= t.len_a; ++i) band += t.max_col[i] - t.min_col[i] + 1;
+        long long band;
+        if (!lcg_host::lane_pair(t, &band)) return false;  // all pairs or none
         cells += 2.0 * t.num_arcmatches * (t.len_a + t.len_b);
-        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + band) / 32 + 50.0 * t.num_arcmatches);
+        longest = std::max(longest, 2.2e3 * (8.0 * t.len_a + (double)band) / 32 + 50.0 * t.num_arcmatches);
     }
+    if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) >= 32;
     return cells / 10 + 0.5 * longest > cells / 50 + 4 * longest;
 }
 
@@ -172,16 +171,6 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     bool lanes = allow_lanes && sizeof(T) == 4 && pf_lanes(pairs, npairs, o);
     const bool dev = lcg_host::index_on_device(pairs, npairs);
     lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], lanes ? 32 : 0, dev); });
-    if (lanes) {
-        // all pairs or none: a pair whose band is too wide keeps the batch off it
-        bool all = true;
-        for (auto &p : prep) all = all && (p.code != LCG_OK || (p.flags & PF_LANES));
-        if (!all) {
-            lanes = false;
-            prep.assign(npairs, lcg_host::Prep());
-            lcg_host::parallel_for(npairs, [&](int q) { lcg_host::prep_pair(pairs[q], ao, prep[q], 0, dev); });
-        }
-    }
     S->lanes = lanes;
     bool need_spec = false;
     for (int k = 2; k < 19; ++k) need_spec |= o->param_delta[k] != 0.0;

@@ -82,6 +82,15 @@ struct Prep {
 lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p, int lanes = 0,
                      bool device_index = false);
 
+// Whether the lane-per-group fill takes a pair (not under struct_local): no anchors,
+// no positive gap opening, the shared-memory rows of its top level (span) and the
+// lines of one item (band cells: 77 MB of a warp's storage at 32 groups an item, 154
+// at 64) bounded. Asked of tables before prep_pair has checked them; false where it
+// cannot tell. *band: the band cells.
+constexpr int LANE_MAX_SPAN = 640;
+constexpr int LANE_MAX_BANDCELLS = 600000;
+bool lane_pair(const lcg_pair_tables &t, long long *band = nullptr);
+
 // whether prep_pair should leave that to the device, for these pairs
 bool index_on_device(const lcg_pair_tables *pairs, int npairs);
 
