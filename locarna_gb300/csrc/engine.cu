@@ -1359,7 +1359,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
     long long stride = (long long)rows_max * sw;
     int blocks = 0, lblocks = 0;
     size_t group_ints = 0, lane_ints = 0;  // scratch of the fill launches
-    int lgroups = 0;
+    int lgroups = 0, lrb = 0;
     long long lslot = 0, lqslot = 0, lwant = 0;
     size_t other_ints = 0;  // what the fill with one warp per group would take for the lane pairs
     if (!sl) CUDA_TRY(trace_prepare(rb));
@@ -1381,15 +1381,20 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         group_ints = (size_t)blocks * (sl ? sl_fill_warps_per_block() * 4 : fill_warps_per_block()) * (size_t)stride;
     }
     if (!of[1].empty()) {
-        int blocks_per_sm = 0, rows = 0;
+        int blocks_per_sm = 0, rows = 0, lspan = 2;
         lgroups = prep[of[1][0]].lane_groups;  // one width per chunk
         for (int q : of[1]) {
+            lspan = std::max(lspan, prep[q].span);
             lslot = std::max(lslot, lgroups * prep[q].lane_slot);
             rows = std::max(rows, prep[q].n + 1);
         }
         if (keep) lslot = 0;
         lqslot = (long long)lgroups * (rows + 3);
-        CUDA_TRY(lane_occupancy(lgroups, rb, lfast, &blocks_per_sm));
+        // rings for these pairs alone: the span of a wide pair beside them would take the
+        // shared memory of three of an SM's four blocks (66 pairs of 150-260 nt and one
+        // of 12 x 1300: fill 17.6 -> 13.9 ms)
+        lrb = lcg_host::ring_size(lspan);
+        CUDA_TRY(lane_occupancy(lgroups, lrb, lfast, &blocks_per_sm));
         if (blocks_per_sm < 1) return fail(LCG_ERR_UNSUPPORTED, "fill kernel does not fit on an SM");
         if (c.bps > 0 && c.bps < blocks_per_sm) blocks_per_sm = c.bps;
         // no more blocks than items, and a bounded amount of slots: a caller's
@@ -1444,7 +1449,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
         key = {(long long)(uintptr_t)Dv, (long long)(uintptr_t)H, (long long)(uintptr_t)scratch, (long long)down_begin,
                (long long)down_end, (long long)off_ctrl, (long long)off_pairs, (long long)off_queue, (long long)nitems[0],
                blocks, sw, rb, stride, fast, ahead, e->counting, sl, sl_fast, keep, opts->do_trace, npairs,
-               (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lfast, lgroups,
+               (long long)off_lqueue, (long long)nitems[1], lblocks, lslot, lqslot, lrb, lfast, lgroups,
                (long long)off_index, index_n, index_lefts};
         if (s.graph->exec && s.graph->key == key) {
             CUDA_TRY(cudaGraphLaunch(s.graph->exec, st));
@@ -1490,7 +1495,7 @@ lcg_status chunk_launch(lcg_engine e, const Slot &s, const lcg_pair_tables *all,
             CUDA_TRY(launch_index(d_pairs, (const IndexPair *)(Dv + off_index), npairs, index_n, index_lefts, st));
         if (!of[1].empty()) {
             CUDA_TRY(launch_lane_fill(lgroups, d_pairs, (const int2 *)(Dv + off_lqueue), (int)nitems[1], scratch,
-                                      lslot, lqslot, rb, lfast, (unsigned int *)(Dv + off_ctrl + 32), status,
+                                      lslot, lqslot, lrb, lfast, (unsigned int *)(Dv + off_ctrl + 32), status,
                                       abort_flag, lblocks, st));
             ++c.launches;
         }
