@@ -23,7 +23,7 @@
 // row. An item waits only for items that come before it.
 //
 // Sums over lanes are taken by one lane per cell or entry over its 32 words in
-// shared memory, with the rounding errors carried along (two-sum), so that they
+// shared memory, with the rounding errors carried along (pfl_row_sum), so that they
 // are as good as the FP64 atomics over single groups they replace; they end in
 // FP64 atomics, 32 times fewer.
 //
@@ -121,17 +121,19 @@ __device__ __forceinline__ void pfl_load8(int at, float (&v)[8]) {
     }
 }
 
-// s += x, the rounding error added to err
-__device__ __forceinline__ void pfl_two_sum(float &s, float &err, float x) {
-    const float y = s + x, z = y - s;
-    err += (s - (y - z)) + (x - z);
+// s += x; returns the rounding error (Knuth's two-sum)
+__device__ __forceinline__ float pfl_two_sum(float &s, float x) {
+    const float y = s + x, z = y - s, err = (s - (y - z)) + (x - z);
     s = y;
+    return err;
 }
 
-// the sum of the 32 words of row `row` of PFL_SUMS, in one thread
+// the sum of the 32 words of row `row` of PFL_SUMS, in one thread: the rounding
+// errors are summed the same way and theirs too (SumK with K = 3; Ogita, Rump, Oishi
+// 2005), which is below FP64's rounding
 __device__ __noinline__ double pfl_row_sum(int sb, int row) {
     const int at = sb + PFL_SUMS + 32 * row;
-    float s0 = 0.f, s1 = 0.f, e0 = 0.f, e1 = 0.f;
+    float s0 = 0.f, s1 = 0.f, e0 = 0.f, e1 = 0.f, c0 = 0.f, c1 = 0.f;
 #pragma unroll
     for (int h = 0; h < 32; h += 16) {
         float x[16];
@@ -139,11 +141,11 @@ __device__ __noinline__ double pfl_row_sum(int sb, int row) {
         for (int t = 0; t < 16; ++t) x[t] = pfl_f(at + ((row + h + t) & 31));  // (lanes on different banks)
 #pragma unroll
         for (int t = 0; t < 16; t += 2) {
-            pfl_two_sum(s0, e0, x[t]);
-            pfl_two_sum(s1, e1, x[t + 1]);
+            c0 += pfl_two_sum(e0, pfl_two_sum(s0, x[t]));
+            c1 += pfl_two_sum(e1, pfl_two_sum(s1, x[t + 1]));
         }
     }
-    return ((double)s0 + (double)s1) + ((double)e0 + (double)e1);
+    return ((double)s0 + (double)s1) + (((double)e0 + (double)e1) + ((double)c0 + (double)c1));
 }
 
 // ---------------------------------------------------------------- forward
