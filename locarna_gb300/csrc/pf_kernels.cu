@@ -384,7 +384,7 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
         const T gAi = P.gA[i];
         const T gAn = (i + 1 < ar) ? P.gA[i + 1] : T(0);
         const T gAo = gAi * o, gAno = gAn * o;
-        T opnE = T(0);  // GRADS: the row's vertical gap openings without their weight
+        T opnE = T(0);  // GRADS in FP64: the row's vertical gap openings without their weight
         // seeds: dZ'/dD(am) w(am) into M(ar-1, br-1) once every use of D(am)
         // has been back-propagated
         while (dwp >= 0) {
@@ -500,8 +500,13 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
                 // gap derivatives: E(i,j) = gA(i) (E(i-1,j) + N(i-1,j) o)
                 if (GRADS) {
                     ext += (double)(Ebar * Ev + Fb * Fv);
-                    opnE += Ebar * (Mup - Eup);
-                    opn += (double)(Fb * (Ml - Fl) * (uni ? guo : g * o));
+                    const T down = Ebar * (Mup - Eup), right = Fb * (Ml - Fl) * (uni ? guo : g * o);
+                    if (sizeof(T) == 8) {
+                        opnE += down;
+                        opn += (double)right;
+                    } else {
+                        opn += (double)(down * gAo + right);
+                    }
                 }
                 // diagonal
                 const T Xd = Xbar * bmj;
@@ -517,7 +522,7 @@ __device__ void pf_group_back(const PFPair<T> &P, int al, int ar, int bl, int br
             }
             Fbc = __shfl_sync(0xffffffffu, Fb, 0);
         }
-        if (GRADS) opn += (double)opnE * gAo;
+        if (GRADS && sizeof(T) == 8) opn += (double)opnE * gAo;
         __syncwarp();
         // arc terms of row i: M_bar(corner) += X_bar D s', D_bar(am) += X_bar M(corner) s'
         // (two batches of 32 entries per step, loads issued together). The

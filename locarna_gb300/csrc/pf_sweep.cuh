@@ -327,7 +327,7 @@ __device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict
             mv = Mg[(size_t)(en.x & 0xffff) * pitch + (en.x >> 16)];
         }
         T Fbc = T(0);
-        T opnE = T(0);
+        T opnE = T(0);  // GRADS in FP64: the row's vertical gap openings without their weight
         for (int top = hi; top >= lo; top -= NT, bf ^= 1) {
             const int j = top - tid;
             const bool act = j >= lo;
@@ -353,8 +353,14 @@ __device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict
                 Xb[RG(j)] = Xbar;
                 if (GRADS) {
                     ext += (double)(Ebar * Eg[c] + Fb * Fg[c]);
-                    opnE += Ebar * (Mg[c - pitch] - Eg[c - pitch]);
-                    opn += (double)(Fb * (Mg[c - 1] - Fg[c - 1]) * (P.gB[j] * o));
+                    const T down = Ebar * (Mg[c - pitch] - Eg[c - pitch]);
+                    const T right = Fb * (Mg[c - 1] - Fg[c - 1]) * (P.gB[j] * o);
+                    if (sizeof(T) == 8) {
+                        opnE += down;
+                        opn += (double)right;
+                    } else {
+                        opn += (double)(down * gAo + right);
+                    }
                 }
                 const T Xd = Xbar * bmj;
                 if (j - 1 >= dlo && j - 1 <= dhi)
@@ -366,7 +372,7 @@ __device__ __noinline__ void pf_top_back(const PFPair<T> &P, const T *__restrict
                 if (j == lo) atomicAdd(Mb + c - 1, Fb * (P.gB[j] * o));
             }
         }
-        if (GRADS) opn += (double)opnE * gAo;
+        if (GRADS && sizeof(T) == 8) opn += (double)opnE * gAo;
         __syncthreads();
         for (int e = e0; e < ra.y; e += NT) {
             if (e != e0) {
