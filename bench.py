@@ -51,11 +51,11 @@ PF_BUCKET = 1024
 PF_FP64_STRIDE = 8  # FP64 (and the FP32 error) on every 8th pair of each launch
 PF_CPU_SECONDS = 20.0
 REF_PAIRS_PER_CORE = 4  # pairs per host core in one step of the reference arm
-# DRAM traffic of the fill kernel per M cell, from the ncu capture of the
-# 496-pair case (profiles/sankoff_fill_small_496pairs.md: dram read + write
-# bytes of one launch / the launch's cells); the traffic of a launch of the
-# workload is this times its cells
-FILL_DRAM_BYTES_PER_CELL = (1.598e9 + 3.921e9) / 1.2018e9
+# DRAM traffic per M cell of the kernel that fills the workload's chunks, the
+# lane-per-group fill with 64 groups an item: dram read + write bytes of one launch
+# over its cells (ncu capture of 66 pairs, profiles/sankoff_lane_66pairs.md). The
+# traffic of the workload is this times its cells
+LANE_DRAM_BYTES_PER_CELL = (7.0e9 + 6.6e9) / 823e6
 
 
 def log(*a):
@@ -660,13 +660,15 @@ def run_ours(args):
                                                          "results"),
                                                      (x / args.steps for x in phases)))},
         "gpu_launches": launches,
-        "roofline": {"bound": "int32", "kernel": "sankoff_fill_kernel",
+        "roofline": {"bound": "int32", "kernel": "sankoff_lane_kernel<2, true>",
                      "achieved": ops / Tf / 1e9, "peak": int_peak, "unit": "Gops/s",
                      "frac": ops / Tf / 1e9 / int_peak,
-                     "traffic": FILL_DRAM_BYTES_PER_CELL * work["cells"],
+                     "traffic": LANE_DRAM_BYTES_PER_CELL * work["cells"],
                      "traffic_note": "DRAM read + write bytes per launch: bytes per cell of the ncu capture of "
-                                     "the 496-pair case times this launch's cells",
+                                     "66 pairs of 180-220 nt times this launch's cells",
                      "ops_per_launch": ops, "fill_ms": Tf * 1e3,
+                     "ops_note": "operations of the recursion on the groups' own cells and valid terms (counted "
+                                 "by the kernel with one warp per group), not what the lanes issue",
                      "peak_source": "measured int32 add+max rate (locarna_gb300/_build/liblcg_probe.so)",
                      "hbm_frac_of_measured": alg_bytes / Tf / 1e9 / peaks.get("hbm_gbs", 6800.0)},
         "int_ops": {"ops_per_step": ops, "cells": work["cells"], "arc_terms": work["arc_terms"],
