@@ -397,7 +397,7 @@ def run_pf(eng, tables, flush_l2, cpu):
         f, bw = eng.pf_last_timing()
         dev[64] += f + bw
         n64 += len(sub)
-        launches += 4
+        launches += 12  # index (2), entries, forward, backward, probabilities; FP32 and FP64
         for k, r in zip(sub, r64):
             am32, bm32 = keep[k]
             ea = float(np.max(np.abs(r["am_prob"] - am32))) if r["am_prob"].size else 0.0
@@ -577,7 +577,7 @@ def run_ours(args):
         f, _ = eng.last_timing()
         kern_ms += ms
         fill_ms += f
-        launches += nl
+        launches += 2 * nl  # fill and traceback; as many for the index structures
     barrier_sync(world)
     res_one = Engine.decode_call(call)
     # end to end: PP texts in, alignments out through the public pipeline,
@@ -601,7 +601,8 @@ def run_ours(args):
         eng.run_pp_call(pcall)  # results are on the host when it returns
         wall_s += time.perf_counter() - s0
         phases = [a + b for a, b in zip(phases, eng.last_phases())]
-        e2e_launches += eng.last_stats()[1] + 2  # + the envelope's two launches
+        # and two for the envelopes of the first chunk's pairs and of the others
+        e2e_launches += 2 * eng.last_stats()[1] + 4
     barrier_sync(world)
     res = Engine.decode_pp_call(pcall)
     graph_captures, graph_replays = eng.last_graphs()
