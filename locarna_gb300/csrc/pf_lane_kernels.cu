@@ -23,9 +23,9 @@
 // row. An item waits only for items that come before it.
 //
 // Sums over lanes are taken by one lane per cell or entry over its 32 words in
-// shared memory, with the rounding errors carried along (pfl_row_sum), so that they
-// are as good as the FP64 atomics over single groups they replace; they end in
-// FP64 atomics, 32 times fewer.
+// shared memory, with next to no rounding (pfl_row_sum), so that they are as good
+// as the FP64 atomics over single groups they replace; they end in FP64 atomics, 32
+// times fewer.
 //
 // What bounds it, and figures (GB300): a warp's serial chain of quads, each some
 // 10,000 cycles backward, half of them latency of L2 and DRAM, and the waits for
@@ -121,31 +121,40 @@ __device__ __forceinline__ void pfl_load8(int at, float (&v)[8]) {
     }
 }
 
-// s += x; returns the rounding error (Knuth's two-sum)
-__device__ __forceinline__ float pfl_two_sum(float &s, float x) {
-    const float y = s + x, z = y - s, err = (s - (y - z)) + (x - z);
-    s = y;
-    return err;
-}
-
-// the sum of the 32 words of row `row` of PFL_SUMS, in one thread: the rounding
-// errors are summed the same way and theirs too (SumK with K = 3; Ogita, Rump, Oishi
-// 2005), which is below FP64's rounding
+// The sum of the 32 words of row `row` of PFL_SUMS, in one thread. Every word is split
+// without error into multiples of a unit that the largest one sets, of a unit 2^18
+// times smaller, and a remainder (vector extraction; Rump, Ogita, Oishi 2008): with
+// top < 2^(e + 1) the units are 2^(e - 17) and 2^(e - 35), so that 32 of the parts add
+// up exactly in FP32, and only the remainders, below 2^(e - 35), are rounded. That is
+// better than a sum in FP64, of which an SM adds two a clock (backward of 21 pairs of
+// 80-500 nt: 47.2 ms; with a two-sum per word, 2^-43 off, 46.7; with a second one for
+// its errors 49.1).
 __device__ __noinline__ double pfl_row_sum(int sb, int row) {
     const int at = sb + PFL_SUMS + 32 * row;
-    float s0 = 0.f, s1 = 0.f, e0 = 0.f, e1 = 0.f, c0 = 0.f, c1 = 0.f;
+    float x[32], top = 0.f;
 #pragma unroll
-    for (int h = 0; h < 32; h += 16) {
-        float x[16];
-#pragma unroll
-        for (int t = 0; t < 16; ++t) x[t] = pfl_f(at + ((row + h + t) & 31));  // (lanes on different banks)
-#pragma unroll
-        for (int t = 0; t < 16; t += 2) {
-            c0 += pfl_two_sum(e0, pfl_two_sum(s0, x[t]));
-            c1 += pfl_two_sum(e1, pfl_two_sum(s1, x[t + 1]));
-        }
+    for (int t = 0; t < 32; ++t) {
+        x[t] = pfl_f(at + ((row + t) & 31));  // (lanes on different banks)
+        top = fmaxf(top, fabsf(x[t]));
     }
-    return ((double)s0 + (double)s1) + (((double)e0 + (double)e1) + ((double)c0 + (double)c1));
+    const int ex = __float_as_int(top) >> 23;
+    if (top != 0.f && (ex < 27 || ex > 227)) {
+        // the units would leave FP32's range (or an infinity)
+        double s = 0.0;
+#pragma unroll 1
+        for (int t = 0; t < 32; ++t) s += (double)pfl_f(at + t);
+        return s;
+    }
+    const float c0 = __int_as_float((ex + 6) << 23) * 1.5f, c1 = c0 * 0x1p-18f;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int t = 0; t < 32; ++t) {
+        const float a = (x[t] + c0) - c0, y = x[t] - a, b = (y + c1) - c1;
+        s0 += a;
+        s1 += b;
+        s2 += y - b;
+    }
+    return (double)s0 + ((double)s1 + (double)s2);
 }
 
 // ---------------------------------------------------------------- forward
