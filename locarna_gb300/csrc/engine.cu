@@ -707,14 +707,17 @@ lcg_status prep_pair(const lcg_pair_tables &t, const lcg_align_opts &o, Prep &p,
     return LCG_OK;
 }
 
-// Whether the device makes the index structures of a chunk: from 2,000 arc
-// matches on its two launches (10 us) cost less than the host's 30 ns per arc
-// match (one 60 x 60 pair: 500 arc matches, 15 us on the host).
+// Whether the device makes the index structures of a chunk: from 1,500 arc matches
+// per host thread on (a thread takes whole pairs), its two launches (20 to 35 us of the
+// fill) cost less than the host's 30 ns per arc match. Calls with the host's and the
+// device's index: one pair of 2,500 arc matches 0.38 and 0.32 ms, 3 pairs of 5,700
+// 0.51 and 0.46, 10 of 21,000 1.53 and 1.45; 10 pairs of 10,800 1.27 and 1.40, 3 of
+// 2,500 0.39 and 0.40 (GB300 host, 16 threads).
 bool index_on_device(const lcg_pair_tables *pairs, int npairs) {
     if (const char *v = std::getenv("LCG_DEVICE_INDEX")) return v[0] != '0';
     long long am = 0;
     for (int q = 0; q < npairs; ++q) am += std::max(pairs[q].num_arcmatches, 0);
-    return am >= 2000;
+    return am >= 1500ll * std::min<long long>(npairs, std::max(1u, std::thread::hardware_concurrency()));
 }
 
 }  // namespace lcg_host
