@@ -120,3 +120,29 @@ def test_pf_lanes_with_less_memory(child, megabytes):
     """)
     first, second, _ = err.split("call")
     assert "refused" in first and "refused" not in second, err
+
+
+# 190 pairs of 55-64 nt in chunks of 40: the envelopes of the pairs behind the first
+# chunk (31 MB at once) are refused where they are enqueued for later, and done in
+# waves; a chunk of the alignment takes less
+@pytest.mark.gpu
+def test_later_envelopes_in_waves(child):
+    err = child("""
+        lens = [55 + k % 10 for k in range(20)]
+        rnas = [make_rna(n, 200 + k).to_pp() for k, n in enumerate(lens)]
+        ids = [(a, b) for a in range(20) for b in range(a + 1, 20)]
+        out = []
+        for nbytes in (0, 30 << 20):
+            eng = Engine(0)
+            eng.set_chunk_pairs(40)
+            os.environ["LCG_LANES"] = "32"
+            call = eng.prepare_pp_call([(rnas[a], rnas[b]) for a, b in ids], [(lens[a], lens[b]) for a, b in ids])
+            limit(nbytes)
+            for _ in range(2):
+                assert eng.run_pp_call(call) == 0
+                out.append([(r.score, r.edges) for r in Engine.decode_pp_call(call)])
+                print("call", file=sys.stderr, flush=True)
+        assert all(o == out[0] for o in out)
+        print("ok")
+    """)
+    assert "refused 3" in err.split("call")[2] and "refused" not in err.split("call")[3], err
