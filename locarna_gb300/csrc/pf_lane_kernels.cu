@@ -121,40 +121,57 @@ __device__ __forceinline__ void pfl_load8(int at, float (&v)[8]) {
     }
 }
 
-// The sum of the 32 words of row `row` of PFL_SUMS, in one thread. Every word is split
-// without error into multiples of a unit that the largest one sets, of a unit 2^18
-// times smaller, and a remainder (vector extraction; Rump, Ogita, Oishi 2008): with
-// top < 2^(e + 1) the units are 2^(e - 17) and 2^(e - 35), so that 32 of the parts add
-// up exactly in FP32, and only the remainders, below 2^(e - 35), are rounded. That is
-// better than a sum in FP64, of which an SM adds two a clock (backward of 21 pairs of
-// 80-500 nt: 47.2 ms; with a two-sum per word, 2^-43 off, 46.7; with a second one for
-// its errors 49.1).
-__device__ __noinline__ double pfl_row_sum(int sb, int row) {
+// The sum of the words [first, last) (multiples of PFL_PART) of row `row` of PFL_SUMS
+// in one thread, PFL_PART at a time. Every word is split without error into multiples
+// of a unit that the largest one sets, of a unit 2^18 times smaller, and a remainder
+// (vector extraction; Rump, Ogita, Oishi 2008): with top < 2^(e + 1) the units are
+// 2^(e - 17) and 2^(e - 35), so that up to 32 of the parts add up exactly in FP32, and
+// only the remainders, below 2^(e - 35), are rounded. That is better than a sum in
+// FP64, of which an SM adds two a clock. Backward of 21 pairs of 80-500 nt: 48.5 ms; a
+// two-sum per word (2^-43 off) 46.1; of 66 pairs of 280-320 nt, whose M is swept again,
+// 271 and 273. All 32 words in straight-line code cost the latter 292 (instruction
+// cache), parts of 8 cost the former 51.
+constexpr int PFL_PART = 16;
+__device__ __noinline__ double pfl_row_sum(int sb, int row, int first, int last) {
     const int at = sb + PFL_SUMS + 32 * row;
-    float x[32], top = 0.f;
-#pragma unroll
-    for (int t = 0; t < 32; ++t) {
-        x[t] = pfl_f(at + ((row + t) & 31));  // (lanes on different banks)
-        top = fmaxf(top, fabsf(x[t]));
-    }
-    const int ex = __float_as_int(top) >> 23;
-    if (top != 0.f && (ex < 27 || ex > 227)) {
-        // the units would leave FP32's range (or an infinity)
-        double s = 0.0;
+    double sum = 0.0;
 #pragma unroll 1
-        for (int t = 0; t < 32; ++t) s += (double)pfl_f(at + t);
-        return s;
-    }
-    const float c0 = __int_as_float((ex + 6) << 23) * 1.5f, c1 = c0 * 0x1p-18f;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    for (int k = first; k < last; k += PFL_PART) {
+        float x[PFL_PART], top = 0.f;
 #pragma unroll
-    for (int t = 0; t < 32; ++t) {
-        const float a = (x[t] + c0) - c0, y = x[t] - a, b = (y + c1) - c1;
-        s0 += a;
-        s1 += b;
-        s2 += y - b;
+        for (int t = 0; t < PFL_PART; ++t) {
+            x[t] = pfl_f(at + ((row + k + t) & 31));  // (lanes on different banks)
+            top = fmaxf(top, fabsf(x[t]));
+        }
+        const int ex = __float_as_int(top) >> 23;
+        if (top != 0.f && (ex < 27 || ex > 227)) {
+            // the units would leave FP32's range (or an infinity)
+#pragma unroll 1
+            for (int t = 0; t < PFL_PART; ++t) sum += (double)pfl_f(at + ((row + k + t) & 31));
+            continue;
+        }
+        const float c0 = __int_as_float((ex + 6) << 23) * 1.5f, c1 = c0 * 0x1p-18f;
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int t = 0; t < PFL_PART; ++t) {
+            const float a = (x[t] + c0) - c0, y = x[t] - a, b = (y + c1) - c1;
+            s0 += a;
+            s1 += b;
+            s2 += y - b;
+        }
+        sum += (double)s0 + ((double)s1 + (double)s2);
     }
-    return (double)s0 + ((double)s1 + (double)s2);
+    return sum;
+}
+
+// the sums of rows [0, n), lane k that of row k: two lanes a row where that is enough
+__device__ __forceinline__ double pfl_row_sums(int sb, int n) {
+    const int lane = threadIdx.x & 31;
+    const bool two = n <= 16;
+    const int row = two ? lane & 15 : lane, first = two ? lane & 16 : 0;
+    double v = row < n ? pfl_row_sum(sb, row, first, two ? first + 16 : 32) : 0.0;
+    if (two) v += __shfl_xor_sync(0xffffffffu, v, 16);
+    return v;
 }
 
 // ---------------------------------------------------------------- forward
@@ -615,7 +632,8 @@ __device__ __forceinline__ void pfl_back_terms(int sb, const float *store, float
             }
             if (!TRUNC) {
                 __syncwarp();
-                if (lane < nb) atomicAdd(P.Dbar + s[4 * lane + 3], pfl_row_sum(sb, lane));
+                const double sum = pfl_row_sums(sb, nb);
+                if (lane < nb) atomicAdd(P.Dbar + s[4 * lane + 3], sum);
                 __syncwarp();
             }
         }
@@ -806,7 +824,7 @@ __device__ __forceinline__ void pfl_back(const PFPair<float> &P, const LaneItem 
                 const int at = (__shfl_sync(0xffffffffu, line, (lane >> 3) + 1) >> 5) + cell0 + (lane & 7);
                 __syncwarp();
                 if (cells >> lane & 1u)
-                    atomicAdd(lc_ptr<const PFPair<float>>(cx, LC_PAIR)->bmacc + at, pfl_row_sum(sb, lane));
+                    atomicAdd(lc_ptr<const PFPair<float>>(cx, LC_PAIR)->bmacc + at, pfl_row_sum(sb, lane, 0, 32));
                 __syncwarp();
                 pfl_back_terms<TRUNC>(sb, store, Mb, raw, cell0, w.z, w.w, d, in, nz, rowwise ? r : -1);
             }
