@@ -244,7 +244,7 @@ lcg_status lcg_engine_set_graphs(lcg_engine eng, int32_t on);
  * hundreds of nt), whichever is more, and where few warps fit in that, the
  * batch is filled by one warp per group. Every in-flight chunk (two at most)
  * has its own, held until the engine is destroyed. LocARNA-P's FP32 batches
- * likewise.
+ * likewise, with twice what one warp per group takes, and at least 4 GiB.
  * LocARNA-P (lcg_pf_forward / lcg_pf_backward) keeps the groups' M (and E, F
  * for the gap gradients) from the forward for the backward pass under the
  * same budget, by default in FP64 (4 GiB) and for FP32 batches swept lane per

@@ -130,11 +130,15 @@ double seq_log_pf(const lcg_pair_tables &t, const std::vector<double> &bm, const
     return logscale + std::log(std::max(Mp[m], 1e-300));
 }
 
-// Bytes of slots that a lane-per-group launch may have: a bounded amount, or the
-// caller's budget (lcg_engine_set_rect_budget), but at least what those of one warp
-// per group take (other).
+// Bytes of slots that a lane-per-group launch may have; other: what those of one warp
+// per group take. By default a bounded amount, or as much as the other. Under a
+// caller's budget (lcg_engine_set_rect_budget) that, or twice the other's, with which
+// nearly all blocks have room: half of them are as slow as one warp per group (190
+// pairs of 90-110 nt 13.1 ms with 608 blocks and 2.9 GB, 17.9 with 304, 17.5 by the
+// other with 0.9 GB; 66 of 280-320 nt 345 with 13.3 GB, 460, 425 with 7.2 GB).
 long long pf_lane_slot_bytes(lcg_engine e, long long other) {
-    return std::max(e->rect_budget < 0 ? PF_LANE_SCRATCH_BYTES : e->rect_budget, other);
+    return e->rect_budget < 0 ? std::max(PF_LANE_SCRATCH_BYTES, other)
+                              : std::max({e->rect_budget, 2 * other, RECT_BUDGET_PLAIN});
 }
 
 // Whether an FP32 batch is swept lane per group (pf_lane_kernels.cu). An
