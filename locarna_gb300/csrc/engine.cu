@@ -850,7 +850,7 @@ long long lane_slot_bytes(lcg_engine e, long long other) {
 // 3.1 ms against 9.6; 15 pairs of 200-300 nt: 6.0 against 7.3), batches to lanes
 // (28 profile pairs of 80-300 columns: 5.6 against 4.9 with 32 groups; 28 pairs of
 // 200-300 nt 10.1 -> 8.8, 45 stacking pairs of 100-300 nt 9.0 -> 6.7; 276 pairs of
-// 60-400 nt in two chunks: 130 -> 84, 70 with 64).
+// 60-400 nt in two chunks: 130 -> 83, 70 with 64).
 int lane_width(lcg_engine e, const lcg_pair_tables *pairs, int npairs, const lcg_align_opts *opts) {
     if (e->counting || opts->struct_local) return 0;
     if (const char *v = std::getenv("LCG_LANES")) return std::atoi(v) == 64 ? 64 : std::atoi(v) == 32 ? 32 : 0;

@@ -291,7 +291,7 @@ lcg_status pf_forward_t(lcg_engine e, PFState *S, const lcg_pair_tables *pairs, 
     // only, as an FP32 recomputation into the warp's slot, read back from L2,
     // is faster than reading the kept rectangle from DRAM (200-nt pair:
     // backward 3.37 ms recomputing, 3.60 ms kept; FP64 7.51 against 6.06 ms).
-    // Lane per group: kept (21 pairs of 80-500 nt: 46 ms, recomputing 89).
+    // Lane per group: kept (21 pairs of 80-500 nt: 48 ms, recomputing 89).
     const int rect_states = o->gap_gradients ? 3 : 1;
     bool keep, top_ef;
     {

@@ -30,9 +30,9 @@
 // What bounds it, and figures (GB300): a warp's serial chain of quads, each some
 // 10,000 cycles backward, half of them latency of L2 and DRAM, and the waits for
 // the uses behind it; issue slots are a quarter used, DRAM at 1.5 of 6.8 TB/s.
-// Backward over 28 pairs of 160-200 nt: 21.5 ms with one warp per group, 9.2 here
-// (M kept by the forward pass; 13.8 recomputing it); 21 pairs of 80-500 nt: 120 and
-// 46 (89); forward 5.0 and 4.8, 31 and 25.5. What mattered on the way: an entry's
+// Backward over 28 pairs of 160-200 nt: 23 ms with one warp per group, 9.7 here (M kept
+// by the forward pass); 21 pairs of 80-500 nt: 123 and 48.5; forward 5.1 and 4.9, 32 and
+// 26. M swept again: 66 pairs of 280-320 nt 333 and 271. What mattered on the way: an entry's
 // lines copied to shared memory in one go (21 pairs: 104 -> 50 ms; loads behind a
 // branch came one by one), no register spilled (64 loads in flight with 460 bytes
 // spilled: 57 instead of 50), and one copy of the entries' code (57 -> 46: a second

@@ -30,10 +30,11 @@
 //
 // What bounds it, and figures (GB300, fill time): a quad is some 1,200 (32
 // groups) to 1,600 (64) warp instructions behind a chain of L2 and DRAM
-// latencies, 16 warps per SM; neither the issue slots (20 to 30 % used) nor DRAM
-// (1.4 of 6.8 TB/s) are full. 276 pairs of 60-400 nt in two chunks: 126 ms with
-// one warp per group, 82 ms here with 32 groups per item, 64 ms with 64 (fewer
-// items to wait for, the per-quad work shared by more groups). Registers hold
+// latencies, 16 warps per SM; neither the issue slots (30 % used) nor DRAM (2.3 of
+// 6.8 TB/s; both for 66 pairs of 180-220 nt, 64 groups) are full. 276 pairs of 60-400
+// nt in two chunks: 130 ms with one warp per group, 83 ms here with 32 groups per item,
+// 70 ms with 64 (fewer items to wait for, the per-quad work shared by more groups).
+// Registers hold
 // the rows and the loads in flight and nothing else: versions that spilled 100
 // to 600 bytes took 1.3 to 2 times as long, since a spilled word comes back
 // from L2 (the lines in flight leave L1 no room).

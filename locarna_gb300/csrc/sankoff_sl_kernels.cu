@@ -60,9 +60,9 @@ __device__ __forceinline__ int maxplus_scan(int a, int b, int x0, int lane) {
 // that a term is one 16-byte load: with a matrix per state its four words came from
 // four sectors of L2 and DRAM (fill of a 400 x 400 pair 8.3 -> 7.8 ms, traceback 0.75 ->
 // 0.64). What bounds the fill is the latency of a row's entries and their terms
-// with 16 warps an SM (116 registers, 14 KB of rows a warp; issue slots a quarter
-// used, DRAM 1.4 of 6.8 TB/s): entries read a row, or 32, ahead 9.6 -> 8.3 ms; 64 at
-// a time gave nothing more.
+// with 16 warps an SM (116 registers; one 250 x 250 pair: issue slots a third used,
+// DRAM 1.2 of 6.8 TB/s): entries read a row, or 32, ahead 9.6 -> 8.3 ms; 64 at a time
+// gave nothing more.
 template <int NS>
 __device__ __forceinline__ void sl_put(int *Mg, long long cell, int m0, int m1, int m2, int m3, int m4, int m5, int m6,
                                        int m7) {
